@@ -44,50 +44,66 @@ struct Vec {
   }
 };
 
-__device__ __forceinline__ float sigmoidf(float x) { return 1.0f / (1.0f + __expf(-x)); }
+__device__ __forceinline__ float sigmoidf(float x) { return __frcp_rn(1.0f + __expf(-x)); }
 
-// out[m, d] = silu(gu[m, d]) * gu[m, D + d]
+// Work of the two gated-activation kernels: `total` vectors, vector v = (row, d) with d the fast index.  The row
+// comes from a multiplication (row = v * magic >> 40): a 64-bit division per vector was a third of the kernels'
+// instructions.
+struct GluGeom {
+  uint32_t total, vec_per_row;
+  uint64_t magic;  // ceil(2^40 / vec_per_row): exact while v < 2^24 and v * vec_per_row < 2^40 (0: a single row)
+  int64_t first_row;
+};
+__device__ __forceinline__ void glu_index(const GluGeom& gg, uint32_t v, uint32_t* row, uint32_t* d) {
+  *row = (uint32_t)(((uint64_t)v * gg.magic) >> 40);
+  *d = v - *row * gg.vec_per_row;
+}
+
+// out[m, d] = silu(gu[m, d]) * gu[m, D + d].  HBM-bound (6 bytes per bf16 output).  Both kernels walk their rows
+// from the last to the first: the GEMM before them wrote the last rows last, so those are read from L2 instead of
+// being written out first.  8192 x 8192 bf16: forward 102 -> 88 us, backward 140 -> 124 us (same box) with the two
+// changes; two vectors per thread in flight (57 registers) made the forward slower.
 template <int DT>
 __global__ void __launch_bounds__(256)
-swiglu_forward_kernel(const void* __restrict__ gu, int64_t rows, int D, void* __restrict__ out) {
+swiglu_forward_kernel(const void* __restrict__ gu, const GluGeom gg, int D, void* __restrict__ out) {
   constexpr int VN = Vec<DT>::N;
-  const int vec_per_row = D / VN;
-  const int64_t total = rows * vec_per_row;
-  for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < total; v += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t m = v / vec_per_row;
-    const int d = (int)(v - m * vec_per_row) * VN;
+  const uint32_t stride = gridDim.x * blockDim.x;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < gg.total; i += stride) {
+    uint32_t row, d;
+    glu_index(gg, gg.total - 1 - i, &row, &d);
+    const int64_t in = (gg.first_row + row) * 2 * D + d * VN;
     float gate[VN], up[VN], o[VN];
-    Vec<DT>::load(gu, m * 2 * D + d, gate);
-    Vec<DT>::load(gu, m * 2 * D + D + d, up);
+    Vec<DT>::load(gu, in, gate);
+    Vec<DT>::load(gu, in + D, up);
 #pragma unroll
     for (int i = 0; i < VN; ++i) o[i] = gate[i] * sigmoidf(gate[i]) * up[i];
-    Vec<DT>::store(out, m * D + d, o);
+    Vec<DT>::store(out, (gg.first_row + row) * D + d * VN, o);
   }
 }
 
 // dgu[m, d] = g * up * silu'(gate),  dgu[m, D + d] = g * silu(gate)
 template <int DT>
 __global__ void __launch_bounds__(256)
-swiglu_backward_kernel(const void* __restrict__ gu, const void* __restrict__ g, int64_t rows, int D,
+swiglu_backward_kernel(const void* __restrict__ gu, const void* __restrict__ g, const GluGeom gg, int D,
                        void* __restrict__ dgu) {
   constexpr int VN = Vec<DT>::N;
-  const int vec_per_row = D / VN;
-  const int64_t total = rows * vec_per_row;
-  for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < total; v += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t m = v / vec_per_row;
-    const int d = (int)(v - m * vec_per_row) * VN;
+  const uint32_t stride = gridDim.x * blockDim.x;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < gg.total; i += stride) {
+    uint32_t row, d;
+    glu_index(gg, gg.total - 1 - i, &row, &d);
+    const int64_t in = (gg.first_row + row) * 2 * D + d * VN;
     float gate[VN], up[VN], go[VN], dgate[VN], dup[VN];
-    Vec<DT>::load(gu, m * 2 * D + d, gate);
-    Vec<DT>::load(gu, m * 2 * D + D + d, up);
-    Vec<DT>::load(g, m * D + d, go);
+    Vec<DT>::load(gu, in, gate);
+    Vec<DT>::load(gu, in + D, up);
+    Vec<DT>::load(g, (gg.first_row + row) * D + d * VN, go);
 #pragma unroll
     for (int i = 0; i < VN; ++i) {
       const float s = sigmoidf(gate[i]);
       dup[i] = go[i] * gate[i] * s;
       dgate[i] = go[i] * up[i] * s * (1.0f + gate[i] * (1.0f - s));
     }
-    Vec<DT>::store(dgu, m * 2 * D + d, dgate);
-    Vec<DT>::store(dgu, m * 2 * D + D + d, dup);
+    Vec<DT>::store(dgu, in, dgate);
+    Vec<DT>::store(dgu, in + D, dup);
   }
 }
 
@@ -146,6 +162,21 @@ inline unsigned glue_grid(int64_t work) {
   const int64_t blocks = (work + 255) / 256;
   return (unsigned)(blocks < 1 ? 1 : blocks < 148 * 16 ? blocks : 148 * 16);
 }
+// Calls fn(GluGeom) for runs of rows short enough for the row index by multiplication (one run up to 2^24 vectors).
+template <class Fn>
+void for_row_runs(int64_t rows, int vec_per_row, Fn fn) {
+  int64_t most = ((int64_t)1 << 24) < ((int64_t)1 << 40) / vec_per_row ? (int64_t)1 << 24 : ((int64_t)1 << 40) / vec_per_row;
+  most = most / vec_per_row > 1 ? most / vec_per_row : 1;
+  for (int64_t r = 0; r < rows; r += most) {
+    const int64_t n = rows - r < most ? rows - r : most;
+    GluGeom gg;
+    gg.vec_per_row = (uint32_t)vec_per_row;
+    gg.total = (uint32_t)(n * vec_per_row);
+    gg.magic = n > 1 ? (((uint64_t)1 << 40) + vec_per_row - 1) / vec_per_row : 0;
+    gg.first_row = r;
+    fn(gg);
+  }
+}
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 }  // namespace
@@ -165,9 +196,11 @@ int al_swiglu_forward(int32_t dtype, const void* gate_up, int64_t rows, int32_t 
   }
   if (rows == 0) return AL_OK;
   cudaStream_t s = (cudaStream_t)stream;
-  const unsigned grid = glue_grid(rows * (width / vn));
-  if (dtype == AL_F32) swiglu_forward_kernel<kF32><<<grid, 256, 0, s>>>(gate_up, rows, width, out);
-  else swiglu_forward_kernel<kBF16><<<grid, 256, 0, s>>>(gate_up, rows, width, out);
+  for_row_runs(rows, width / vn, [&](const GluGeom& gg) {
+    const unsigned grid = glue_grid(gg.total);
+    if (dtype == AL_F32) swiglu_forward_kernel<kF32><<<grid, 256, 0, s>>>(gate_up, gg, width, out);
+    else swiglu_forward_kernel<kBF16><<<grid, 256, 0, s>>>(gate_up, gg, width, out);
+  });
   return check_launch("swiglu_forward");
 }
 
@@ -181,9 +214,11 @@ int al_swiglu_backward(int32_t dtype, const void* gate_up, const void* grad_out,
   }
   if (rows == 0) return AL_OK;
   cudaStream_t s = (cudaStream_t)stream;
-  const unsigned grid = glue_grid(rows * (width / vn));
-  if (dtype == AL_F32) swiglu_backward_kernel<kF32><<<grid, 256, 0, s>>>(gate_up, grad_out, rows, width, grad_gate_up);
-  else swiglu_backward_kernel<kBF16><<<grid, 256, 0, s>>>(gate_up, grad_out, rows, width, grad_gate_up);
+  for_row_runs(rows, width / vn, [&](const GluGeom& gg) {
+    const unsigned grid = glue_grid(gg.total);
+    if (dtype == AL_F32) swiglu_backward_kernel<kF32><<<grid, 256, 0, s>>>(gate_up, grad_out, gg, width, grad_gate_up);
+    else swiglu_backward_kernel<kBF16><<<grid, 256, 0, s>>>(gate_up, grad_out, gg, width, grad_gate_up);
+  });
   return check_launch("swiglu_backward");
 }
 
