@@ -542,17 +542,17 @@ int64_t al_smallm_scratch_floats(int32_t M, int32_t N, int32_t T) {
 }
 
 namespace {
-// reductions of the bias / range / clip gradients, rounded up to 16 bytes; the partial sums of
-// a split CUDA-core weight gradient follow
-int64_t backward_reduce_floats(int32_t M, int32_t N, int32_t T) {
-  const int64_t n = 256 * (int64_t)N + 3 * (int64_t)T * M + 16 + 2 * (int64_t)T + 16;
+// reductions of the range / clip gradients, rounded up to 16 bytes; the partial sums of a split weight gradient
+// follow
+int64_t backward_reduce_floats(int32_t M, int32_t T) {
+  const int64_t n = 3 * (int64_t)T * M + 16 + 2 * (int64_t)T + 16;
   return (n + 3) / 4 * 4;
 }
 }  // namespace
 
 int64_t al_backward_scratch_floats(int32_t M, int32_t K, int32_t N, int32_t T) {
   if (M <= 0 || K <= 0 || N <= 0 || T <= 0) return 0;
-  return backward_reduce_floats(M, N, T) + al::wgrad_simt_partial_floats(M, K, N, T);
+  return backward_reduce_floats(M, T) + al::wgrad_simt_partial_floats(M, K, N, T);
 }
 
 int al_pair_work_item(int32_t num_blocks, int32_t n_pairs, int32_t item, int32_t* total, int32_t* block, int32_t* half) {
@@ -656,7 +656,7 @@ int al_backward(const AlDesc* desc, const AlBackwardArgs* a, void* stream) {
       }
       rc = launch_static_ir_backward(d.dtype, a->x, a->ir_rows, a->grad_x, d.M, d.K, tt, dv.decay,
                                      dv.input_min_percentage, a->grad_input_range,
-                                     a->reduce_scratch + 256 * (int64_t)d.N, d.ir_mode == AL_IR_FAST, s);
+                                     a->reduce_scratch, d.ir_mode == AL_IR_FAST, s);
       if (rc) return rc;
     }
   } else if (a->grad_input_range) {
@@ -670,7 +670,7 @@ int al_backward(const AlDesc* desc, const AlBackwardArgs* a, void* stream) {
     wgrad_simt_plan(d.M, d.K, d.N, d.T, &w_splits, &w_chunk);
     float* w_partial = nullptr;
     if (w_splits > 1) {
-      const int64_t fixed = backward_reduce_floats(d.M, d.N, d.T);
+      const int64_t fixed = backward_reduce_floats(d.M, d.T);
       w_partial = a->reduce_scratch ? a->reduce_scratch + fixed : nullptr;
       const int64_t capacity = a->reduce_scratch ? a->reduce_scratch_floats - fixed : 0;
       if (w_partial == nullptr || (int64_t)w_splits * d.N * d.K > capacity) {
@@ -700,7 +700,7 @@ int al_backward(const AlDesc* desc, const AlBackwardArgs* a, void* stream) {
     }
     // the partial sums of a split CUDA-core weight gradient sit behind the reductions; what is
     // left of the caller's buffer there is the capacity the launch may use
-    const int64_t fixed = backward_reduce_floats(d.M, d.N, d.T);
+    const int64_t fixed = backward_reduce_floats(d.M, d.T);
     float* partial = a->reduce_scratch ? a->reduce_scratch + fixed : nullptr;
     const int64_t partial_capacity = a->reduce_scratch ? a->reduce_scratch_floats - fixed : 0;
     rc = tc ? launch_wgrad_tc(a->grad_out, a->xq, mask, mask_words, d.M, d.K, d.N, gt, pairing, a->grad_w, s)
@@ -715,7 +715,7 @@ int al_backward(const AlDesc* desc, const AlBackwardArgs* a, void* stream) {
                 "and reduce_scratch");
       return AL_ERR_BAD_ARGUMENT;
     }
-    float* tile_max = a->reduce_scratch + 256 * (int64_t)d.N + 3 * (int64_t)d.T * d.M + 16;
+    float* tile_max = a->reduce_scratch + 3 * (int64_t)d.T * d.M + 16;
     int32_t* flags = (int32_t*)(tile_max + d.T);
     const int discretize = dv.weight_quant == AL_QUANT_DISCRETIZE_PER_CHANNEL;
     rc = launch_tile_max(d.dtype, a->learnable_weight_clip, d.N, tt, discretize ? dv.weight_quant : kQuantLearnClamp,
@@ -727,11 +727,7 @@ int al_backward(const AlDesc* desc, const AlBackwardArgs* a, void* stream) {
     if (rc) return rc;
   }
   if (a->grad_bias) {
-    if (!a->reduce_scratch) {
-      set_error("al_backward: reduce_scratch missing");
-      return AL_ERR_BAD_ARGUMENT;
-    }
-    rc = launch_bias_grad(d.dtype, a->grad_out, d.M, d.N, a->grad_bias, a->reduce_scratch, s);
+    rc = launch_bias_grad(d.dtype, a->grad_out, d.M, d.N, a->grad_bias, s);
     if (rc) return rc;
   }
   return AL_OK;

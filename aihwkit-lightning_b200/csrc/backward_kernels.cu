@@ -2,95 +2,188 @@
 // the upstream gradient) and, for learned/fixed input ranges, the input-range gradient with
 // its decay term followed by the straight-through zeroing of clipped inputs.  Both reduce in
 // two stages with a fixed order (no floating-point atomics).
+#include <cooperative_groups.h>
+
 #include "analog_math.cuh"
 #include "internal.h"
+
+namespace cg = cooperative_groups;
 
 namespace al {
 
 namespace {
 
-constexpr int kBiasChunks = 256;
-
-// partial[c, n] = sum of g[m, n] over the rows m of chunk c
-template <int DT>
-__global__ void bias_partial_kernel(const void* __restrict__ g, int M, int N, int rows_per_chunk,
-                                    float* __restrict__ partial) {
-  int n = blockIdx.x * blockDim.x + threadIdx.x;
-  int c = blockIdx.y;
-  if (n >= N) return;
-  int m_lo = c * rows_per_chunk, m_hi = min(M, m_lo + rows_per_chunk);
-  float s = 0.0f;
-  for (int m = m_lo; m < m_hi; ++m) s += Elem<DT>::load(g, (int64_t)m * N + n);
-  partial[(int64_t)c * N + n] = s;
+// Column sums of g [M, N] in one launch.  A cluster of kBiasCluster CTAs owns 64 columns; each CTA adds every
+// kBiasCluster-th group of rows (a thread: VN columns of every (kBiasCluster * rows-per-pass)-th row, kBiasAhead
+// loads in flight), then the row groups are added in shared memory and the CTAs of the cluster through distributed
+// shared memory, always in the same order.  Bound by reading g once.
+constexpr int kBiasCluster = 8, kBiasCols = 64, kBiasThreads = 256, kBiasAhead = 8;
+template <int DT, int VN>
+__device__ __forceinline__ void load_cols(const void* p, int64_t idx, float v[VN]) {
+  if (VN == 1) {
+    v[0] = Elem<DT>::load(p, idx);
+  } else if (DT == kF32) {
+    const float4 f = *reinterpret_cast<const float4*>(static_cast<const float*>(p) + idx);
+    v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+  } else {
+    const uint2 u = *reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(p) + idx);
+    v[0] = __uint_as_float(u.x << 16); v[1] = __uint_as_float(u.x & 0xffff0000u);
+    v[2] = __uint_as_float(u.y << 16); v[3] = __uint_as_float(u.y & 0xffff0000u);
+  }
 }
-template <int DT>
-__global__ void bias_final_kernel(const float* __restrict__ partial, int chunks, int N,
-                                  void* __restrict__ grad_bias) {
-  int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= N) return;
-  float s = 0.0f;
-  for (int c = 0; c < chunks; ++c) s += partial[(int64_t)c * N + n];
-  Elem<DT>::store(grad_bias, n, s);
+template <int DT, int VN>
+__global__ void __cluster_dims__(1, kBiasCluster, 1) __launch_bounds__(kBiasThreads)
+bias_grad_kernel(const void* __restrict__ g, int M, int N, void* __restrict__ grad_bias) {
+  constexpr int kColThreads = kBiasCols / VN, kRowThreads = kBiasThreads / kColThreads;
+  __shared__ float part[kRowThreads][kBiasCols];
+  __shared__ float total[kBiasCols];
+  const int tc = threadIdx.x % kColThreads, tr = threadIdx.x / kColThreads;
+  const int n = blockIdx.x * kBiasCols + tc * VN;  // N % VN == 0
+  float s[VN];
+#pragma unroll
+  for (int i = 0; i < VN; ++i) s[i] = 0.0f;
+  constexpr int kStep = kRowThreads * kBiasCluster;
+  if (n < N) {
+    int m = (int)blockIdx.y * kRowThreads + tr;
+    for (; m + (kBiasAhead - 1) * kStep < M; m += kBiasAhead * kStep) {
+      float v[kBiasAhead][VN];
+#pragma unroll
+      for (int u = 0; u < kBiasAhead; ++u) load_cols<DT, VN>(g, (int64_t)(m + u * kStep) * N + n, v[u]);
+#pragma unroll
+      for (int u = 0; u < kBiasAhead; ++u)
+#pragma unroll
+        for (int i = 0; i < VN; ++i) s[i] = fadd(s[i], v[u][i]);
+    }
+    for (; m < M; m += kStep) {
+      float v[VN];
+      load_cols<DT, VN>(g, (int64_t)m * N + n, v);
+#pragma unroll
+      for (int i = 0; i < VN; ++i) s[i] = fadd(s[i], v[i]);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < VN; ++i) part[tr][tc * VN + i] = s[i];
+  __syncthreads();
+  if (threadIdx.x < kBiasCols) {
+    float sum = part[0][threadIdx.x];
+#pragma unroll
+    for (int r = 1; r < kRowThreads; ++r) sum = fadd(sum, part[r][threadIdx.x]);
+    total[threadIdx.x] = sum;
+  }
+  cg::cluster_group cluster = cg::this_cluster();
+  cluster.sync();
+  if (blockIdx.y == 0 && threadIdx.x < kBiasCols && blockIdx.x * kBiasCols + threadIdx.x < N) {
+    float sum = total[threadIdx.x];
+#pragma unroll
+    for (int c = 1; c < kBiasCluster; ++c) sum = fadd(sum, cluster.map_shared_rank(total, c)[threadIdx.x]);
+    Elem<DT>::store(grad_bias, blockIdx.x * kBiasCols + threadIdx.x, sum);
+  }
+  cluster.sync();  // no CTA leaves while another still reads its sums
 }
 
-// One warp per (row, tile): partial sums for the range gradient, then zero grad_x where the
-// input was clipped and does not sit exactly on the range.
-template <int DT>
+// Partial sums for the range gradient, then zero grad_x where the input was clipped and does not sit exactly on
+// the range.  A block takes `block_rows` consecutive rows of one tile and writes one triple of partial sums.  Bound by reading x and grad_x once.  VEC: every (row, tile) segment starts and ends on a 16-byte
+// boundary (the launcher checked), so a lane moves 16-byte vectors; single elements otherwise.
+struct IrSums {
+  float up, lo, cnt;
+};
+// one element: sums, and whether its gradient is blocked
+__device__ __forceinline__ bool ir_element(float xv, float gv, float ir, int fast_mode, IrSums& s) {
+  if (fast_mode) {
+    // plain clamp with tensor bounds: the bounds collect the gradient outside [-ir, ir]
+    const bool up = xv > ir, dn = xv < -ir;
+    if (up) s.up += gv;
+    if (dn) s.lo += gv;
+    return up || dn;
+  }
+  const bool up = xv >= ir, dn = xv <= -ir;
+  if (up) s.up += fminf(gv, 0.0f);
+  if (dn) s.lo += fmaxf(gv, 0.0f);
+  if (!(up || dn)) return false;
+  s.cnt += 1.0f;
+  return fabsf(xv) != ir;
+}
+template <int DT, bool VEC>
 __global__ void __launch_bounds__(256)
 static_ir_partial_kernel(const void* __restrict__ x, const void* __restrict__ ir_used,
                          void* __restrict__ grad_x, int M, int K, TileTable tt,
-                         float* __restrict__ partial, int fast_mode) {
-  const unsigned seg = blockIdx.x * 8 + (threadIdx.x >> 5);  // rows * T < 2^31 (checked by the host)
-  int lane = threadIdx.x & 31;
-  if (seg >= (unsigned)M * (unsigned)tt.T) return;
-  const int m = (int)(seg / (unsigned)tt.T), t = (int)(seg - (unsigned)m * (unsigned)tt.T);
-  int lo = tt.lo(t), len = tt.hi(t) - lo;
-  int64_t start = (int64_t)m * K + lo;
-  float ir = Elem<DT>::load(ir_used, t);
-  float s_up = 0.0f, s_lo = 0.0f, cnt = 0.0f;
-  for (int i = lane; i < len; i += 32) {
-    float xv = Elem<DT>::load(x, start + i);
-    float gv = Elem<DT>::load(grad_x, start + i);
-    if (fast_mode) {
-      // plain clamp with tensor bounds: the bounds collect the gradient outside [-ir, ir]
-      bool up = xv > ir, dn = xv < -ir;
-      if (up) s_up += gv;
-      if (dn) s_lo += gv;
-      if (up || dn) Elem<DT>::store(grad_x, start + i, 0.0f);
-      continue;
-    }
-    bool up = xv >= ir, dn = xv <= -ir;
-    if (up) s_up += fminf(gv, 0.0f);
-    if (dn) s_lo += fmaxf(gv, 0.0f);
-    if (up || dn) {
-      cnt += 1.0f;
-      if (fabsf(xv) != ir) Elem<DT>::store(grad_x, start + i, 0.0f);
+                         float* __restrict__ partial, int fast_mode, int block_rows) {
+  __shared__ float part[8][3];
+  const int t = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int lo = tt.lo(t), len = tt.hi(t) - lo;
+  const float ir = Elem<DT>::load(ir_used, t);
+  IrSums s = {0.0f, 0.0f, 0.0f};
+  const int m_end = min(M, (int)(blockIdx.x + 1) * block_rows);
+  for (int m = (int)blockIdx.x * block_rows + warp; m < m_end; m += 8) {
+    const int64_t start = (int64_t)m * K + lo;
+    if (VEC) {
+      constexpr int VN = DT == kF32 ? 4 : 8;
+      constexpr int ES = 16 / VN;
+      const uint4* xv = reinterpret_cast<const uint4*>(reinterpret_cast<const char*>(x) + start * ES);
+      uint4* gv = reinterpret_cast<uint4*>(reinterpret_cast<char*>(grad_x) + start * ES);
+      const int nvec = len / VN;
+#pragma unroll 4
+      for (int v = lane; v < nvec; v += 32) {
+        const uint4 xq = xv[v], gq = gv[v];
+        const uint32_t xw[4] = {xq.x, xq.y, xq.z, xq.w};
+        uint32_t gw[4] = {gq.x, gq.y, gq.z, gq.w};
+        bool blocked = false;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          if (DT == kF32) {
+            if (ir_element(__uint_as_float(xw[i]), __uint_as_float(gw[i]), ir, fast_mode, s)) {
+              gw[i] = 0u;
+              blocked = true;
+            }
+          } else {
+            if (ir_element(__uint_as_float(xw[i] << 16), __uint_as_float(gw[i] << 16), ir, fast_mode, s)) {
+              gw[i] &= 0xffff0000u;
+              blocked = true;
+            }
+            if (ir_element(__uint_as_float(xw[i] & 0xffff0000u), __uint_as_float(gw[i] & 0xffff0000u), ir, fast_mode, s)) {
+              gw[i] &= 0x0000ffffu;
+              blocked = true;
+            }
+          }
+        }
+        if (blocked) gv[v] = make_uint4(gw[0], gw[1], gw[2], gw[3]);
+      }
+    } else {
+      for (int i = lane; i < len; i += 32)
+        if (ir_element(Elem<DT>::load(x, start + i), Elem<DT>::load(grad_x, start + i), ir, fast_mode, s))
+          Elem<DT>::store(grad_x, start + i, 0.0f);
     }
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
-    s_up += __shfl_xor_sync(0xffffffffu, s_up, o);
-    s_lo += __shfl_xor_sync(0xffffffffu, s_lo, o);
-    cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+    s.up += __shfl_xor_sync(0xffffffffu, s.up, o);
+    s.lo += __shfl_xor_sync(0xffffffffu, s.lo, o);
+    s.cnt += __shfl_xor_sync(0xffffffffu, s.cnt, o);
   }
   if (lane == 0) {
-    float* p = partial + ((int64_t)t * M + m) * 3;
-    p[0] = s_up;
-    p[1] = s_lo;
-    p[2] = cnt;
+    part[warp][0] = s.up;
+    part[warp][1] = s.lo;
+    part[warp][2] = s.cnt;
+  }
+  __syncthreads();
+  if (threadIdx.x < 3) {
+    float sum = part[0][threadIdx.x];
+#pragma unroll
+    for (int w = 1; w < 8; ++w) sum += part[w][threadIdx.x];
+    partial[((int64_t)t * gridDim.x + blockIdx.x) * 3 + threadIdx.x] = sum;
   }
 }
 
 template <int DT>
 __global__ void static_ir_final_kernel(const float* __restrict__ partial,
-                                       const void* __restrict__ ir_used, int M, TileTable tt,
+                                       const void* __restrict__ ir_used, int M, int n_partials, TileTable tt,
                                        float decay, float input_min_percentage,
                                        void* __restrict__ grad_ir, int fast_mode) {
   __shared__ double sm[3][256];
   int t = blockIdx.x;
   double a = 0.0, b = 0.0, c = 0.0;
-  for (int m = threadIdx.x; m < M; m += blockDim.x) {
-    const float* p = partial + ((int64_t)t * M + m) * 3;
+  for (int i = threadIdx.x; i < n_partials; i += blockDim.x) {
+    const float* p = partial + ((int64_t)t * n_partials + i) * 3;
     a += (double)p[0];
     b += (double)p[1];
     c += (double)p[2];
@@ -200,19 +293,17 @@ int launch_learn_clip_backward(int dtype, const void* w, const void* clip, const
   return check_launch("learn_clip_backward");
 }
 
-int launch_bias_grad(int dtype, const void* g, int M, int N, void* grad_bias, float* scratch,
-                     cudaStream_t s) {
-  ProfScope prof(AL_K_BIAS_GRAD, s, 2);
-  int chunks = M < kBiasChunks ? M : kBiasChunks;
-  int rows_per_chunk = (M + chunks - 1) / chunks;
-  chunks = (M + rows_per_chunk - 1) / rows_per_chunk;
-  dim3 grid((N + 127) / 128, chunks);
+int launch_bias_grad(int dtype, const void* g, int M, int N, void* grad_bias, cudaStream_t s) {
+  ProfScope prof(AL_K_BIAS_GRAD, s);
+  const dim3 grid((N + kBiasCols - 1) / kBiasCols, kBiasCluster);
+  const uintptr_t align = dtype == AL_F32 ? 16 : 8;
+  const bool vec = N % 4 == 0 && reinterpret_cast<uintptr_t>(g) % align == 0;
   if (dtype == AL_F32) {
-    bias_partial_kernel<kF32><<<grid, 128, 0, s>>>(g, M, N, rows_per_chunk, scratch);
-    bias_final_kernel<kF32><<<(N + 127) / 128, 128, 0, s>>>(scratch, chunks, N, grad_bias);
+    if (vec) bias_grad_kernel<kF32, 4><<<grid, kBiasThreads, 0, s>>>(g, M, N, grad_bias);
+    else bias_grad_kernel<kF32, 1><<<grid, kBiasThreads, 0, s>>>(g, M, N, grad_bias);
   } else {
-    bias_partial_kernel<kBF16><<<grid, 128, 0, s>>>(g, M, N, rows_per_chunk, scratch);
-    bias_final_kernel<kBF16><<<(N + 127) / 128, 128, 0, s>>>(scratch, chunks, N, grad_bias);
+    if (vec) bias_grad_kernel<kBF16, 4><<<grid, kBiasThreads, 0, s>>>(g, M, N, grad_bias);
+    else bias_grad_kernel<kBF16, 1><<<grid, kBiasThreads, 0, s>>>(g, M, N, grad_bias);
   }
   return check_launch("bias_grad");
 }
@@ -221,15 +312,24 @@ int launch_static_ir_backward(int dtype, const void* x, const void* ir_used, voi
                               int K, const TileTable& tt, float decay, float input_min_percentage,
                               void* grad_ir, float* scratch, int fast_mode, cudaStream_t s) {
   ProfScope prof(AL_K_IR_BACKWARD, s, grad_ir ? 2 : 1);
-  int64_t segs = (int64_t)M * tt.T;
-  unsigned blocks = (unsigned)((segs + 7) / 8);
-  if (dtype == AL_F32) {
-    static_ir_partial_kernel<kF32><<<blocks, 256, 0, s>>>(x, ir_used, grad_x, M, K, tt, scratch, fast_mode);
-    if (grad_ir) static_ir_final_kernel<kF32><<<tt.T, 256, 0, s>>>(scratch, ir_used, M, tt, decay, input_min_percentage, grad_ir, fast_mode);
-  } else {
-    static_ir_partial_kernel<kBF16><<<blocks, 256, 0, s>>>(x, ir_used, grad_x, M, K, tt, scratch, fast_mode);
-    if (grad_ir) static_ir_final_kernel<kBF16><<<tt.T, 256, 0, s>>>(scratch, ir_used, M, tt, decay, input_min_percentage, grad_ir, fast_mode);
-  }
+  // 32 rows per block; 8 (a row per warp) where that leaves SMs without a block
+  const int block_rows = (int64_t)M * tt.T >= 32 * 4 * 148 ? 32 : 8;
+  const int n_partials = (M + block_rows - 1) / block_rows;
+  const dim3 grid(n_partials, tt.T);
+  const int vn = dtype == AL_F32 ? 4 : 8;
+  bool vec = reinterpret_cast<uintptr_t>(x) % 16 == 0 && reinterpret_cast<uintptr_t>(grad_x) % 16 == 0 && K % vn == 0;
+  for (int t = 0; t < tt.T; ++t) vec = vec && tt.hi(t) % vn == 0;
+#define AL_STATIC_IR(DT_)                                                                                             \
+  do {                                                                                                                \
+    if (vec) static_ir_partial_kernel<DT_, true><<<grid, 256, 0, s>>>(x, ir_used, grad_x, M, K, tt, scratch, fast_mode, block_rows); \
+    else static_ir_partial_kernel<DT_, false><<<grid, 256, 0, s>>>(x, ir_used, grad_x, M, K, tt, scratch, fast_mode, block_rows);    \
+    if (grad_ir)                                                                                                      \
+      static_ir_final_kernel<DT_><<<tt.T, 256, 0, s>>>(scratch, ir_used, M, n_partials, tt, decay,                    \
+                                                       input_min_percentage, grad_ir, fast_mode);                     \
+  } while (0)
+  if (dtype == AL_F32) AL_STATIC_IR(kF32);
+  else AL_STATIC_IR(kBF16);
+#undef AL_STATIC_IR
   return check_launch("static_ir_backward");
 }
 

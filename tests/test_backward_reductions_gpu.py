@@ -1,0 +1,63 @@
+"""Reductions of the backward pass against float64 sums: the bias gradient (column sums over a cluster of CTAs) and
+the gradient of a static input range with its straight-through zeroing."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("m,n", [(1, 1), (7, 63), (129, 64), (512, 1024), (1000, 1500), (1023, 65), (4097, 260)])
+def test_bias_gradient_is_the_column_sum(dtype, m, n):
+    from aihwkit_lightning_b200 import _lib
+
+    lib = _lib.load()
+    gen = torch.Generator(device="cuda").manual_seed(m + n)
+    g = torch.randn(m, n, device="cuda", generator=gen).to(dtype)
+    out = torch.full((n + 8,), 7.0, device="cuda", dtype=dtype)
+    desc = _lib.AlDesc()
+    desc.M, desc.K, desc.N, desc.T = m, 8, n, 1
+    desc.dtype = _lib.AL_F32 if dtype == torch.float32 else _lib.AL_BF16
+    desc.inp_res = desc.out_res = desc.out_bound = -1.0
+    args = _lib.AlBackwardArgs()
+    args.tile_ends = _lib.tile_ends_array([8])
+    args.grad_out, args.grad_bias = g.data_ptr(), out.data_ptr()
+    _lib.check(lib.al_backward(desc, args, torch.cuda.current_stream().cuda_stream))
+    want, scale = g.double().sum(0), g.double().abs().sum(0)
+    # a chain of at most m / 32 additions per thread, 64 row groups and 8 CTAs, each rounding to 2^-24 of the partial
+    # sum (below the sum of magnitudes); bf16 results round once more
+    bound = (m / 32 + 80) * 2.0 ** -24 * scale + (2.0 ** -8 * want.abs() if dtype == torch.bfloat16 else 0)
+    assert bool(((out[:n].double() - want).abs() <= bound).all())
+    assert bool((out[n:] == 7.0).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("m,k,tiles", [(1, 8, 1), (31, 72, 3), (33, 75, 2), (2500, 1024, 8)])
+def test_static_range_gradient_and_clipped_inputs(dtype, m, k, tiles):
+    from aihwkit_lightning_b200.nn import AnalogLinear
+    from aihwkit_lightning_b200.simulator.configs import TorchInferenceRPUConfig
+
+    rpu = TorchInferenceRPUConfig()
+    rpu.mapping.max_input_size = -(-k // tiles)
+    irp = rpu.pre_post.input_range
+    irp.enable, irp.dynamic, irp.learn_input_range, irp.init_value, irp.init_from_data = True, False, True, 1.5, 0
+    irp.decay = 0.0
+    torch.manual_seed(k)
+    layer = AnalogLinear(k, 16, bias=False, rpu_config=rpu).to(device="cuda", dtype=dtype).train()
+    x = torch.randn(m, k, device="cuda").to(dtype).requires_grad_(True)
+    g = torch.randn(m, 16, device="cuda").to(dtype)
+    layer(x).backward(g)
+    full = torch.empty(m, k, device="cuda", dtype=dtype)  # the gradient before the clipped entries were zeroed
+    full.copy_(g.float() @ layer.weight.float())
+    xd, clipped = x.detach().double(), x.detach().abs() >= 1.5
+    assert bool((x.grad[clipped & (x.detach().abs() != 1.5)] == 0).all())
+    assert bool((x.grad[~clipped] != 0).float().mean() > 0.9)
+    lo = 0
+    tol = 1e-5 if dtype == torch.float32 else 2e-2  # fp32 sums of products; bf16 gradients and results
+    for t, size in enumerate(layer.in_sizes):
+        cols = slice(lo, lo + size)
+        gx, xt = full[:, cols].double(), xd[:, cols]
+        want = 1.5 * (gx[xt >= 1.5].clamp(max=0).sum() - gx[xt <= -1.5].clamp(min=0).sum())
+        scale = 1.5 * gx[clipped[:, cols]].abs().sum() + 1e-6
+        assert abs(layer.input_range.grad[t].double() - want) <= tol * scale
+        lo += size
