@@ -30,7 +30,7 @@ class AlDesc(Structure):
         ("out_noise_per_channel", c_int32), ("noise_type", c_int32), ("quant_type", c_int32),
         ("std_dev", c_double), ("mod_res", c_double),
         ("clip_type", c_int32), ("no_rounding", c_int32), ("ref_rounding", c_int32),
-        ("engine", c_int32), ("save_for_backward", c_int32),
+        ("engine", c_int32), ("save_for_backward", c_int32), ("operand_pitch", c_int32),
     ]
 
 
@@ -80,6 +80,7 @@ SYMBOLS = {
     "al_backward_scratch_floats": (c_int64, [c_int32, c_int32, c_int32, c_int32]),
     "al_smallm_scratch_floats": (c_int64, [c_int32, c_int32, c_int32]),
     "al_backward_plane_elems": (c_int64, [POINTER(AlDesc), POINTER(c_int32)]),
+    "al_operand_pitch": (c_int32, [POINTER(AlDesc), POINTER(c_int32)]),
     "al_f32_planes": (c_int32, []),
     "al_clip_weights": (c_int32, [c_int32, c_void_p, c_int32, c_int32, c_int32, c_float, c_void_p, c_void_p]),
     "al_unfold2d": (c_int32, [c_int32, c_void_p] + [c_int32] * 12 + [c_void_p, c_void_p]),

@@ -317,6 +317,15 @@ def _analog_forward(ctx, inp, weight, bias, input_range, input_range_update_idx,
             args.learnable_weight_clip = _ptr(lwc)
         modifies = desc.quant_type != 0 or (training and desc.noise_type != 0) or learn_clip
         need_std = static and training and desc.init_from_data > 0
+        # sizes that are no multiples of 8: the tensor-core route takes its operands in a pitched layout (a layer whose
+        # pitch equals K reads x and w themselves where nothing modifies them: those must be aligned)
+        if (dtype == torch.bfloat16 and (n % 8 or k % 8 or in_sizes[0] % 8 or in_sizes[-1] % 8) and prequant is None
+                and settings.capture is None and settings.w_noise is None and settings.out_noise is None):
+            pitch = lib.al_operand_pitch(desc, ends)
+            if pitch != k or not (x2d.data_ptr() % 16 or w.data_ptr() % 16):
+                desc.operand_pitch = pitch
+        k_rows = desc.operand_pitch or k
+        pitched = k_rows != k
         few_rows = m <= 16 and not needs_grad and dtype == torch.bfloat16 and settings.capture is None
         xq = x2d
         ir_rows = w_amax = w_tile_max = keep_mask = None
@@ -328,10 +337,10 @@ def _analog_forward(ctx, inp, weight, bias, input_range, input_range_update_idx,
             # nothing of the workspace outlives the call: one allocation, carved by offset
             es = w.element_size()
             plan = [("w_amax", t * n * es), ("w_tile_max", 2 * t * 4)]
-            if desc.ir_mode != _lib.AL_IR_OFF and prequant is None:
-                plan += [("xq", m * k * es), ("ir_rows", (t if static else t * m) * es)]
-            if modifies:
-                plan.append(("w_mod", n * k * es))
+            if (desc.ir_mode != _lib.AL_IR_OFF or pitched) and prequant is None:
+                plan += [("xq", m * k_rows * es), ("ir_rows", (t if static else t * m) * es)]
+            if modifies or pitched:
+                plan.append(("w_mod", n * k_rows * es))
             if need_std:
                 plan.append(("std_scratch", lib.al_std_scratch_floats(m, t) * 4))
             if few_rows:
@@ -354,14 +363,14 @@ def _analog_forward(ctx, inp, weight, bias, input_range, input_range_update_idx,
         else:
             if prequant is not None:
                 xq, ir_rows = prequant[0], prequant[1]
-            elif desc.ir_mode != _lib.AL_IR_OFF:
-                xq = torch.empty_like(x2d)
+            elif desc.ir_mode != _lib.AL_IR_OFF or pitched:
+                xq = torch.empty(m, k_rows, device=dev, dtype=dtype)
                 ir_rows = torch.empty((t, m) if not static else (t,), device=dev, dtype=dtype)
             args.xq, args.ir_rows = _ptr(xq), _ptr(ir_rows)
             w_amax = torch.empty(t, n, device=dev, dtype=dtype)
             w_tile_max = torch.empty(2 * t, device=dev, dtype=torch.float32)
             args.w_amax, args.w_tile_max = _ptr(w_amax), _ptr(w_tile_max)
-            w_mod = torch.empty_like(w) if modifies else w
+            w_mod = torch.empty(n, k_rows, device=dev, dtype=dtype) if modifies or pitched else w
             args.w_mod = _ptr(w_mod)
             if desc.out_bound > 0 and needs_grad:
                 keep_mask = torch.empty(t, (n + 31) // 32, m, device=dev, dtype=torch.int32)
@@ -467,6 +476,9 @@ def _analog_backward(ctx, grad_out, skip_input_grad=False):
             g_planes = torch.empty(lib.al_backward_plane_elems(desc, ends), device=dev, dtype=torch.bfloat16)
             args.codes16, args.w_planes, args.g_planes = _ptr(codes16), _ptr(w_planes), _ptr(g_planes)
             args.g_planes_elems = g_planes.numel()
+        elif desc.operand_pitch and (n % 8 or g.data_ptr() % 16):
+            g_planes = torch.empty(m * ((n + 7) // 8 * 8), device=dev, dtype=dtype)  # rows TMA can address
+            args.g_planes, args.g_planes_elems = _ptr(g_planes), g_planes.numel()
         grad_clip = None
         if need_clip:
             grad_clip = torch.empty(t, n, device=dev, dtype=dtype)

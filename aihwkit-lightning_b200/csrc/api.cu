@@ -148,6 +148,13 @@ static bool needs_wmax(const Derived& dv) {
 }
 static size_t elem_size(int dtype) { return dtype == AL_BF16 ? 2 : 4; }
 
+// the pitched layout the caller announced must be the one the kernels assume
+static int check_ragged(const AlDesc& d, const TileTable& tt, RaggedTiles* rt) {
+  if (tc_ragged_supported(d, tt, rt) && d.operand_pitch == rt->T * rt->pitch) return AL_OK;
+  set_error("operand_pitch = %d is not al_operand_pitch() of this layer", d.operand_pitch);
+  return AL_ERR_BAD_ARGUMENT;
+}
+
 static bool pick_tc(const AlDesc& d, const TileTable& tt, bool backward) {
   if (d.engine == AL_ENGINE_SIMT) return false;
   return backward ? tc_backward_supported(d, tt) : tc_forward_supported(d, tt);
@@ -282,6 +289,14 @@ int64_t al_backward_plane_elems(const AlDesc* desc, const int32_t* tile_ends_hos
   return kPlanes * plane * (sets_d + sets_w);
 }
 
+int32_t al_operand_pitch(const AlDesc* desc, const int32_t* tile_ends_host) {
+  if (!desc) return 0;
+  TileTable tt;
+  RaggedTiles rt;
+  if (make_tile_table(tile_ends_host, desc->T, desc->K, &tt) || !tc_ragged_supported(*desc, tt, &rt)) return 0;
+  return rt.T * rt.pitch;
+}
+
 int al_forward(const AlDesc* desc, const AlForwardArgs* a, void* stream) {
   if (!desc || !a) {
     set_error("al_forward: null descriptor");
@@ -306,6 +321,21 @@ int al_forward(const AlDesc* desc, const AlForwardArgs* a, void* stream) {
   if ((!a->x && !prequantised) || !a->w || !a->out) {
     set_error("al_forward: x, w and out must be given");
     return AL_ERR_BAD_ARGUMENT;
+  }
+
+  // ragged layer on the tensor cores: xq and w_mod in the pitched layout
+  RaggedTiles rt;
+  const bool ragged = d.operand_pitch != 0;
+  // the pitched layout of a layer with only N ragged is the dense one: its operands come from the dense pre-passes
+  const bool pitched = ragged && d.operand_pitch != d.K;
+  if (ragged) {
+    rc = check_ragged(d, tt, &rt);
+    if (rc) return rc;
+    if (prequantised || a->w_noise || a->out_noise || a->codes ||
+        (pitched && (!a->xq || !a->w_mod || a->w_mod == a->w || a->xq == a->x))) {
+      set_error("al_forward: operand_pitch needs separate xq and w_mod; not with x_prequantised, replayed noise or codes");
+      return AL_ERR_BAD_ARGUMENT;
+    }
   }
 
   // 1. input range (static mode): optional init-from-data update, then copy the ranges used
@@ -387,6 +417,15 @@ int al_forward(const AlDesc* desc, const AlForwardArgs* a, void* stream) {
   SideStream* side = nullptr;  // non-null: forked, the weight pre-pass goes there
   if (prequantised) {
     xq = a->xq;
+  } else if (pitched) {
+    if (d.ir_mode == AL_IR_DYNAMIC && !a->ir_rows) {
+      set_error("al_forward: ir_rows workspace missing");
+      return AL_ERR_BAD_ARGUMENT;
+    }
+    rc = launch_dac_ragged(a->x, d.M, d.K, rt, d.ir_mode == AL_IR_FAST ? AL_IR_STATIC : d.ir_mode, ir_static,
+                           dv.has_dac ? dv.inp_res : -1.0f, d.no_rounding, a->xq, a->ir_rows, s);
+    if (rc) return rc;
+    xq = a->xq;
   } else if (d.ir_mode != AL_IR_OFF && !smallm_dac) {
     if (!a->xq || (d.ir_mode == AL_IR_DYNAMIC && !a->ir_rows)) {
       set_error("al_forward: xq / ir_rows workspace missing");
@@ -451,9 +490,12 @@ int al_forward(const AlDesc* desc, const AlForwardArgs* a, void* stream) {
     const int quant = dv.weight_quant == AL_QUANT_NONE ? kQuantLearnClamp : dv.weight_quant;
     rc = launch_tile_max(d.dtype, a->w_amax, d.N, tt, quant, dv.n_states, tile_max, flags, s);
     if (rc) return rc;
-    rc = launch_weight_modify(d.dtype, a->w, d.N, d.K, tt, a->w_amax, tile_max, flags, quant, dv.n_states,
-                              dv.max_state, dv.weight_noise, dv.std_dev, a->w_noise, a->seed, a->offset,
-                              d.no_rounding, a->w_mod, s, a->offset_base);
+    rc = pitched ? launch_weight_ragged(false, a->w, d.N, d.K, rt, a->w_amax, tile_max, flags, quant, dv.n_states,
+                                        dv.max_state, dv.weight_noise, dv.std_dev, a->seed, a->offset, d.no_rounding,
+                                        a->w_mod, s, a->offset_base)
+                 : launch_weight_modify(d.dtype, a->w, d.N, d.K, tt, a->w_amax, tile_max, flags, quant, dv.n_states,
+                                        dv.max_state, dv.weight_noise, dv.std_dev, a->w_noise, a->seed, a->offset,
+                                        d.no_rounding, a->w_mod, s, a->offset_base);
     if (rc) return rc;
     w_mod = a->w_mod;
   } else if (needs_wmax(dv)) {
@@ -470,9 +512,12 @@ int al_forward(const AlDesc* desc, const AlForwardArgs* a, void* stream) {
     }
     if (dv.weight_quant == AL_QUANT_NONE && dv.weight_noise != AL_NOISE_ADD_NORMAL) {
       // every scale the modifier needs is the segment's own abs-max: one sweep over w
-      rc = launch_weight_fused(d.dtype, a->w, d.N, d.K, tt, a->w_amax, tile_max, dv.weight_noise,
-                               dv.std_dev, a->w_noise, a->seed, a->offset, modifies ? a->w_mod : nullptr,
-                               side ? side->stream : s, a->offset_base, tile_max_zeroed);
+      rc = pitched ? launch_weight_ragged(true, a->w, d.N, d.K, rt, a->w_amax, tile_max, nullptr, AL_QUANT_NONE, 1.0f,
+                                          1.0f, dv.weight_noise, dv.std_dev, a->seed, a->offset, 0, a->w_mod, s,
+                                          a->offset_base)
+                   : launch_weight_fused(d.dtype, a->w, d.N, d.K, tt, a->w_amax, tile_max, dv.weight_noise,
+                                         dv.std_dev, a->w_noise, a->seed, a->offset, modifies ? a->w_mod : nullptr,
+                                         side ? side->stream : s, a->offset_base, tile_max_zeroed);
       if (side) {  // join, also after a failed launch: the caller's stream must not stay forked
         const cudaError_t ej = cudaEventRecord(side->join, side->stream);
         const cudaError_t ew = ej == cudaSuccess ? cudaStreamWaitEvent(s, side->join, 0) : ej;
@@ -489,14 +534,22 @@ int al_forward(const AlDesc* desc, const AlForwardArgs* a, void* stream) {
       rc = launch_tile_max(d.dtype, a->w_amax, d.N, tt, dv.weight_quant, dv.n_states, tile_max, flags, s);
       if (rc) return rc;
       if (modifies) {
-        rc = launch_weight_modify(d.dtype, a->w, d.N, d.K, tt, a->w_amax, tile_max, flags,
-                                  dv.weight_quant, dv.n_states, dv.max_state, dv.weight_noise,
-                                  dv.std_dev, a->w_noise, a->seed, a->offset, d.no_rounding, a->w_mod, s,
-                                  a->offset_base);
+        rc = pitched ? launch_weight_ragged(false, a->w, d.N, d.K, rt, a->w_amax, tile_max, flags, dv.weight_quant,
+                                            dv.n_states, dv.max_state, dv.weight_noise, dv.std_dev, a->seed, a->offset,
+                                            d.no_rounding, a->w_mod, s, a->offset_base)
+                     : launch_weight_modify(d.dtype, a->w, d.N, d.K, tt, a->w_amax, tile_max, flags,
+                                            dv.weight_quant, dv.n_states, dv.max_state, dv.weight_noise,
+                                            dv.std_dev, a->w_noise, a->seed, a->offset, d.no_rounding, a->w_mod, s,
+                                            a->offset_base);
         if (rc) return rc;
       }
     }
-    if (modifies) w_mod = a->w_mod;
+    if (modifies || pitched) w_mod = a->w_mod;
+  } else if (pitched) {
+    rc = launch_weight_ragged(true, a->w, d.N, d.K, rt, nullptr, nullptr, nullptr, AL_QUANT_NONE, 1.0f, 1.0f,
+                              AL_NOISE_NONE, 0.0f, 0, 0, 0, a->w_mod, s, nullptr);
+    if (rc) return rc;
+    w_mod = a->w_mod;
   }
 
   // 4. tiled GEMM with the per-tile output stage
@@ -526,6 +579,7 @@ int al_forward(const AlDesc* desc, const AlForwardArgs* a, void* stream) {
     if (rc) return rc;
     return launch_fwd_tc_f32(a->codes16, a->w_planes, d.K, tt, ep, dv.inp_res, a->out, s);
   }
+  if (ragged) return launch_fwd_tc_ragged(dv.round_dt, xq, w_mod, rt, ep, a->out, s);
   if (d.engine >= AL_ENGINE_TCGEN05 && !tc_forward_supported(d, tt)) {
     set_error("tcgen05 engine requested but the problem does not qualify (bf16, 16-byte aligned tiles)");
     return AL_ERR_UNSUPPORTED;
@@ -629,6 +683,24 @@ int al_backward(const AlDesc* desc, const AlBackwardArgs* a, void* stream) {
     return AL_ERR_UNSUPPORTED;
   }
   bool tc = !tc_f32 && pick_tc(d, tt, true);
+  RaggedTiles rt;
+  const bool ragged = d.operand_pitch != 0;
+  const void* g_rows = a->grad_out;  // ragged: rows of a multiple of 8 elements, 16-byte aligned
+  if (ragged) {
+    rc = check_ragged(d, tt, &rt);
+    if (rc) return rc;
+    if ((a->grad_x || a->grad_w) && (d.N % 8 != 0 || ((uintptr_t)a->grad_out % 16) != 0)) {
+      const int64_t need = (int64_t)d.M * ((d.N + 7) / 8 * 8);
+      if (!a->g_planes || a->g_planes_elems < need) {
+        set_error("al_backward: g_planes holds %lld elements, %lld needed", (long long)(a->g_planes ? a->g_planes_elems : 0),
+                  (long long)need);
+        return AL_ERR_BAD_ARGUMENT;
+      }
+      rc = launch_pitch_rows(a->grad_out, d.M, d.N, a->g_planes, s);
+      if (rc) return rc;
+      g_rows = a->g_planes;
+    }
+  }
   // an fp32 layer with fewer than 64 output channels: the input gradient reduces over those few channels
   // only, which the CUDA-core kernel does faster (52 against 76 us at 65536 x 288 x 32); it needs w_mod
   const bool dgrad_tc_f32 = tc_f32 && (d.N >= 64 || d.engine >= AL_ENGINE_TCGEN05 || !a->w_mod);
@@ -645,7 +717,8 @@ int al_backward(const AlDesc* desc, const AlBackwardArgs* a, void* stream) {
       set_error("al_backward: w_mod missing");
       return AL_ERR_BAD_ARGUMENT;
     }
-    rc = dgrad_tc_f32 ? launch_dgrad_tc_f32(a->g_planes, sets_d, a->w_planes, d.M, d.K, d.N, tt, pairing, a->grad_x, s)
+    rc = ragged ? launch_dgrad_tc_ragged(g_rows, a->w_mod, mask, mask_words, d.M, d.K, d.N, rt, a->grad_x, s)
+         : dgrad_tc_f32 ? launch_dgrad_tc_f32(a->g_planes, sets_d, a->w_planes, d.M, d.K, d.N, tt, pairing, a->grad_x, s)
          : tc   ? launch_dgrad_tc(a->grad_out, a->w_mod, mask, mask_words, d.M, d.K, d.N, gt, pairing, a->grad_x, s)
                 : launch_dgrad_simt(d.dtype, a->grad_out, a->w_mod, mask, mask_words, d.M, d.K, d.N, gt, a->grad_x, s);
     if (rc) return rc;
@@ -703,7 +776,8 @@ int al_backward(const AlDesc* desc, const AlBackwardArgs* a, void* stream) {
     const int64_t fixed = backward_reduce_floats(d.M, d.T);
     float* partial = a->reduce_scratch ? a->reduce_scratch + fixed : nullptr;
     const int64_t partial_capacity = a->reduce_scratch ? a->reduce_scratch_floats - fixed : 0;
-    rc = tc ? launch_wgrad_tc(a->grad_out, a->xq, mask, mask_words, d.M, d.K, d.N, gt, pairing, a->grad_w, s)
+    rc = ragged ? launch_wgrad_tc_ragged(g_rows, a->xq, mask, mask_words, d.M, d.K, d.N, rt, a->grad_w, s)
+         : tc ? launch_wgrad_tc(a->grad_out, a->xq, mask, mask_words, d.M, d.K, d.N, gt, pairing, a->grad_w, s)
             : launch_wgrad_simt(d.dtype, a->grad_out, a->xq, mask, mask_words, d.M, d.K, d.N, gt, d.T, partial,
                                 partial_capacity, a->grad_w, s);
     if (rc) return rc;

@@ -29,6 +29,30 @@ struct FwdTcParams {
   void* out;
 };
 
+constexpr int kRagStageWords = 32 * 9;
+constexpr int kRagStageBytes = F_EPI_WARPS * kRagStageWords * 4;
+
+// normals of elements idx .. idx + 15 of the output-noise stream (normal4's groups of four, any idx)
+__device__ __forceinline__ void normals16(uint64_t seed, uint64_t offset, uint64_t idx, float z[16]) {
+  float b[20];
+  const int r = (int)(idx & 3);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) normal4(seed, offset, 1u, (idx >> 2) + q, b + 4 * q);
+  if (r != 0) {
+    normal4(seed, offset, 1u, (idx >> 2) + 4, b + 16);
+    if (r & 1) {
+#pragma unroll
+      for (int i = 0; i < 19; ++i) b[i] = b[i + 1];
+    }
+    if (r & 2) {
+#pragma unroll
+      for (int i = 0; i < 18; ++i) b[i] = b[i + 2];
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 16; ++i) z[i] = b[i];
+}
+
 // MODE >= 0: the output stage is fixed at compile time (bit 0 output noise from the internal
 // generator, bit 1 ADC quantisation, bit 2 clamp; reference rounding, per-tile scalar scales,
 // rounding on, small ADC codes).  MODE < 0: every switch is read at run time.
@@ -46,10 +70,14 @@ struct FwdTcParams {
 // leader.
 //
 // IO: element type of the layer's tensors (input ranges, bias, replayed noise, per-channel scales,
-// outputs).  IO = fp32: the A operand holds the DAC codes as bf16 integers and the weights come as
+// outputs).  RAG: the row pitch of the outputs is no multiple of 8 (single CTAs, run-time output stage only): the
+// output noise is addressed element by element -- with the generator of the CUDA-core GEMM, so that a layer draws the
+// same noise on either engine -- and the outputs leave through a staging buffer, two rows of 16 columns per store,
+// because a thread's own 16 columns start at no particular alignment (1000 x 2500 x 1500 with noise and ADC: 361 us on
+// the CUDA cores, 43 us here).  IO = fp32: the A operand holds the DAC codes as bf16 integers and the weights come as
 // bf16 planes (fourth dimension of their tensor map) that are accumulated one after the other;
 // the output stage multiplies the accumulator by the DAC step of its (row, tile) first.
-template <int RD, int MODE, bool PAIR, int IO = kBF16>
+template <int RD, int MODE, bool PAIR, int IO = kBF16, bool RAG = false>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 fwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
               const FwdTcParams p) {
@@ -64,6 +92,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
   uint8_t* sum_base = stage_base + kStages * kStageBytes;      // PAIR: [128 rows][256 bf16], 16-byte chunks swizzled
   Barriers* bars = reinterpret_cast<Barriers*>(sum_base + kSumBytes);
   volatile uint32_t* abort_flag = &bars->abort_flag;
+  static_assert(!RAG || (MODE < 0 && !PAIR && IO == kBF16), "ragged outputs: run-time output stage on single CTAs");
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const FwdEpilogueParams& ep = p.ep;
@@ -361,7 +390,10 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
             keep_bits |= ((kept | (kept >> 16)) & 0xffffu) << ((h & 1) * 16);
           } else {
           float z[16];
-          if (noise_now) {
+          if (RAG && noise_now) {
+            normals16(ep.seed, ep.offset + (ep.offset_base != nullptr ? *ep.offset_base : 0ull),
+                      ((uint64_t)t * M + (row_ok ? m : 0)) * N + nh, z);
+          } else if (noise_now) {
 #pragma unroll
             for (int g8 = 0; g8 < 2; ++g8) {
               const int nq = nh + g8 * 8;
@@ -478,6 +510,37 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
             } else {
               tmem_st16(tmem_base + lane_base + (uint32_t)(2 * F_BN + cc), sumr);
             }
+          } else if (RAG) {
+            // final (ragged outputs): bias, convert, transpose through this warp's staging buffer
+            uint32_t* const st = reinterpret_cast<uint32_t*>(bars + 1) + (warp - 4) * kRagStageWords;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              float b0 = 0.0f, b1 = 0.0f;
+              if (ep.bias) {
+                if (nh + 2 * e < N) b0 = Elem<kBF16>::load(ep.bias, nh + 2 * e);
+                if (nh + 2 * e + 1 < N) b1 = Elem<kBF16>::load(ep.bias, nh + 2 * e + 1);
+              }
+              uint32_t w;
+              if (packed) {
+                w = ep.bias ? as_u32(__hadd2_rn(as_bf162(sumr[e]), __floats2bfloat162_rn(b0, b1))) : sumr[e];
+              } else {
+                float f0 = __uint_as_float(sumr[2 * e]), f1 = __uint_as_float(sumr[2 * e + 1]);
+                if (ep.bias) {
+                  f0 = fadd(rnd<RD>(f0), b0);
+                  f1 = fadd(rnd<RD>(f1), b1);
+                }
+                w = pack_bf16x2_rn(f0, f1);
+              }
+              st[lane * 9 + e] = w;  // nine words a row: the rows of a warp start on different banks
+            }
+            __syncwarp();
+            const int m_first = mb * kBlockRows + quad * 32, col = lane & 15;
+#pragma unroll 4
+            for (int rr = lane >> 4; rr < 32; rr += 2)
+              if (m_first + rr < M && nh + col < N)
+                reinterpret_cast<uint16_t*>(p.out)[(int64_t)(m_first + rr) * N + nh + col] =
+                    reinterpret_cast<const uint16_t*>(st + rr * 9)[col];
+            __syncwarp();
           } else if (row_ok && IO == kF32) {
             // final (fp32 layer): bias, store 16 floats of this row
             float* dst = reinterpret_cast<float*>(p.out) + (int64_t)m * N + nh;
@@ -574,6 +637,13 @@ static FwdKernel pick_fwd_kernel(int mode, int round_dt) {
   }
 }
 
+static int small_adc_codes(int tile_w, const FwdEpilogueParams& ep) {
+  // |o| <= tile_w * ir * wmax * (1 + noise) and step = 2 * out_bound * ir * wmax / states
+  const double states = ep.out_res > 1.0f ? ep.out_res : (ep.out_res > 0.0f ? 1.0 / ep.out_res : 1.0);
+  const double max_code = 8.0 * (double)tile_w * states / (2.0 * (ep.out_bound > 0.0f ? ep.out_bound : 1.0));
+  return max_code < 274877906944.0 ? 1 : 0;  // 2^38
+}
+
 // how many CTA pairs of the forward kernel the device runs at once (0: it cannot)
 static int max_fwd_pairs(FwdKernel kernel, int smem) {
   static FwdKernel seen[24];
@@ -612,12 +682,7 @@ int launch_fwd_tc(int round_dt, const void* xq, const void* w_mod, int K, const 
   p.out = out;
   p.planes_b = 1;
   p.inp_res = 0.0f;
-  {
-    // |o| <= tile_w * ir * wmax * (1 + noise) and step = 2 * out_bound * ir * wmax / states
-    double states = ep.out_res > 1.0f ? ep.out_res : (ep.out_res > 0.0f ? 1.0 / ep.out_res : 1.0);
-    double max_code = 8.0 * (double)w * states / (2.0 * (ep.out_bound > 0.0f ? ep.out_bound : 1.0));
-    p.small_adc_codes = max_code < 274877906944.0 ? 1 : 0;  // 2^38
-  }
+  p.small_adc_codes = small_adc_codes(w, ep);
   const bool per_channel = ep.w_amax != nullptr && (ep.noise_pc || ep.bound_pc);
   // the compile-time output stages quantise in packed bf16 arithmetic, which needs every ADC code
   // beyond +-127 to end on the clamp (up to 254 states: the 8-bit converter and below)
@@ -677,6 +742,59 @@ int launch_fwd_tc(int round_dt, const void* xq, const void* w_mod, int K, const 
   int grid = tiles < sm_count() ? tiles : sm_count();
   kernel<<<grid, kFwdThreads, F_SMEM, s>>>(map_a, map_b, p);
   return check_launch("fwd_tc");
+}
+
+// Ragged bf16 layers (tile widths, K or N no multiples of 8; operands in the pitched layout).  Measured on B200 against
+// the CUDA-core kernels, device time of an evaluation and of forward + backward in us (CUDA cores -> here):
+//   1000 x 2500 x 1500 train (tiles of 500)  1152 -> 122     1 x 1000 x 777      79 -> 25, 150 -> 54
+//   333 x 1000 x 777 evaluation                99 -> 25     64 x 300 x 100       40 -> 20,  65 -> 49
+//   16 x 4001 x 4001                          408 -> 66     32 x 70 x 70         25 -> 18,  42 -> 36
+//   100 x 2000 x 20 (tiles of 20)            1039 -> 261    8000 x 100 x 10      36 -> 22, 125 -> 97
+// so there is no lower size.  Three lines: tiles narrower than 8 columns would be mostly padding; tiles that are not as
+// even as possible have no closed-form start (no module makes them); and the weight gradient here does not split its
+// reduction over the rows, so a layer of few output blocks leaves from 8192 rows on.
+bool tc_ragged_supported(const AlDesc& d, const TileTable& tt, RaggedTiles* rt) {
+  if (d.dtype != AL_BF16 || d.engine != AL_ENGINE_AUTO || tc_tiling_ok(d, tt) || !ragged_tiles(tt, rt)) return false;
+  const int64_t blocks = (int64_t)((d.N + BM - 1) / BM) * rt->T * ((rt->widest() + B_BN - 1) / B_BN);
+  if (rt->widest() < 8 || (d.M > 8192 && blocks < 37)) return false;
+  return (int64_t)rt->T * rt->pitch < (1ll << 31);
+}
+
+int launch_fwd_tc_ragged(int round_dt, const void* xq, const void* w_mod, const RaggedTiles& rt,
+                         const FwdEpilogueParams& ep, void* out, cudaStream_t s) {
+  ProfScope prof(AL_K_FWD_GEMM, s);
+  if (!aligned16(xq) || !aligned16(w_mod)) {
+    set_error("fwd_tc_ragged: operands must be 16-byte aligned");
+    return AL_ERR_UNSUPPORTED;
+  }
+  FwdTcParams p;
+  p.tile_w = rt.widest();
+  p.ksteps = (p.tile_w + BK - 1) / BK;
+  p.num_mb = (ep.M + BM - 1) / BM;
+  p.num_nb = (ep.N + F_BN - 1) / F_BN;
+  p.planes_b = 1;
+  p.inp_res = 0.0f;
+  p.ep = ep;
+  p.noise = make_noise_keys(ep.seed, ep.offset, 1u, ep.offset_base);
+  p.out = out;
+  p.small_adc_codes = small_adc_codes(p.tile_w, ep);
+  FwdKernel kernel = round_dt == AL_BF16 ? fwd_tc_kernel<kBF16, -1, false, kBF16, true>
+                                         : fwd_tc_kernel<kF32, -1, false, kBF16, true>;
+  const int smem = F_SMEM + kRagStageBytes;
+  int rc = ensure_smem(kernel, smem);
+  if (rc) return rc;
+  CUtensorMap map_a, map_b;
+  const uint64_t row_bytes = (uint64_t)rt.T * rt.pitch * 2;
+  for (int b = 0; b < 2; ++b) {
+    uint64_t dims[3] = {(uint64_t)p.tile_w, (uint64_t)rt.T, (uint64_t)(b ? ep.N : ep.M)};
+    uint64_t strides[2] = {(uint64_t)rt.pitch * 2, row_bytes};
+    uint32_t box[3] = {BK, 1, (uint32_t)(b ? F_BN : BM)};
+    rc = make_map(b ? &map_b : &map_a, b ? w_mod : xq, 3, dims, strides, box);
+    if (rc) return rc;
+  }
+  const int tiles = p.num_mb * p.num_nb;
+  kernel<<<tiles < sm_count() ? tiles : sm_count(), kFwdThreads, smem, s>>>(map_a, map_b, p);
+  return check_launch("fwd_tc_ragged");
 }
 
 // fp32 with the DAC on and integer codes of at most 9 bits (exact in bf16), tiles as for bf16

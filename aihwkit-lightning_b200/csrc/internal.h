@@ -19,6 +19,15 @@ struct TileTable {
   __host__ __device__ int hi(int t) const { return ends[t]; }
 };
 
+// Tiles as even as possible (the first `extra` one column wider than `base`, the others `base` wide) whose operands
+// are laid out `pitch` columns apart: the layout of layers with sizes TMA cannot address (ragged_kernels.cu).
+struct RaggedTiles {
+  int32_t T, base, extra, pitch;
+  __host__ __device__ int lo(int t) const { return t * base + (t < extra ? t : extra); }
+  __host__ __device__ int width(int t) const { return base + (t < extra ? 1 : 0); }
+  __host__ __device__ int widest() const { return base + (extra > 0 ? 1 : 0); }
+};
+
 // Host-side derived constants of a forward/backward call (double -> float narrowing happens
 // here, once, the way the Python reference narrows its scalars).
 struct Derived {
@@ -120,6 +129,19 @@ int launch_weight_fused(int dtype, const void* w, int N, int K, const TileTable&
                         uint64_t seed, uint64_t offset, void* w_mod, cudaStream_t s,
                         const uint64_t* offset_base = nullptr, bool tile_max_zeroed = false);
 
+// ---- operands in the pitched layout of ragged bf16 layers (ragged_kernels.cu) ----------------
+// false: the widths are not as even as possible (out is then undefined)
+bool ragged_tiles(const TileTable& tt, RaggedTiles* out);
+int launch_dac_ragged(const void* x, int M, int K, const RaggedTiles& rt, int ir_mode, const void* ir_static,
+                      float inp_res, int no_rounding, void* xq, void* ir_rows, cudaStream_t s);
+// fused: launch_weight_fused (w_amax / tile_max are outputs, tile_max may be null); else launch_weight_modify
+int launch_weight_ragged(bool fused, const void* w, int N, int K, const RaggedTiles& rt, void* w_amax, float* tile_max,
+                         const int32_t* flags, int quant_type, float n_states, float max_state, int noise_type,
+                         float std_dev, uint64_t seed, uint64_t offset, int no_rounding, void* out, cudaStream_t s,
+                         const uint64_t* offset_base);
+// dst[M][N rounded up to 8] = src[M][N], zeros behind
+int launch_pitch_rows(const void* src, int M, int N, void* dst, cudaStream_t s);
+
 // ---- SIMT GEMMs (gemm_simt.cu) ------------------------------------------------------------
 // c_out[e] = sum over s of partial[s][e], e < count, added in the order of s
 int launch_sum_partials(int dtype, const float* partial, int splits, int64_t count, void* c_out, cudaStream_t s);
@@ -165,6 +187,14 @@ bool tc_forward_supported(const AlDesc& d, const TileTable& tt);
 // pairing: 0 = CTA pairs when they fill the machine, 1 = always pairs, -1 = never
 int launch_fwd_tc(int round_dt, const void* xq, const void* w_mod, int K, const TileTable& tt,
                   const FwdEpilogueParams& ep, int pairing, void* out, cudaStream_t s);
+// Ragged bf16 layers: operands as written by the launchers of ragged_kernels.cu
+bool tc_ragged_supported(const AlDesc& d, const TileTable& tt, RaggedTiles* rt);
+int launch_fwd_tc_ragged(int round_dt, const void* xq, const void* w_mod, const RaggedTiles& rt,
+                         const FwdEpilogueParams& ep, void* out, cudaStream_t s);
+int launch_dgrad_tc_ragged(const void* g, const void* w_mod, const uint32_t* keep_mask, int mask_words, int M, int K,
+                           int N, const RaggedTiles& rt, void* grad_x, cudaStream_t s);
+int launch_wgrad_tc_ragged(const void* g, const void* xq, const uint32_t* keep_mask, int mask_words, int M, int K,
+                           int N, const RaggedTiles& rt, void* grad_w, cudaStream_t s);
 bool tc_backward_supported(const AlDesc& d, const TileTable& tt);
 void tc_pair_work_item(int num_work, int n_pairs, int item, int* total, int* block, int* half);
 // pairing: 0 = CTA pairs when they fill the machine, 1 = always pairs, -1 = never

@@ -92,6 +92,12 @@ typedef struct AlDesc {
   int32_t ref_rounding;      /* bf16: round to bf16 after every op like the reference does */
   int32_t engine;            /* AlEngine                                                    */
   int32_t save_for_backward; /* write `keep_mask` (forward) so that al_backward can run     */
+  int32_t operand_pitch;     /* 0: xq and w_mod are dense.  Otherwise al_operand_pitch() of the layer, the same
+                                 in the forward and the backward call: xq and w_mod hold that many
+                                 elements per row (separate from x and w unless the pitch is K), the GEMMs run
+                                 on the tensor cores, and the backward takes g_planes as a workspace of
+                                 g_planes_elems >= M * (N rounded up to 8) bf16 elements unless N is a
+                                 multiple of 8.  Not with x_prequantised, replayed noise or `codes` */
 } AlDesc;
 
 /*
@@ -245,6 +251,9 @@ int al_pair_work_item(int32_t num_blocks, int32_t n_pairs, int32_t item, int32_t
 int64_t al_backward_plane_elems(const AlDesc* desc, const int32_t* tile_ends_host);
 /* Number of bf16 planes an fp32 operand is split into for the tensor cores (first dimension of w_planes). */
 int32_t al_f32_planes(void);
+/* Elements per row of xq and w_mod with which a bf16 layer whose sizes are no multiples of 8 runs on the tensor
+ * cores (every analog tile padded to a multiple of 8 columns); 0 when the layer takes the dense layout. */
+int32_t al_operand_pitch(const AlDesc* desc, const int32_t* tile_ends_host);
 /* floats of AlForwardArgs.smallm_scratch; 0 when the problem has more than 16 rows */
 int64_t al_smallm_scratch_floats(int32_t M, int32_t N, int32_t T);
 

@@ -1,0 +1,146 @@
+"""bf16 layers whose sizes are no multiples of 8 on the tensor cores, against the CUDA-core GEMMs of the same layer:
+the operands of the two (DAC output, modified weights, noise included) are the same bits, laid out differently."""
+import pytest
+import torch
+
+from util import rel_fro
+
+pytestmark = pytest.mark.gpu
+
+# One bf16 rounding per tile and per partial sum separates two orders of the same fp32 sum (2^-9 relative each), and
+# a share of the ADC codes moves by one level: the bar of every other bf16 comparison of this repository.
+BF16_REL = 1e-2
+
+SHAPES = [
+    # rows, K, N, tile: what is at the edge
+    (333, 1000, 777, 512),    # tiles of 500, odd N
+    (65, 2049, 513, 512),     # uneven tiles (410 and 409), one row and one column beyond a block
+    (128, 2048, 130, 256),    # K aligned: the pitched layout is the dense one
+    (200, 777, 512, -1),      # one tile of 777, N aligned
+    (32, 4100, 1030, -1),     # a tile wider than a warp keeps in registers
+    (1000, 2500, 1500, 512),
+    (300, 1001, 67, 77),      # 13 narrow tiles of 77, few channels
+    (1, 70, 9, 35),           # the smallest calls: one row, a few channels, tiles narrower than a k-step
+]
+OPTIONS = {
+    "train": dict(dynamic=True, adc=True, noise=True, discretize=False, learn_clip=False),
+    "no_adc": dict(dynamic=True, adc=False, noise=True, discretize=False, learn_clip=False),
+    "static_discretize": dict(dynamic=False, adc=True, noise=True, discretize=True, learn_clip=False),
+    "plain": dict(dynamic=False, adc=False, noise=False, discretize=False, learn_clip=False),
+    "learn_clip": dict(dynamic=True, adc=True, noise=False, discretize=False, learn_clip=True),
+}
+
+
+def _layer(k, n, tile, o):
+    from aihwkit_lightning_b200.nn import AnalogLinear
+    from aihwkit_lightning_b200.simulator.configs import TorchInferenceRPUConfig
+    from aihwkit_lightning_b200.simulator.enums import (WeightClipType, WeightNoiseInjectionType,
+                                                        WeightQuantizationType)
+
+    rpu = TorchInferenceRPUConfig()
+    rpu.mapping.max_input_size = tile
+    rpu.forward.inp_res = 254.0
+    if o["adc"]:
+        rpu.forward.out_res, rpu.forward.out_bound = 254.0, 10.0
+    irp = rpu.pre_post.input_range
+    irp.enable, irp.dynamic = True, o["dynamic"]
+    if not o["dynamic"]:
+        irp.learn_input_range, irp.init_value, irp.init_from_data = True, 2.5, 0
+    if o["noise"]:
+        rpu.forward.out_noise = 0.04
+        rpu.modifier.noise_type, rpu.modifier.std_dev = WeightNoiseInjectionType.ADD_NORMAL_PER_CHANNEL, 0.02
+    if o["discretize"]:
+        rpu.modifier.quantization_type, rpu.modifier.res = WeightQuantizationType.DISCRETIZE_PER_CHANNEL, 254.0
+    if o["learn_clip"]:
+        rpu.clip.type = WeightClipType.LEARNABLE_PER_CHANNEL
+    torch.manual_seed(3)
+    return AnalogLinear(k, n, bias=True, rpu_config=rpu, device="cuda", dtype=torch.bfloat16)
+
+
+def _pass(layer, x, g, engine):
+    from aihwkit_lightning_b200.nn import functional as F
+
+    x = x.detach().clone().requires_grad_(True)
+    layer.zero_grad()
+    torch.cuda.manual_seed(11)
+    with F.operator_settings(engine=engine):
+        out = layer(x)
+        node = out.grad_fn
+        while not hasattr(node, "saved_tensors") or len(node.saved_tensors) < 9:  # the layer's own node
+            node = node.next_functions[0][0]
+        xq, w_mod = node.saved_tensors[1:3]
+        out.backward(g)
+    return out.detach(), x.grad, {n: p.grad for n, p in layer.named_parameters() if p.grad is not None}, xq, w_mod
+
+
+def _dense(t, in_sizes):
+    """The tiles of a pitched operand side by side; its padding must be zero."""
+    pitch = t.shape[1] // len(in_sizes)
+    parts = t.view(t.shape[0], len(in_sizes), pitch)
+    for i, width in enumerate(in_sizes):
+        assert not parts[:, i, width:].any()
+    return torch.cat([parts[:, i, :width] for i, width in enumerate(in_sizes)], dim=1)
+
+
+@pytest.mark.parametrize("name", OPTIONS)
+@pytest.mark.parametrize("shape", SHAPES, ids=lambda s: "x".join(map(str, s)))
+def test_ragged_layer_matches_cuda_cores(shape, name):
+    rows, k, n, tile = shape
+    layer = _layer(k, n, tile, OPTIONS[name])
+    layer.train()
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    x = torch.randn(rows, k, device="cuda", generator=gen, dtype=torch.float32).bfloat16()
+    g = torch.randn(rows, n, device="cuda", generator=gen, dtype=torch.float32).bfloat16()
+    out, gx, grads, xq, w_mod = _pass(layer, x, g, "auto")
+    out_s, gx_s, grads_s, xq_s, w_mod_s = _pass(layer, x, g, "simt")
+    torch.cuda.synchronize()
+    assert (xq.shape[1] != k) == (k % 8 != 0 or any(w % 8 for w in layer.in_sizes))  # the pitched route was taken
+    assert torch.equal(_dense(xq, layer.in_sizes), xq_s)
+    assert torch.equal(_dense(w_mod, layer.in_sizes), w_mod_s)
+    assert rel_fro(out, out_s) <= BF16_REL
+    assert rel_fro(gx, gx_s) <= BF16_REL
+    assert grads.keys() == grads_s.keys()
+    for key in grads:
+        assert rel_fro(grads[key], grads_s[key]) <= BF16_REL, key
+    layer.eval()
+    with torch.no_grad():
+        from aihwkit_lightning_b200.nn import functional as F
+
+        ev = layer(x)
+        with F.operator_settings(engine="simt"):
+            ev_s = layer(x)
+    assert rel_fro(ev, ev_s) <= BF16_REL
+
+
+def test_ragged_layer_unaligned_inputs_and_gradients():
+    """Views that start two bytes into an allocation: the sources of the pitched layout have no alignment."""
+    rows, k, n = 130, 1001, 515
+    layer = _layer(k, n, 512, OPTIONS["train"])
+    layer.train()
+    x = torch.randn(rows * k + 1, device="cuda").bfloat16()[1:].view(rows, k)
+    g = torch.randn(rows * n + 1, device="cuda").bfloat16()[1:].view(rows, n)
+    a, b = _pass(layer, x, g, "auto"), _pass(layer, x, g, "simt")
+    assert rel_fro(a[0], b[0]) <= BF16_REL and rel_fro(a[1], b[1]) <= BF16_REL
+    assert rel_fro(a[2]["weight"], b[2]["weight"]) <= BF16_REL
+
+
+def test_operand_pitch_is_checked_on_the_host():
+    from aihwkit_lightning_b200 import _lib
+    from aihwkit_lightning_b200.nn import functional as F
+
+    lib = _lib.load()
+    layer = _layer(1001, 515, 512, OPTIONS["train"])
+    ends = _lib.tile_ends_array(layer.in_sizes)
+    desc = F.make_desc(layer.rpu_config, 130, 1001, 515, 2, torch.bfloat16, False)
+    assert lib.al_operand_pitch(desc, ends) == 2 * 504
+    with F.operator_settings(engine="simt"):
+        other = F.make_desc(layer.rpu_config, 130, 1001, 515, 2, torch.bfloat16, False)
+    assert lib.al_operand_pitch(other, ends) == 0  # another engine: the dense layout
+    tall = F.make_desc(layer.rpu_config, 8193, 1001, 515, 2, torch.bfloat16, False)
+    assert lib.al_operand_pitch(tall, ends) == 0   # 5 x 4 blocks of the weight gradient, a long reduction
+    desc.operand_pitch = 1008 + 8
+    args = _lib.AlForwardArgs()
+    buf = torch.zeros(4 << 20, device="cuda", dtype=torch.uint8)
+    args.x = args.w = args.out = args.xq = args.w_mod = args.ir_rows = buf.data_ptr()
+    args.tile_ends = ends
+    assert lib.al_forward(desc, args, None) != _lib.AL_OK
