@@ -5,7 +5,7 @@
 // dimension as MN-major tiles), groups of four warps apply the ADC clamp mask of the analog tile
 // to the staged gradient tile, tcgen05.mma accumulates in tensor memory, four warps drain it.
 // Large problems run on CTA pairs (256 x 256 blocks, cta_group::2, six stages), small ones on
-// single CTAs (128 x 256 blocks, four stages).
+// single CTAs (128 x 256, 128 x 128 or 128 x 64 blocks, four to eight stages).
 #include "tcgen05_common.cuh"
 
 namespace al {
@@ -23,6 +23,7 @@ struct BwdTcParams {
   int32_t T;           // analog tiles that carry their own mask (1 when there is no mask)
   int32_t tile_w;      // width of a tile (K when there is no mask)
   int32_t num_ib, num_jb, lsteps;
+  int32_t a_rows;      // input gradient on single CTAs: rows a copy of A brings (fewer than 128 when M is smaller)
   const uint32_t* keep_mask;
   int32_t mask_words;
   void* c_out;
@@ -125,13 +126,15 @@ __device__ __forceinline__ void rewrite_row_masked(uint32_t row_addr, int sw, ui
   }
 }
 
-template <bool WGRAD, bool RAG = false>
+// BN: columns of a block (pick_blocks)
+template <bool WGRAD, bool RAG, int BN>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 bwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
               const BwdTcParams p) {
+  constexpr int kStages = bwd_stages(BN), kStageBytes = bwd_stage_bytes(BN);
   extern __shared__ uint8_t smem_raw[];
   uint8_t* stage_base = align_1024(smem_raw);
-  Barriers* bars = reinterpret_cast<Barriers*>(stage_base + B_STAGES * B_STAGE_BYTES);
+  Barriers* bars = reinterpret_cast<Barriers*>(stage_base + kStages * kStageBytes);
   volatile uint32_t* abort_flag = &bars->abort_flag;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -141,7 +144,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
   const int num_work = per_split * p.splits;  // item w: copy w / per_split of output block w % per_split
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < B_STAGES; ++s) {
+    for (int s = 0; s < kStages; ++s) {
       mbar_init(&bars->full[s], 1);
       mbar_init(&bars->ready[s], B_XFORM_THREADS / 32);
       mbar_init(&bars->empty[s], 1);
@@ -172,22 +175,22 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
         const int ib = blk / (p.T * p.num_jb);
         const int rem = blk % (p.T * p.num_jb);
         const int t = rem / p.num_jb, jb = rem % p.num_jb;
-        const int j0 = t * p.tile_w + jb * B_BN;
+        const int j0 = t * p.tile_w + jb * BN;
         const int ls0 = sp * p.split_lsteps, ls1 = min(ls0 + p.split_lsteps, p.lsteps);
         for (int q = 0; q < p.products && ok; ++q) {
           const int plane_a = p.pa[q] + t * p.a_planes_per_tile, plane_b = p.pb[q];
           for (int ls = ls0; ls < ls1; ++ls, ++it) {
-            const int s = it % B_STAGES;
-            const uint32_t ph = (it / B_STAGES) & 1u;
+            const int s = it % kStages;
+            const uint32_t ph = (it / kStages) & 1u;
             if (!mbar_wait(&bars->empty[s], ph ^ 1u, abort_flag)) {
               raise_error(kErrProducer, abort_flag);
               ok = false;
               break;
             }
-            uint8_t* sa = stage_base + s * B_STAGE_BYTES;
+            uint8_t* sa = stage_base + s * kStageBytes;
             uint8_t* sb = sa + B_A_BYTES;
             const int l0 = ls * BK;
-            mbar_expect_tx(&bars->full[s], B_STAGE_BYTES);
+            mbar_expect_tx(&bars->full[s], (uint32_t)(WGRAD ? kStageBytes : kStageBytes - B_A_BYTES + p.a_rows * BK * 2));
             if (WGRAD) {
               // A = g^T: two MN-major boxes [64 rows of m] x [64 n]
               tma_load_3d(sa, &map_a, &bars->full[s], ib * BM, l0, plane_a);
@@ -197,15 +200,15 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
               tma_load_3d(sa, &map_a, &bars->full[s], l0, ib * BM, plane_a);
             }
 #pragma unroll
-            for (int c = 0; c < B_BN / 64; ++c)
+            for (int c = 0; c < BN / 64; ++c)
               tma_load_3d(sb + c * B_BOX_BYTES, &map_b, &bars->full[s], j0 + c * 64, l0, plane_b);
           }
         }
       }
-      const uint32_t n_back = it < (uint32_t)B_STAGES ? it : (uint32_t)B_STAGES;
+      const uint32_t n_back = it < (uint32_t)kStages ? it : (uint32_t)kStages;
       for (uint32_t j = it - n_back; j < it; ++j) {
-        const int s = j % B_STAGES;
-        const uint32_t ph = (j / B_STAGES) & 1u;
+        const int s = j % kStages;
+        const uint32_t ph = (j / kStages) & 1u;
         uint64_t t0 = globaltimer_ns();
         while (!mbar_try(&bars->full[s], ph)) {
           if (globaltimer_ns() - t0 > wait_limit_ns()) {
@@ -218,7 +221,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
   } else if (warp == 1) {
     // ---- MMA issuer --------------------------------------------------------------------
     if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc(BM, B_BN, WGRAD ? 1 : 0, 1);
+      constexpr uint32_t idesc = make_idesc(BM, BN, WGRAD ? 1 : 0, 1);
       uint32_t it = 0, acc_it = 0;
       bool ok = true;
       for (int w = blockIdx.x; w < num_work && ok; w += gridDim.x, ++acc_it) {
@@ -238,10 +241,10 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
         const int steps = nls * p.products;  // every plane product runs over the whole range
         for (int ls = 0; ls < steps; ++ls, ++it) {
           const bool cross = split_acc && ls >= nls;
-          const uint32_t d_tmem = tmem_base + (uint32_t)((cross ? 1 : b) * B_BN);
+          const uint32_t d_tmem = tmem_base + (uint32_t)((cross ? 1 : b) * BN);
           const bool first = ls == 0 || (split_acc && ls == nls);
-          const int s = it % B_STAGES;
-          const uint32_t ph = (it / B_STAGES) & 1u;
+          const int s = it % kStages;
+          const uint32_t ph = (it / kStages) & 1u;
           // the transform warps vouch for a stage on `ready` before its copy has landed when
           // the stage has nothing to zero, so both barriers gate the MMA
           if (!mbar_wait(&bars->full[s], ph, abort_flag) ||
@@ -251,7 +254,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
             break;
           }
           tc_fence_after();
-          const uint32_t sa = smem_u32(stage_base + s * B_STAGE_BYTES);
+          const uint32_t sa = smem_u32(stage_base + s * kStageBytes);
           const uint32_t sb = sa + B_A_BYTES;
           const uint64_t da = WGRAD ? desc_mn_major(sa, B_BOX_BYTES) : desc_k_major(sa);
           const uint64_t db = desc_mn_major(sb, B_BOX_BYTES);
@@ -285,7 +288,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
       const int ib = blk / (p.T * p.num_jb);
       const int rem = blk % (p.T * p.num_jb);
       const int t = rem / p.num_jb, jb = rem % p.num_jb;
-      const int j0 = t * p.tile_w + jb * B_BN;
+      const int j0 = t * p.tile_w + jb * BN;
       const int j_end = RAG ? t * p.tile_w + p.rt.width(t) : min((t + 1) * p.tile_w, p.K);
       const int i = ib * BM + quad * 32 + lane;
       void* const c_dst = p.splits > 1 ? static_cast<void*>(p.partial + (int64_t)sp * p.I * p.K) : p.c_out;
@@ -300,13 +303,13 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
       tc_fence_after();
       const float c_scale = p.c_scale_ir != nullptr ? quant_step<kF32>(p.c_scale_ir[t], p.inp_res) : 1.0f;
 #pragma unroll 1
-      for (int c = 0; c < B_BN / 32; ++c) {
+      for (int c = 0; c < BN / 32; ++c) {
         const int jc = j0 + c * 32;
         if (jc >= j_end) break;  // uniform across the warp
         uint32_t r[32];
-        tmem_ld32(tmem_base + lane_base + (uint32_t)(b * B_BN + c * 32), r);
+        tmem_ld32(tmem_base + lane_base + (uint32_t)(b * BN + c * 32), r);
         tmem_wait_ld();
-        if (split_acc) add_cross_terms(tmem_base + lane_base + (uint32_t)(B_BN + c * 32), r);
+        if (split_acc) add_cross_terms(tmem_base + lane_base + (uint32_t)(BN + c * 32), r);
         if (RAG)
           store_c_ragged(c_dst, p.K, i - lane, p.I, p.rt.lo(t) + jc - t * p.tile_w, min(32, j_end - jc), r,
                          reinterpret_cast<uint32_t*>(bars + 1) + quad * kRagStageWords, lane);
@@ -373,8 +376,8 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
     const int sw = r & 7;  // 128-byte swizzle: 16-byte chunk index is XORed with row % 8
     // one stage-iteration of this thread's row; false = the wait gave up
     auto process = [&](int it, uint32_t lo, uint32_t hi) -> bool {
-      const int s = it % B_STAGES;
-      const uint32_t ph = ((uint32_t)it / B_STAGES) & 1u;
+      const int s = it % kStages;
+      const uint32_t ph = ((uint32_t)it / kStages) & 1u;
       uint64_t zeros = ~((uint64_t)lo | ((uint64_t)hi << 32));
       // A parity wait tells phases apart only one phase deep, and a warp that had nothing to
       // zero on the stage's previous use never looked at `full` then: first wait until that
@@ -398,7 +401,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
         return false;
       }
       if (zeros != 0ull) {
-        const uint32_t row_addr = smem_u32(row_base + s * B_STAGE_BYTES);
+        const uint32_t row_addr = smem_u32(row_base + s * kStageBytes);
         if (__popcll(zeros) <= kScanLimit) {
           // one 2-byte store of zero per blocked element (typically one or two per row)
           while (zeros != 0ull) {
@@ -859,6 +862,11 @@ struct PlaneSpec {
 };
 
 using BwdKernel = void (*)(const CUtensorMap, const CUtensorMap, const BwdTcParams);
+template <int BN>
+static BwdKernel pick_bwd_kernel(bool wgrad, bool ragged) {
+  if (ragged) return wgrad ? bwd_tc_kernel<true, true, BN> : bwd_tc_kernel<false, true, BN>;
+  return wgrad ? bwd_tc_kernel<true, false, BN> : bwd_tc_kernel<false, false, BN>;
+}
 
 static int launch_bwd_tc(bool wgrad, const void* g, const void* b_op, const uint32_t* keep_mask,
                          int mask_words, int M, int K, int N, const TileTable& tt, int pairing, void* c_out,
@@ -881,7 +889,8 @@ static int launch_bwd_tc(bool wgrad, const void* g, const void* b_op, const uint
   p.T = tt.T;
   p.tile_w = w;
   p.num_ib = (p.I + BM - 1) / BM;
-  p.num_jb = ((rt ? rt->widest() : w) + B_BN - 1) / B_BN;
+  const int width = rt ? rt->widest() : w;  // columns of C per analog tile
+  p.a_rows = p.I < BM ? (p.I + 7) / 8 * 8 : BM;
   p.lsteps = (p.L + BK - 1) / BK;
   p.keep_mask = keep_mask;
   p.mask_words = mask_words;
@@ -908,10 +917,27 @@ static int launch_bwd_tc(bool wgrad, const void* g, const void* b_op, const uint
     p.splits = (p.lsteps + p.split_lsteps - 1) / p.split_lsteps;  // no empty copy
     p.partial = spec.partial;
   }
-  const BwdKernel single = rt ? (wgrad ? bwd_tc_kernel<true, true> : bwd_tc_kernel<false, true>)
-                              : (wgrad ? bwd_tc_kernel<true, false> : bwd_tc_kernel<false, false>);
-  const int single_smem = B_SMEM + (rt ? kRagStageBytes : 0);
-  int rc = ensure_smem(single, single_smem);
+  // CTA pairs (256-row blocks) or single CTAs; a split reduction and ragged outputs exist on single CTAs only
+  const int64_t pair_work = (int64_t)((p.I + 2 * BM - 1) / (2 * BM)) * p.T * ((width + P_BN - 1) / P_BN);
+  const int keep_free = comm_reserved_sms();
+  int pairs = rt || p.splits > 1 || pairing < 0 ? 0 : max_pairs(wgrad);
+  if (pairs > 1 && keep_free > 0) pairs = pairs - (keep_free + 1) / 2 > 1 ? pairs - (keep_free + 1) / 2 : 1;
+  const int sms = sm_count() - keep_free > 1 ? sm_count() - keep_free : 1;
+  int bn = pick_blocks(pairs, pair_work, sms, 256, 64, [&](int b) {
+    return (int64_t)p.num_ib * p.T * ((width + b - 1) / b) * p.splits;
+  });
+  if (pairing > 0 && pairs > 0) bn = 0;
+  const bool pair = bn == 0;
+  p.num_jb = (width + (pair ? P_BN : bn) - 1) / (pair ? P_BN : bn);
+  if (pair) p.a_rows = BM;
+  // before the maps: this runtime call also binds the device's context to the calling thread (autograd's own threads),
+  // which the driver entry point that encodes them needs
+  const BwdKernel kernel = pair        ? (wgrad ? bwd_tc_pair_kernel<true> : bwd_tc_pair_kernel<false>)
+                           : bn == 256 ? pick_bwd_kernel<256>(wgrad, rt != nullptr)
+                           : bn == 128 ? pick_bwd_kernel<128>(wgrad, rt != nullptr)
+                                       : pick_bwd_kernel<64>(wgrad, rt != nullptr);
+  const int smem = pair ? P_SMEM : bwd_smem(bn) + (rt ? kRagStageBytes : 0);
+  int rc = ensure_smem(kernel, smem);
   if (rc) return rc;
   CUtensorMap map_a, map_b;
   const uint64_t row_a = rt ? (uint64_t)(N + 7) / 8 * 8 : (uint64_t)N;              // elements per row of g
@@ -920,7 +946,7 @@ static int launch_bwd_tc(bool wgrad, const void* g, const void* b_op, const uint
     // g [planes][M,N]: dims innermost first {N, M, planes}
     uint64_t dims[3] = {(uint64_t)N, (uint64_t)M, (uint64_t)spec.a_planes};
     uint64_t strides[2] = {row_a * 2, (uint64_t)M * row_a * 2};
-    uint32_t box_k[3] = {BK, BM, 1};   // dgrad: 64 n (reduction) x 128 m
+    uint32_t box_k[3] = {BK, (uint32_t)p.a_rows, 1};   // dgrad: 64 n (reduction) x 128 m
     uint32_t box_mn[3] = {64, BK, 1};  // wgrad: 64 n (MMA-M) x 64 m (reduction)
     rc = make_map(&map_a, g, 3, dims, strides, wgrad ? box_mn : box_k);
     if (rc) return rc;
@@ -933,26 +959,14 @@ static int launch_bwd_tc(bool wgrad, const void* g, const void* b_op, const uint
     rc = make_map(&map_b, b_op, 3, dims, strides, box);
     if (rc) return rc;
   }
-  // CTA pairs (256-row blocks) when they fill the machine; single CTAs for smaller problems
-  const int pair_work = ((p.I + 2 * BM - 1) / (2 * BM)) * p.T * p.num_jb;
-  int pairs = max_pairs(wgrad);
-  const int keep_free = comm_reserved_sms();
-  if (pairs > 1 && keep_free > 0) pairs = pairs - (keep_free + 1) / 2 > 1 ? pairs - (keep_free + 1) / 2 : 1;
-  if (!rt && p.splits == 1 && pairs > 0 && pairing >= 0 && (pair_work >= pairs || pairing > 0)) {
+  if (pair) {
     p.num_ib = (p.I + 2 * BM - 1) / (2 * BM);
-    rc = wgrad ? ensure_smem(bwd_tc_pair_kernel<true>, P_SMEM) : ensure_smem(bwd_tc_pair_kernel<false>, P_SMEM);
-    if (rc) return rc;
-    const int grid = 2 * (pair_work < pairs ? pair_work : pairs);
-    if (wgrad)
-      bwd_tc_pair_kernel<true><<<grid, kBwdThreads, P_SMEM, s>>>(map_a, map_b, p);
-    else
-      bwd_tc_pair_kernel<false><<<grid, kBwdThreads, P_SMEM, s>>>(map_a, map_b, p);
+    kernel<<<2 * (int)(pair_work < pairs ? pair_work : pairs), kBwdThreads, smem, s>>>(map_a, map_b, p);
     return check_launch(wgrad ? "wgrad_tc_pair" : "dgrad_tc_pair");
   }
   int work = p.num_ib * p.T * p.num_jb * p.splits;
-  const int sms = sm_count() - keep_free > 1 ? sm_count() - keep_free : 1;
   int grid = work < sms ? work : sms;
-  single<<<grid, kBwdThreads, single_smem, s>>>(map_a, map_b, p);
+  kernel<<<grid, kBwdThreads, smem, s>>>(map_a, map_b, p);
   rc = check_launch(wgrad ? "wgrad_tc" : "dgrad_tc");
   if (rc || p.splits == 1) return rc;
   return launch_sum_partials(spec.f32_out ? AL_F32 : AL_BF16, p.partial, p.splits, (int64_t)p.I * K, c_out, s);

@@ -7,7 +7,7 @@
 // tensor core works on tile t+1 sixteen epilogue warps run tile t's output stage (rounding,
 // output noise, ADC quantisation, clamp, clamp-mask bits) and add it to a running sum.  Large
 // problems run on CTA pairs (256 x 256 blocks, cta_group::2), small ones on single CTAs
-// (128 x 128 blocks).
+// (128 x 128 blocks, or 128 x 64 and 128 x 32 where those fill more of the chip).
 #include "tcgen05_common.cuh"
 
 namespace al {
@@ -22,7 +22,8 @@ struct FwdTcParams {
   int32_t tile_w;      // width of every analog tile (all equal on this path)
   int32_t ksteps;      // ceil(tile_w / 64)
   int32_t num_mb, num_nb;
-  int32_t planes_b;    // bf16 planes of the weights (kPlanes for an fp32 layer, else 1): accumulated per analog tile
+  int32_t a_rows;      // single CTAs: rows a copy of A brings (fewer than 128 when M is smaller; the others of the
+                       // stage keep what was there: they only reach outputs of rows that do not exist)
   float inp_res;       // fp32 layers: the A operand holds integer DAC codes, the accumulator is scaled by the DAC step
   FwdEpilogueParams ep;
   NoiseKeys noise;     // output-noise stream of this call, prepared on the host
@@ -30,7 +31,7 @@ struct FwdTcParams {
 };
 
 constexpr int kRagStageWords = 32 * 9;
-constexpr int kRagStageBytes = F_EPI_WARPS * kRagStageWords * 4;
+constexpr int rag_stage_bytes(int bn) { return fwd_epi_warps(false, bn) * kRagStageWords * 4; }
 
 // normals of elements idx .. idx + 15 of the output-noise stream (normal4's groups of four, any idx)
 __device__ __forceinline__ void normals16(uint64_t seed, uint64_t offset, uint64_t idx, float z[16]) {
@@ -77,15 +78,23 @@ __device__ __forceinline__ void normals16(uint64_t seed, uint64_t offset, uint64
 // the CUDA cores, 43 us here).  IO = fp32: the A operand holds the DAC codes as bf16 integers and the weights come as
 // bf16 planes (fourth dimension of their tensor map) that are accumulated one after the other;
 // the output stage multiplies the accumulator by the DAC step of its (row, tile) first.
-template <int RD, int MODE, bool PAIR, int IO = kBF16, bool RAG = false>
-__global__ void __launch_bounds__(kFwdThreads, 1)
+//
+// BN: columns of a single CTA's block.  What bounds a small problem is how fast the operands reach the SMs it runs on
+// (about 50 bytes per clock and SM, whatever the number of SMs busy): a copy brings no rows beyond M, and the block
+// width follows from bytes per k-step and rounds of blocks (pick_blocks).
+template <int RD, int MODE, bool PAIR, int IO = kBF16, bool RAG = false, int BN = F_BN>
+__global__ void __launch_bounds__(fwd_threads(PAIR, BN), 1)
 fwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
               const FwdTcParams p) {
-  constexpr int kStages = PAIR ? FP_STAGES : F_STAGES;
-  constexpr int kBRows = F_BN;                                 // weight rows this CTA stages
-  constexpr int kStageBytes = F_STAGE_BYTES;
+  constexpr int kPlanesB = IO == kF32 ? kPlanes : 1;           // planes of the weights per stage
+  constexpr int kStages = PAIR ? FP_STAGES : fwd_stages(BN, kPlanesB);
+  constexpr int kBRows = BN;                                   // weight rows this CTA stages
+  constexpr int kPlaneBytes = kBRows * BK * 2;
+  constexpr int kStageBytes = fwd_stage_bytes(BN, kPlanesB);
+  constexpr int kEpiWarps = fwd_epi_warps(PAIR, BN);
+  static_assert(!PAIR || (BN == F_BN && IO == kBF16), "CTA pairs: 256 x 256 blocks of bf16 layers");
   constexpr int kBlockRows = PAIR ? 2 * BM : BM;               // rows of the outputs per work item
-  constexpr int kBN = PAIR ? 2 * F_BN : F_BN;                  // columns of the outputs per work item
+  constexpr int kBN = PAIR ? 2 * BN : BN;                      // columns of the outputs per work item
   constexpr int kSumBytes = PAIR ? FP_SUM_BYTES : 0;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* stage_base = align_1024(smem_raw);
@@ -111,7 +120,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&bars->acc_full[b], 1);
-      mbar_init(&bars->acc_empty[b], PAIR ? 2 * F_EPI_WARPS : F_EPI_WARPS);
+      mbar_init(&bars->acc_empty[b], PAIR ? 2 * kEpiWarps : kEpiWarps);
     }
     mbar_init(&bars->mma_done, 1);
     bars->abort_flag = 0;
@@ -137,9 +146,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
       for (int tile = worker; tile < num_tiles && ok; tile += n_workers) {
         const int mb = tile / p.num_nb, nb = tile % p.num_nb;
         for (int t = 0; t < T && ok; ++t) {
-          const int steps = p.ksteps * p.planes_b;
-          for (int st = 0; st < steps; ++st, ++it) {
-            const int ks = st % p.ksteps, plane = st / p.ksteps;
+          for (int ks = 0; ks < p.ksteps; ++ks, ++it) {
             const int s = it % kStages;
             const uint32_t ph = (it / kStages) & 1u;
             if (!mbar_wait(&bars->empty[s], ph ^ 1u, abort_flag)) {
@@ -155,10 +162,15 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
               tma_load_3d_pair(sa, &map_a, bar, ks * BK, t, mb * kBlockRows + row_off);
               tma_load_3d_pair(sa + F_A_BYTES, &map_b, bar, ks * BK, t, nb * kBN + (int)rank * kBRows);
             } else {
-              mbar_expect_tx(&bars->full[s], kStageBytes);
+              mbar_expect_tx(&bars->full[s], (uint32_t)(p.a_rows * BK * 2 + kPlanesB * kPlaneBytes));
               tma_load_3d(sa, &map_a, &bars->full[s], ks * BK, t, mb * BM);
-              if (IO == kF32) tma_load_4d(sa + F_A_BYTES, &map_b, &bars->full[s], ks * BK, t, nb * F_BN, plane);
-              else tma_load_3d(sa + F_A_BYTES, &map_b, &bars->full[s], ks * BK, t, nb * F_BN);
+              if (IO == kF32) {
+#pragma unroll
+                for (int plane = 0; plane < kPlanesB; ++plane)
+                  tma_load_4d(sa + F_A_BYTES + plane * kPlaneBytes, &map_b, &bars->full[s], ks * BK, t, nb * BN, plane);
+              } else {
+                tma_load_3d(sa + F_A_BYTES, &map_b, &bars->full[s], ks * BK, t, nb * BN);
+              }
             }
           }
         }
@@ -198,8 +210,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
           }
           tc_fence_after();
           const uint32_t d_tmem = tmem_base + (uint32_t)(b * kBN);
-          const int steps = p.ksteps * p.planes_b;
-          for (int ks = 0; ks < steps; ++ks, ++it) {
+          for (int ks = 0; ks < p.ksteps; ++ks, ++it) {
             const int s = it % kStages;
             const uint32_t ph = (it / kStages) & 1u;
             if (!mbar_wait(&bars->full[s], ph, abort_flag)) {
@@ -211,10 +222,14 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
             const uint32_t sa = smem_u32(stage_base + s * kStageBytes);
             const uint64_t da = desc_k_major(sa), db = desc_k_major(sa + F_A_BYTES);
 #pragma unroll
-            for (int k4 = 0; k4 < BK / 16; ++k4) {
-              if (PAIR) umma_bf16_pair(d_tmem, da + (uint64_t)(k4 * 2), db + (uint64_t)(k4 * 2), idesc, (ks | k4) != 0 ? 1u : 0u);
-              else umma_bf16(d_tmem, da + (uint64_t)(k4 * 2), db + (uint64_t)(k4 * 2), idesc, (ks | k4) != 0 ? 1u : 0u);
-            }
+            for (int plane = 0; plane < kPlanesB; ++plane)  // fp32: both planes meet the codes staged once
+#pragma unroll
+              for (int k4 = 0; k4 < BK / 16; ++k4) {
+                const uint64_t dbp = db + (uint64_t)(plane * (kPlaneBytes >> 4) + k4 * 2);
+                const uint32_t acc = (ks | k4 | plane) != 0 ? 1u : 0u;
+                if (PAIR) umma_bf16_pair(d_tmem, da + (uint64_t)(k4 * 2), dbp, idesc, acc);
+                else umma_bf16(d_tmem, da + (uint64_t)(k4 * 2), dbp, idesc, acc);
+              }
             if (PAIR) umma_commit_pair(&bars->empty[s], 3);  // frees the stage in both CTAs
             else umma_commit(&bars->empty[s]);
           }
@@ -237,8 +252,8 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
     }
   } else if (warp >= 4) {
     // ---- epilogue: per-tile output stage and running sum ----------------------------------
-    // 16 warps: warp & 3 selects the TMEM lane quadrant (rows), (warp - 4) >> 2 the kCols columns.
-    constexpr int kCols = kBN / 4;
+    // warp & 3 selects the TMEM lane quadrant (rows), (warp - 4) >> 2 the kCols columns
+    constexpr int kCols = PAIR ? kBN / 4 : 32;
     const int quad = warp & 3;
     const int col0 = ((warp - 4) >> 2) * kCols;
     const uint32_t lane_base = (uint32_t)(quad * 32) << 16;
@@ -346,9 +361,9 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
                              : "r"(addr) : "memory");
               }
             } else if (packed) {
-              tmem_ld8(tmem_base + lane_base + (uint32_t)(2 * F_BN + (cc >> 1)), sumr);
+              tmem_ld8(tmem_base + lane_base + (uint32_t)(2 * BN + (cc >> 1)), sumr);
             } else {
-              tmem_ld16(tmem_base + lane_base + (uint32_t)(2 * F_BN + cc), sumr);
+              tmem_ld16(tmem_base + lane_base + (uint32_t)(2 * BN + cc), sumr);
             }
           }
           tmem_wait_ld();
@@ -506,9 +521,9 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
                              "r"(sumr[4 * v + 1]), "r"(sumr[4 * v + 2]), "r"(sumr[4 * v + 3]) : "memory");
               }
             } else if (packed) {
-              tmem_st8(tmem_base + lane_base + (uint32_t)(2 * F_BN + (cc >> 1)), sumr);
+              tmem_st8(tmem_base + lane_base + (uint32_t)(2 * BN + (cc >> 1)), sumr);
             } else {
-              tmem_st16(tmem_base + lane_base + (uint32_t)(2 * F_BN + cc), sumr);
+              tmem_st16(tmem_base + lane_base + (uint32_t)(2 * BN + cc), sumr);
             }
           } else if (RAG) {
             // final (ragged outputs): bias, convert, transpose through this warp's staging buffer
@@ -619,23 +634,33 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
 bool tc_forward_supported(const AlDesc& d, const TileTable& tt) { return tc_shape_ok(d, tt); }
 
 using FwdKernel = void (*)(const CUtensorMap, const CUtensorMap, const FwdTcParams);
-template <bool PAIR>
+template <bool PAIR, int BN = F_BN>
 static FwdKernel pick_fwd_kernel(int mode, int round_dt) {
   switch (mode) {
-    case 0: return fwd_tc_kernel<kBF16, 0, PAIR>;
-    case 1: return fwd_tc_kernel<kBF16, 1, PAIR>;
-    case 2: return fwd_tc_kernel<kBF16, 2, PAIR>;
-    case 3: return fwd_tc_kernel<kBF16, 3, PAIR>;
-    case 4: return fwd_tc_kernel<kBF16, 4, PAIR>;
-    case 5: return fwd_tc_kernel<kBF16, 5, PAIR>;
-    case 6: return fwd_tc_kernel<kBF16, 6, PAIR>;
-    case 7: return fwd_tc_kernel<kBF16, 7, PAIR>;
+    case 0: return fwd_tc_kernel<kBF16, 0, PAIR, kBF16, false, BN>;
+    case 1: return fwd_tc_kernel<kBF16, 1, PAIR, kBF16, false, BN>;
+    case 2: return fwd_tc_kernel<kBF16, 2, PAIR, kBF16, false, BN>;
+    case 3: return fwd_tc_kernel<kBF16, 3, PAIR, kBF16, false, BN>;
+    case 4: return fwd_tc_kernel<kBF16, 4, PAIR, kBF16, false, BN>;
+    case 5: return fwd_tc_kernel<kBF16, 5, PAIR, kBF16, false, BN>;
+    case 6: return fwd_tc_kernel<kBF16, 6, PAIR, kBF16, false, BN>;
+    case 7: return fwd_tc_kernel<kBF16, 7, PAIR, kBF16, false, BN>;
     default:
       // CTA pairs exist for bf16 rounding only
       if (PAIR) return fwd_tc_kernel<kBF16, -1, PAIR>;
-      return round_dt == AL_BF16 ? fwd_tc_kernel<kBF16, -1, false> : fwd_tc_kernel<kF32, -1, false>;
+      return round_dt == AL_BF16 ? fwd_tc_kernel<kBF16, -1, false, kBF16, false, BN>
+                                 : fwd_tc_kernel<kF32, -1, false, kBF16, false, BN>;
   }
 }
+
+// Columns of a single CTA's block (128, 64 or 32), or 0 when CTA pairs are the better choice
+static int fwd_block_columns(int M, int N, int n_pairs = 0) {
+  const int64_t pair_blocks = (int64_t)((M + 2 * BM - 1) / (2 * BM)) * ((N + 2 * F_BN - 1) / (2 * F_BN));
+  return pick_blocks(n_pairs, pair_blocks, sm_count(), 128, 32,
+                     [&](int bn) { return (int64_t)((M + BM - 1) / BM) * ((N + bn - 1) / bn); });
+}
+
+static int fwd_copy_rows(int M) { return M < BM ? (M + 7) / 8 * 8 : BM; }
 
 static int small_adc_codes(int tile_w, const FwdEpilogueParams& ep) {
   // |o| <= tile_w * ir * wmax * (1 + noise) and step = 2 * out_bound * ir * wmax / states
@@ -652,7 +677,7 @@ static int max_fwd_pairs(FwdKernel kernel, int smem) {
   for (int i = 0; i < n_seen; ++i)
     if (seen[i] == kernel) return count[i];
   int clusters = 0;
-  PairLaunch pl(2 * sm_count(), kFwdThreads, smem, nullptr);
+  PairLaunch pl(2 * sm_count(), fwd_threads(true, F_BN), smem, nullptr);
   if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &pl.cfg) != cudaSuccess) {
     cudaGetLastError();
     clusters = 0;
@@ -676,11 +701,10 @@ int launch_fwd_tc(int round_dt, const void* xq, const void* w_mod, int K, const 
   p.tile_w = w;
   p.ksteps = (w + BK - 1) / BK;
   p.num_mb = (ep.M + BM - 1) / BM;
-  p.num_nb = (ep.N + F_BN - 1) / F_BN;
+  p.a_rows = fwd_copy_rows(ep.M);
   p.ep = ep;
   p.noise = make_noise_keys(ep.seed, ep.offset, 1u, ep.offset_base);
   p.out = out;
-  p.planes_b = 1;
   p.inp_res = 0.0f;
   p.small_adc_codes = small_adc_codes(w, ep);
   const bool per_channel = ep.w_amax != nullptr && (ep.noise_pc || ep.bound_pc);
@@ -689,8 +713,7 @@ int launch_fwd_tc(int round_dt, const void* xq, const void* w_mod, int K, const 
   const bool fixed = round_dt == AL_BF16 && !per_channel && ep.out_noise == nullptr && !ep.no_rounding &&
                      p.small_adc_codes && (!ep.has_adc || adc_codes_fit_a_byte(ep.out_res, ep.has_bound != 0));
   const int mode = fixed ? ((ep.has_noise ? 1 : 0) | (ep.has_adc ? 2 : 0) | (ep.has_bound ? 4 : 0)) : -1;
-  // CTA pairs (256 x 256 blocks, packed bf16 output stage only) when there is a block per pair
-  // of SMs; single CTAs (128 x 128) otherwise.
+  // CTA pairs (256 x 256 blocks, packed bf16 output stage only) or single CTAs: pick_blocks.
   // The runtime calls below also bind the device's primary context to the calling thread
   // (autograd runs backward on its own threads); the driver entry point that encodes the
   // tensor maps needs a current context.
@@ -705,32 +728,38 @@ int launch_fwd_tc(int round_dt, const void* xq, const void* w_mod, int K, const 
     if (rc) return rc;
     pairs = max_fwd_pairs(kernel, pair_smem);
   }
-  const bool pair = pairs > 0 && (pair_tiles >= pairs || pairing > 0);
+  const int columns = pairing > 0 && pairs > 0 ? 0 : fwd_block_columns(ep.M, ep.N, pairs);
+  const bool pair = columns == 0;
+  const int bn = pair ? F_BN : columns;
+  const int single_smem = fwd_smem(bn, 1);
   if (!pair) {
-    kernel = pick_fwd_kernel<false>(mode, round_dt);
-    rc = ensure_smem(kernel, F_SMEM);
+    kernel = bn == 128 ? pick_fwd_kernel<false, 128>(mode, round_dt)
+             : bn == 64 ? pick_fwd_kernel<false, 64>(mode, round_dt) : pick_fwd_kernel<false, 32>(mode, round_dt);
+    rc = ensure_smem(kernel, single_smem);
     if (rc) return rc;
+    p.num_nb = (ep.N + bn - 1) / bn;
   } else {
     p.num_mb = (ep.M + 2 * BM - 1) / (2 * BM);
+    p.a_rows = BM;
     p.num_nb = (ep.N + 2 * F_BN - 1) / (2 * F_BN);
   }
   CUtensorMap map_a, map_b;
   {
     uint64_t dims[3] = {(uint64_t)w, (uint64_t)tt.T, (uint64_t)ep.M};
     uint64_t strides[2] = {(uint64_t)w * 2, (uint64_t)K * 2};
-    uint32_t box[3] = {BK, 1, BM};
+    uint32_t box[3] = {BK, 1, (uint32_t)p.a_rows};
     rc = make_map(&map_a, xq, 3, dims, strides, box);
     if (rc) return rc;
   }
   {
     uint64_t dims[3] = {(uint64_t)w, (uint64_t)tt.T, (uint64_t)ep.N};
     uint64_t strides[2] = {(uint64_t)w * 2, (uint64_t)K * 2};
-    uint32_t box[3] = {BK, 1, F_BN};
+    uint32_t box[3] = {BK, 1, (uint32_t)bn};
     rc = make_map(&map_b, w_mod, 3, dims, strides, box);
     if (rc) return rc;
   }
   if (pair) {
-    PairLaunch pl(2 * (pair_tiles < pairs ? pair_tiles : pairs), kFwdThreads, pair_smem, s);
+    PairLaunch pl(2 * (pair_tiles < pairs ? pair_tiles : pairs), fwd_threads(true, F_BN), pair_smem, s);
     cudaError_t e = cudaLaunchKernelEx(&pl.cfg, kernel, map_a, map_b, p);
     if (e != cudaSuccess) {
       set_error("fwd_tc (pairs): %s", cudaGetErrorString(e));
@@ -740,7 +769,7 @@ int launch_fwd_tc(int round_dt, const void* xq, const void* w_mod, int K, const 
   }
   int tiles = p.num_mb * p.num_nb;
   int grid = tiles < sm_count() ? tiles : sm_count();
-  kernel<<<grid, kFwdThreads, F_SMEM, s>>>(map_a, map_b, p);
+  kernel<<<grid, fwd_threads(false, bn), single_smem, s>>>(map_a, map_b, p);
   return check_launch("fwd_tc");
 }
 
@@ -755,9 +784,15 @@ int launch_fwd_tc(int round_dt, const void* xq, const void* w_mod, int K, const 
 // reduction over the rows, so a layer of few output blocks leaves from 8192 rows on.
 bool tc_ragged_supported(const AlDesc& d, const TileTable& tt, RaggedTiles* rt) {
   if (d.dtype != AL_BF16 || d.engine != AL_ENGINE_AUTO || tc_tiling_ok(d, tt) || !ragged_tiles(tt, rt)) return false;
-  const int64_t blocks = (int64_t)((d.N + BM - 1) / BM) * rt->T * ((rt->widest() + B_BN - 1) / B_BN);
+  const int64_t blocks = (int64_t)((d.N + BM - 1) / BM) * rt->T * ((rt->widest() + 255) / 256);
   if (rt->widest() < 8 || (d.M > 8192 && blocks < 37)) return false;
   return (int64_t)rt->T * rt->pitch < (1ll << 31);
+}
+
+template <int BN>
+static FwdKernel pick_ragged_kernel(int round_dt) {
+  return round_dt == AL_BF16 ? fwd_tc_kernel<kBF16, -1, false, kBF16, true, BN>
+                             : fwd_tc_kernel<kF32, -1, false, kBF16, true, BN>;
 }
 
 int launch_fwd_tc_ragged(int round_dt, const void* xq, const void* w_mod, const RaggedTiles& rt,
@@ -771,16 +806,17 @@ int launch_fwd_tc_ragged(int round_dt, const void* xq, const void* w_mod, const 
   p.tile_w = rt.widest();
   p.ksteps = (p.tile_w + BK - 1) / BK;
   p.num_mb = (ep.M + BM - 1) / BM;
-  p.num_nb = (ep.N + F_BN - 1) / F_BN;
-  p.planes_b = 1;
+  p.a_rows = fwd_copy_rows(ep.M);
+  const int bn = fwd_block_columns(ep.M, ep.N);
+  p.num_nb = (ep.N + bn - 1) / bn;
   p.inp_res = 0.0f;
   p.ep = ep;
   p.noise = make_noise_keys(ep.seed, ep.offset, 1u, ep.offset_base);
   p.out = out;
   p.small_adc_codes = small_adc_codes(p.tile_w, ep);
-  FwdKernel kernel = round_dt == AL_BF16 ? fwd_tc_kernel<kBF16, -1, false, kBF16, true>
-                                         : fwd_tc_kernel<kF32, -1, false, kBF16, true>;
-  const int smem = F_SMEM + kRagStageBytes;
+  FwdKernel kernel = bn == 128  ? pick_ragged_kernel<128>(round_dt)
+                     : bn == 64 ? pick_ragged_kernel<64>(round_dt) : pick_ragged_kernel<32>(round_dt);
+  const int smem = fwd_smem(bn, 1) + rag_stage_bytes(bn);
   int rc = ensure_smem(kernel, smem);
   if (rc) return rc;
   CUtensorMap map_a, map_b;
@@ -788,12 +824,12 @@ int launch_fwd_tc_ragged(int round_dt, const void* xq, const void* w_mod, const 
   for (int b = 0; b < 2; ++b) {
     uint64_t dims[3] = {(uint64_t)p.tile_w, (uint64_t)rt.T, (uint64_t)(b ? ep.N : ep.M)};
     uint64_t strides[2] = {(uint64_t)rt.pitch * 2, row_bytes};
-    uint32_t box[3] = {BK, 1, (uint32_t)(b ? F_BN : BM)};
+    uint32_t box[3] = {BK, 1, (uint32_t)(b ? bn : p.a_rows)};
     rc = make_map(b ? &map_b : &map_a, b ? w_mod : xq, 3, dims, strides, box);
     if (rc) return rc;
   }
   const int tiles = p.num_mb * p.num_nb;
-  kernel<<<tiles < sm_count() ? tiles : sm_count(), kFwdThreads, smem, s>>>(map_a, map_b, p);
+  kernel<<<tiles < sm_count() ? tiles : sm_count(), fwd_threads(false, bn), smem, s>>>(map_a, map_b, p);
   return check_launch("fwd_tc_ragged");
 }
 
@@ -820,34 +856,38 @@ int launch_fwd_tc_f32(const void* codes16, const void* w_planes, int K, const Ti
   p.tile_w = w;
   p.ksteps = (w + BK - 1) / BK;
   p.num_mb = (ep.M + BM - 1) / BM;
-  p.num_nb = (ep.N + F_BN - 1) / F_BN;
+  p.a_rows = fwd_copy_rows(ep.M);
+  const int bn = fwd_block_columns(ep.M, ep.N);
+  p.num_nb = (ep.N + bn - 1) / bn;
   p.ep = ep;
   p.noise = make_noise_keys(ep.seed, ep.offset, 1u, ep.offset_base);
   p.out = out;
-  p.planes_b = kPlanes;
   p.inp_res = inp_res;
   p.small_adc_codes = 0;  // fp32 accumulators: guarded rint
-  auto kernel = fwd_tc_kernel<kF32, -1, false, kF32>;
-  int rc = ensure_smem(kernel, F_SMEM);
+  FwdKernel kernel = bn == 128  ? fwd_tc_kernel<kF32, -1, false, kF32, false, 128>
+                     : bn == 64 ? fwd_tc_kernel<kF32, -1, false, kF32, false, 64>
+                                : fwd_tc_kernel<kF32, -1, false, kF32, false, 32>;
+  const int smem = fwd_smem(bn, kPlanes);
+  int rc = ensure_smem(kernel, smem);
   if (rc) return rc;
   CUtensorMap map_a, map_b;
   {
     uint64_t dims[3] = {(uint64_t)w, (uint64_t)tt.T, (uint64_t)ep.M};
     uint64_t strides[2] = {(uint64_t)w * 2, (uint64_t)K * 2};
-    uint32_t box[3] = {BK, 1, BM};
+    uint32_t box[3] = {BK, 1, (uint32_t)p.a_rows};
     rc = make_map(&map_a, codes16, 3, dims, strides, box);
     if (rc) return rc;
   }
   {
     uint64_t dims[4] = {(uint64_t)w, (uint64_t)tt.T, (uint64_t)ep.N, (uint64_t)kPlanes};
     uint64_t strides[3] = {(uint64_t)w * 2, (uint64_t)K * 2, (uint64_t)ep.N * K * 2};
-    uint32_t box[4] = {BK, 1, F_BN, 1};
+    uint32_t box[4] = {BK, 1, (uint32_t)bn, 1};
     rc = make_map(&map_b, w_planes, 4, dims, strides, box);
     if (rc) return rc;
   }
   const int tiles = p.num_mb * p.num_nb;
   const int grid = tiles < sm_count() ? tiles : sm_count();
-  kernel<<<grid, kFwdThreads, F_SMEM, s>>>(map_a, map_b, p);
+  kernel<<<grid, fwd_threads(false, bn), smem, s>>>(map_a, map_b, p);
   return check_launch("fwd_tc_f32");
 }
 

@@ -43,20 +43,26 @@ constexpr uint32_t kSuspendHintNs = 20000u;
 
 // forward kernel
 constexpr int F_BN = 128;
-constexpr int F_STAGES = 6;
 constexpr int FP_STAGES = 5;   // CTA pairs: 64 KiB of shared memory hold the running sum
 constexpr int FP_SUM_BYTES = BM * 2 * F_BN * 2;
+constexpr int F_RING_BYTES = 192 * 1024;  // single CTAs: what the pipeline stages share
 constexpr int F_A_BYTES = BM * BK * 2;     // 16 KiB
 constexpr int F_B_BYTES = F_BN * BK * 2;   // 16 KiB
 constexpr int F_STAGE_BYTES = F_A_BYTES + F_B_BYTES;
-constexpr int F_EPI_WARPS = 16;
-constexpr int kFwdThreads = (4 + F_EPI_WARPS) * 32;  // producer, MMA, two idle, 16 epilogue warps
+constexpr int F_EPI_WARPS = 16;  // CTA pairs, and single CTAs with 128 columns
+// producer, MMA, two idle warps and the epilogue: four warps (one per 32 rows) per 32 columns of the block
+constexpr int fwd_epi_warps(bool pair, int bn) { return pair ? F_EPI_WARPS : bn / 8; }
+constexpr int fwd_threads(bool pair, int bn) { return (4 + fwd_epi_warps(pair, bn)) * 32; }
+// a stage holds 64 k of the block's rows and of its `bn` weight rows (`planes` bf16 planes of them)
+constexpr int fwd_stage_bytes(int bn, int planes) { return F_A_BYTES + planes * bn * BK * 2; }
+constexpr int fwd_stages(int bn, int planes) {
+  return F_RING_BYTES / fwd_stage_bytes(bn, planes) < 8 ? F_RING_BYTES / fwd_stage_bytes(bn, planes) : 8;
+}
 // backward kernel
-constexpr int B_BN = 256;
-constexpr int B_STAGES = 4;
+constexpr int B_RING_BYTES = 192 * 1024;   // what the pipeline stages share
 constexpr int B_A_BYTES = BM * BK * 2;     // 16 KiB
-constexpr int B_B_BYTES = B_BN * BK * 2;   // 32 KiB
-constexpr int B_STAGE_BYTES = B_A_BYTES + B_B_BYTES;
+constexpr int bwd_stage_bytes(int bn) { return B_A_BYTES + bn * BK * 2; }
+constexpr int bwd_stages(int bn) { return B_RING_BYTES / bwd_stage_bytes(bn); }  // 256: 4, 128: 6, 64: 8
 constexpr int B_BOX_BYTES = 64 * BK * 2;   // one 64x64 MN-major box: 8 KiB
 constexpr int B_EPI_WARPS = 4;
 constexpr int B_XFORM_THREADS = 128;   // per group; each group handles one stage at a time
@@ -443,8 +449,28 @@ int sm_count() {
   return n;
 }
 
-constexpr int F_SMEM = F_STAGES * F_STAGE_BYTES + (int)sizeof(Barriers) + 1024;
-constexpr int B_SMEM = B_STAGES * B_STAGE_BYTES + (int)sizeof(Barriers) + 1024;
+constexpr int fwd_smem(int bn, int planes) {
+  return fwd_stages(bn, planes) * fwd_stage_bytes(bn, planes) + (int)sizeof(Barriers) + 1024;
+}
+constexpr int bwd_smem(int bn) { return bwd_stages(bn) * bwd_stage_bytes(bn) + (int)sizeof(Barriers) + 1024; }
+
+// Blocks for a GEMM whose output is `mb128` x 128 rows.  What bounds a k-step is the copy of its operands into the SM
+// (about 50 bytes per clock and SM, whatever the number of SMs busy): KiB per k-step x rounds of blocks over the SMs.
+// n_pairs: CTA pairs the device runs at once (0: none), pair_blocks their 256 x 256 blocks; blocks_of(bn): blocks of
+// 128 x bn columns.  Returns 0 for pairs, else the block width; the narrower of two that cost the same.
+template <class BlocksOf>
+int pick_blocks(int n_pairs, int64_t pair_blocks, int sms, int widest, int narrowest, BlocksOf blocks_of) {
+  int best = 0;
+  int64_t cost = n_pairs > 0 ? (pair_blocks + n_pairs - 1) / n_pairs * 32 : INT64_MAX;
+  for (int bn = widest; bn >= narrowest; bn /= 2) {
+    const int64_t c = (blocks_of(bn) + sms - 1) / sms * (16 + bn / 8);
+    if (c <= cost) {
+      cost = c;
+      best = bn;
+    }
+  }
+  return best;
+}
 constexpr int P_SMEM = P_STAGES * P_STAGE_BYTES + (int)sizeof(Barriers) + 1024;
 constexpr int FP_SMEM = FP_STAGES * F_STAGE_BYTES + FP_SUM_BYTES + (int)sizeof(Barriers) + 1024;
 
