@@ -165,7 +165,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
 
   if (warp == 0) {
     // ---- TMA producer ------------------------------------------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       tma_prefetch_desc(&map_a);
       tma_prefetch_desc(&map_b);
       uint32_t it = 0;
@@ -220,7 +220,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
     }
   } else if (warp == 1) {
     // ---- MMA issuer --------------------------------------------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = make_idesc(BM, BN, WGRAD ? 1 : 0, 1);
       uint32_t it = 0, acc_it = 0;
       bool ok = true;
@@ -540,7 +540,7 @@ bwd_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
 
   if (warp == 0) {
     // ---- TMA producer (both CTAs) --------------------------------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       tma_prefetch_desc(&map_a);
       tma_prefetch_desc(&map_b);
       uint32_t it = 0;
@@ -608,7 +608,7 @@ bwd_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     }
   } else if (warp == 1) {
     // ---- MMA issuer (leader only) --------------------------------------------------------
-    if (lane == 0 && leader) {
+    if (leader && elect_one()) {
       constexpr uint32_t idesc_block = make_idesc(2 * BM, P_BN, WGRAD ? 1 : 0, 1);
       constexpr uint32_t idesc_half = make_idesc(2 * BM, P_BN / 2, WGRAD ? 1 : 0, 1);
       uint32_t it = 0, acc_it = 0;

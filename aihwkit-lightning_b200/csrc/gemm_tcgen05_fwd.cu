@@ -138,7 +138,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
 
   if (warp == 0) {
     // ---- TMA producer ------------------------------------------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       tma_prefetch_desc(&map_a);
       tma_prefetch_desc(&map_b);
       uint32_t it = 0;
@@ -194,7 +194,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
     }
   } else if (warp == 1) {
     // ---- MMA issuer --------------------------------------------------------------------
-    if (lane == 0 && leader) {
+    if (leader && elect_one()) {
       constexpr uint32_t idesc = make_idesc(kBlockRows, kBN, 0, 0);
       uint32_t it = 0, acc_it = 0;
       bool ok = true;

@@ -90,6 +90,18 @@ enum ErrCode : uint32_t {
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
+// True in one thread of the (converged) warp.  The roles that issue TMA copies and MMAs are entered through this and not
+// through `lane == 0`: both instructions take uniform operands, and only under an elected thread does the compiler know
+// that one thread is active (otherwise it wraps every one of them in code that serialises the active threads).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t pred;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(pred));
+  return pred != 0;
+}
 __device__ __forceinline__ uint64_t globaltimer_ns() {
   uint64_t t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
