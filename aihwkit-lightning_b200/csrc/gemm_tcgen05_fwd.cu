@@ -79,9 +79,8 @@ __device__ __forceinline__ void normals16(uint64_t seed, uint64_t offset, uint64
 // bf16 planes (fourth dimension of their tensor map) that are accumulated one after the other;
 // the output stage multiplies the accumulator by the DAC step of its (row, tile) first.
 //
-// BN: columns of a single CTA's block.  What bounds a small problem is how fast the operands reach the SMs it runs on
-// (about 50 bytes per clock and SM, whatever the number of SMs busy): a copy brings no rows beyond M, and the block
-// width follows from bytes per k-step and rounds of blocks (pick_blocks).
+// BN: columns of a single CTA's block (pick_blocks; 256 x 4096 x 4096 with ADC: 27 us in 64 blocks of 128 columns, 15.8 us
+// in 128 of 64 issued by elected threads).  A copy of A brings no rows beyond M.
 template <int RD, int MODE, bool PAIR, int IO = kBF16, bool RAG = false, int BN = F_BN>
 __global__ void __launch_bounds__(fwd_threads(PAIR, BN), 1)
 fwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,

@@ -92,7 +92,9 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 }
 // True in one thread of the (converged) warp.  The roles that issue TMA copies and MMAs are entered through this and not
 // through `lane == 0`: both instructions take uniform operands, and only under an elected thread does the compiler know
-// that one thread is active (otherwise it wraps every one of them in code that serialises the active threads).
+// that one thread is active (otherwise it wraps every one of them in code that serialises the active threads).  That
+// code was the bound of a k-step wherever the block is small: 64 x 8192 x 512 forward 34.0 -> 19.1 us, the same with four
+// stages instead of eight; at 8192 x 4096 x 4096 input gradient 192 -> 185 us, weight gradient 222 -> 214 us.
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred;
   asm volatile(
@@ -466,8 +468,11 @@ constexpr int fwd_smem(int bn, int planes) {
 }
 constexpr int bwd_smem(int bn) { return bwd_stages(bn) * bwd_stage_bytes(bn) + (int)sizeof(Barriers) + 1024; }
 
-// Blocks for a GEMM whose output is `mb128` x 128 rows.  What bounds a k-step is the copy of its operands into the SM
-// (about 50 bytes per clock and SM, whatever the number of SMs busy): KiB per k-step x rounds of blocks over the SMs.
+// Blocks of a GEMM.  A block stages its rows of both operands per k-step, whatever the other SMs do, so the measure is
+// KiB staged per k-step x rounds of blocks over the SMs: small outputs take narrow blocks, because more SMs then share
+// the copies, and CTA pairs are taken as soon as they save a round (64 pairs instead of 256 single blocks at 1024 x
+// 4096).  Against 128-wide (forward) and 128- or 256-wide (backward) blocks throughout: 1.12x (geometric mean of 41 sizes
+// from 17 x 1024 x 1024 to 4096^3), 512 x 1024 x 1024 training 39.8 -> 33.9 us, 2048^3 105 -> 82, none slower by over 1 %.
 // n_pairs: CTA pairs the device runs at once (0: none), pair_blocks their 256 x 256 blocks; blocks_of(bn): blocks of
 // 128 x bn columns.  Returns 0 for pairs, else the block width; the narrower of two that cost the same.
 template <class BlocksOf>
