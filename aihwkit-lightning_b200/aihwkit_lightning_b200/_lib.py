@@ -4,6 +4,7 @@ There is no CPU fallback: if the library is missing the first call raises, namin
 command.  Nothing in here touches torch; callers pass raw device pointers and a stream handle.
 """
 import ctypes
+import importlib.util
 import os
 from ctypes import POINTER, Structure, c_char_p, c_double, c_float, c_int32, c_int64, c_uint32, c_uint64, c_void_p
 
@@ -113,6 +114,22 @@ SYMBOLS = {
 }
 
 _lib = None
+_host = None
+
+
+def host():
+    """The extension that runs one analog call (``csrc/host_calls.cpp``); it needs torch to be imported."""
+    global _host
+    if _host is None:
+        load()
+        path = os.path.join(os.path.dirname(LIB_PATH), "_host_calls.so")
+        if not os.path.exists(path):
+            raise RuntimeError(f"{path} is missing: build it with `python aihwkit-lightning_b200/build.py`")
+        spec = importlib.util.spec_from_file_location("_host_calls", path)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        _host = module
+    return _host
 
 
 def load():

@@ -157,13 +157,18 @@ class _OnDevice:
         return False
 
 
-def _next_seed(device):
-    """(seed, offset) from torch's CUDA generator so that ``torch.manual_seed`` governs the
-    analog noise; advances the generator like a kernel drawing 4 values per thread would."""
-    gen = torch.cuda.default_generators[device.index if device.index is not None else torch.cuda.current_device()]
-    seed, offset = gen.initial_seed(), gen.get_offset()
-    gen.set_offset(offset + 4)
-    return seed & 0xFFFFFFFFFFFFFFFF, offset
+@contextmanager
+def _reserved_sms(count):
+    """The backward GEMMs launched inside leave ``count`` SMs unoccupied."""
+    if count <= 0:
+        yield
+        return
+    lib = _lib.load()
+    lib.al_reserve_sms(int(count))
+    try:
+        yield
+    finally:
+        lib.al_reserve_sms(0)
 
 
 _DESC_CACHE: dict = {}
@@ -255,7 +260,6 @@ def _analog_forward(ctx, inp, weight, bias, input_range, input_range_update_idx,
     """One forward call of the library; ``ctx`` receives what the backward pass needs.
     ``prequant``: (xq [M,K], ir_rows [T,M]) when the DAC already ran (convolutions: fused into the patch
     extraction); ``inp`` is then ``xq`` itself."""
-    lib = _lib.load()
     if not inp.is_cuda or not weight.is_cuda:
         raise ValueError(
             "analog layers of this package run on CUDA tensors only (no CPU fallback): "
@@ -293,131 +297,52 @@ def _analog_forward(ctx, inp, weight, bias, input_range, input_range_update_idx,
         return inp.new_zeros(*inp.shape[:-1], n) + (bias if bias is not None else 0)
     ctx.empty = False
 
-    with _OnDevice(dev):
-        out = torch.empty(m, n, device=dev, dtype=dtype)
-        args = _lib.AlForwardArgs()
-        args.x, args.w, args.bias, args.out = _ptr(x2d), _ptr(w), _ptr(bias), _ptr(out)
-        if prequant is not None:
-            args.x, args.x_prequantised = None, (2 if pre_codes is not None else 1)
-        args.tile_ends = ends
-        ir_data = iridx_data = None
-        if static:
-            ir_data = input_range.data if input_range.is_contiguous() else input_range.data.contiguous()
-            iridx_data = input_range_update_idx
-            args.input_range, args.input_range_update_idx = _ptr(ir_data), _ptr(iridx_data)
-            if desc.ir_mode == _lib.AL_IR_FAST:
-                assert x_min is not None and x_max is not None, "x_min and x_max must be provided"
-                args.x_min, args.x_max = _ptr(x_min), _ptr(x_max)
-        learn_clip = desc.clip_type == _CLIP[WeightClipType.LEARNABLE_PER_CHANNEL]
-        lwc = None
-        if learn_clip:
-            assert learnable_weight_clip is not None, "learnable_weight_clip should not be None"
-            assert tuple(learnable_weight_clip.shape) == (t, n), f"learnable_weight_clip.shape must be ({t}, {n})"
-            lwc = learnable_weight_clip.detach().to(dtype).contiguous()
-            args.learnable_weight_clip = _ptr(lwc)
-        modifies = desc.quant_type != 0 or (training and desc.noise_type != 0) or learn_clip
-        need_std = static and training and desc.init_from_data > 0
-        # sizes that are no multiples of 8: the tensor-core route takes its operands in a pitched layout (a layer whose
-        # pitch equals K reads x and w themselves where nothing modifies them: those must be aligned)
-        if (dtype == torch.bfloat16 and (n % 8 or k % 8 or in_sizes[0] % 8 or in_sizes[-1] % 8) and prequant is None
-                and settings.capture is None and settings.w_noise is None and settings.out_noise is None):
-            pitch = lib.al_operand_pitch(desc, ends)
-            if pitch != k or not (x2d.data_ptr() % 16 or w.data_ptr() % 16):
-                desc.operand_pitch = pitch
-        k_rows = desc.operand_pitch or k
-        pitched = k_rows != k
-        few_rows = m <= 16 and not needs_grad and dtype == torch.bfloat16 and settings.capture is None
-        xq = x2d
-        ir_rows = w_amax = w_tile_max = keep_mask = None
-        w_mod = w
-        # fp32 layer on the tensor cores: the GEMMs read the DAC codes and the weights as bf16 planes
-        planes = dtype == torch.float32 and bool(lib.al_uses_tcgen05(desc, ends))
-        codes16 = w_planes = None
-        if not needs_grad and settings.capture is None:
-            # nothing of the workspace outlives the call: one allocation, carved by offset
-            es = w.element_size()
-            plan = [("w_amax", t * n * es), ("w_tile_max", 2 * t * 4)]
-            if (desc.ir_mode != _lib.AL_IR_OFF or pitched) and prequant is None:
-                plan += [("xq", m * k_rows * es), ("ir_rows", (t if static else t * m) * es)]
-            if modifies or pitched:
-                plan.append(("w_mod", n * k_rows * es))
-            if need_std:
-                plan.append(("std_scratch", lib.al_std_scratch_floats(m, t) * 4))
-            if few_rows:
-                plan.append(("smallm_scratch", lib.al_smallm_scratch_floats(m, n, t) * 4))
-            if planes:
-                plan.append(("w_planes", lib.al_f32_planes() * n * k * 2))
-                if pre_codes is None:
-                    plan.append(("codes16", m * k * 2))
-            total = 0
-            for _, nbytes in plan:
-                total += (nbytes + 255) & ~255
-            arena = torch.empty(total, device=dev, dtype=torch.uint8)
-            cursor = arena.data_ptr()
-            args.xq, args.w_mod = _ptr(x2d), _ptr(w)
-            for field, nbytes in plan:
-                setattr(args, field, cursor)
-                cursor += (nbytes + 255) & ~255
-            if prequant is not None:
-                args.xq, args.ir_rows, args.codes16 = _ptr(prequant[0]), _ptr(prequant[1]), _ptr(pre_codes)
-        else:
-            if prequant is not None:
-                xq, ir_rows = prequant[0], prequant[1]
-            elif desc.ir_mode != _lib.AL_IR_OFF or pitched:
-                xq = torch.empty(m, k_rows, device=dev, dtype=dtype)
-                ir_rows = torch.empty((t, m) if not static else (t,), device=dev, dtype=dtype)
-            args.xq, args.ir_rows = _ptr(xq), _ptr(ir_rows)
-            w_amax = torch.empty(t, n, device=dev, dtype=dtype)
-            w_tile_max = torch.empty(2 * t, device=dev, dtype=torch.float32)
-            args.w_amax, args.w_tile_max = _ptr(w_amax), _ptr(w_tile_max)
-            w_mod = torch.empty(n, k_rows, device=dev, dtype=dtype) if modifies or pitched else w
-            args.w_mod = _ptr(w_mod)
-            if desc.out_bound > 0 and needs_grad:
-                keep_mask = torch.empty(t, (n + 31) // 32, m, device=dev, dtype=torch.int32)
-            args.keep_mask = _ptr(keep_mask)
-            std_scratch = None
-            if need_std:
-                std_scratch = torch.empty(lib.al_std_scratch_floats(m, t), device=dev, dtype=torch.float32)
-            args.std_scratch = _ptr(std_scratch)
-            smallm_scratch = None
-            if few_rows:
-                smallm_scratch = torch.empty(lib.al_smallm_scratch_floats(m, n, t), device=dev, dtype=torch.float32)
-            args.smallm_scratch = _ptr(smallm_scratch)
-            if planes:
-                codes16 = pre_codes if pre_codes is not None else torch.empty(m, k, device=dev, dtype=torch.bfloat16)
-                w_planes = torch.empty(lib.al_f32_planes(), n, k, device=dev, dtype=torch.bfloat16)
-                args.codes16, args.w_planes = _ptr(codes16), _ptr(w_planes)
-        std_shared = None
-        if need_std and desc.ir_mode == _lib.AL_IR_STATIC and settings.sync_tile_std is not None:
-            std_shared = settings.sync_tile_std(sliced_std(in_sizes, x2d)).to(torch.float32).contiguous()
-            args.std_override = _ptr(std_shared)
-        w_noise, out_noise = settings.w_noise, settings.out_noise
-        if w_noise is not None:
-            w_noise = w_noise.to(device=dev, dtype=dtype).contiguous()
-            assert w_noise.shape == w.shape, "replayed weight noise must be [N,K]"
-        if out_noise is not None:
-            out_noise = out_noise.to(device=dev, dtype=dtype).contiguous()
-            assert out_noise.numel() == t * m * n, "replayed output noise must be [T,M,N]"
-        args.w_noise, args.out_noise = _ptr(w_noise), _ptr(out_noise)
-        codes = None
-        if settings.capture is not None and settings.capture_codes and desc.ir_mode != _lib.AL_IR_OFF:
-            codes = torch.empty_like(x2d)
-        args.codes = _ptr(codes)
-        if training and (desc.noise_type != 0 or desc.out_noise > 0):
-            if settings.graph_noise is not None:
-                args.seed, args.offset = settings.graph_noise.next()
-                args.offset_base = settings.graph_noise.counter.data_ptr()
-            else:
-                args.seed, args.offset = _next_seed(dev)
-        _lib.check(lib.al_forward(desc, args, _stream(dev)))
-        if static and ir_data is not input_range.data:
-            input_range.data.copy_(ir_data)
+    ir_data = iridx_data = None
+    if static:
+        ir_data = input_range.data if input_range.is_contiguous() else input_range.data.contiguous()
+        iridx_data = input_range_update_idx
+    fast = desc.ir_mode == _lib.AL_IR_FAST
+    if fast:
+        assert x_min is not None and x_max is not None, "x_min and x_max must be provided"
+    learn_clip = desc.clip_type == _CLIP[WeightClipType.LEARNABLE_PER_CHANNEL]
+    lwc = None
+    if learn_clip:
+        assert learnable_weight_clip is not None, "learnable_weight_clip should not be None"
+        assert tuple(learnable_weight_clip.shape) == (t, n), f"learnable_weight_clip.shape must be ({t}, {n})"
+        lwc = learnable_weight_clip.detach().to(dtype).contiguous()
+    modifies = desc.quant_type != 0 or (training and desc.noise_type != 0) or learn_clip
+    need_std = static and training and desc.init_from_data > 0
+    std_shared = None
+    if need_std and desc.ir_mode == _lib.AL_IR_STATIC and settings.sync_tile_std is not None:
+        std_shared = settings.sync_tile_std(sliced_std(in_sizes, x2d)).to(torch.float32).contiguous()
+    w_noise, out_noise = settings.w_noise, settings.out_noise
+    if w_noise is not None:
+        w_noise = w_noise.to(device=dev, dtype=dtype).contiguous()
+        assert w_noise.shape == w.shape, "replayed weight noise must be [N,K]"
+    if out_noise is not None:
+        out_noise = out_noise.to(device=dev, dtype=dtype).contiguous()
+        assert out_noise.numel() == t * m * n, "replayed output noise must be [T,M,N]"
+    capture = settings.capture is not None
+    seed = offset = offset_base = 0
+    draw = training and (desc.noise_type != 0 or desc.out_noise > 0)
+    if draw and settings.graph_noise is not None:
+        seed, offset = settings.graph_noise.next()
+        offset_base = settings.graph_noise.counter.data_ptr()
+        draw = False
+    pre_xq, pre_ir, pre_kind = (None, None, 0) if prequant is None else (prequant[0], prequant[1], 2 if pre_codes is not None else 1)
+    status, out, xq, ir_rows, w_amax, w_tile_max, w_mod, keep_mask, codes, codes16, w_planes = _lib.host().forward(
+        desc, ends, x2d, w, bias, ir_data, iridx_data, x_min if fast else None, x_max if fast else None, lwc, std_shared,
+        w_noise, out_noise, pre_xq, pre_ir, pre_codes, pre_kind, modifies, need_std, needs_grad, capture,
+        capture and settings.capture_codes and desc.ir_mode != _lib.AL_IR_OFF, draw, seed, offset, offset_base)
+    _lib.check(status)
+    if static and ir_data is not input_range.data:
+        input_range.data.copy_(ir_data)
 
-    if settings.capture is not None:
+    if capture:
         settings.capture.update(
-            codes=codes, xq=xq, ir_rows=ir_rows, w_amax=w_amax, w_tile_max=w_tile_max[:t],
-            w_mod=w_mod, keep_mask=keep_mask,
-            uses_tcgen05=bool(lib.al_uses_tcgen05(desc, ends)),
+            codes=codes, xq=x2d if xq is None else xq, ir_rows=ir_rows if prequant is None else pre_ir, w_amax=w_amax,
+            w_tile_max=w_tile_max[:t], w_mod=w if w_mod is None else w_mod, keep_mask=keep_mask,
+            uses_tcgen05=bool(_lib.load().al_uses_tcgen05(desc, ends)),
         )
     ctx.desc, ctx.in_sizes, ctx.dtype = desc, list(in_sizes), dtype
     ctx.weight_address = weight.data_ptr()
@@ -426,10 +351,13 @@ def _analog_forward(ctx, inp, weight, bias, input_range, input_range_update_idx,
     ctx.ir_needs_grad = static and input_range is not None and input_range.requires_grad
     ctx.learn_clip = learn_clip
     if needs_grad:
+        if prequant is not None:
+            xq, ir_rows, codes16 = pre_xq, pre_ir, pre_codes if pre_codes is not None else codes16
+        planes = w_planes is not None
         # with bf16 planes the backward GEMMs read those: the fp32 copies need not be kept, except the (small)
         # modified weights of a layer with fewer than 64 channels, whose input gradient runs on the CUDA cores
-        ctx.save_for_backward(x2d if static else None, None if planes else xq,
-                              None if (planes and n >= 64) else w_mod, ir_rows,
+        ctx.save_for_backward(x2d if static else None, None if planes else (x2d if xq is None else xq),
+                              None if (planes and n >= 64) else (w if w_mod is None else w_mod), ir_rows,
                               keep_mask, w if learn_clip else None, lwc, codes16, w_planes)
     return out.view(*inp.shape[:-1], n) if prequant is None else out
 
@@ -440,11 +368,10 @@ def _analog_backward(ctx, grad_out, skip_input_grad=False):
     patch gradient)."""
     if ctx.empty:
         return (None,) * 12
-    lib = _lib.load()
     x2d, xq, w_mod, ir_rows, keep_mask, w_saved, lwc, codes16, w_planes = ctx.saved_tensors
     desc = ctx.desc
     m, k, n, t = desc.M, desc.K, desc.N, desc.T
-    dev, dtype = grad_out.device, ctx.dtype
+    dtype = ctx.dtype
     g = grad_out.reshape(m, n).to(dtype).contiguous()
     need_x, need_w, need_b, need_ir = ctx.needs_input_grad[:4]
     need_x = need_x and not skip_input_grad
@@ -452,66 +379,29 @@ def _analog_backward(ctx, grad_out, skip_input_grad=False):
     need_ir = need_ir and ctx.ir_needs_grad
     need_clip = ctx.learn_clip and (ctx.needs_input_grad[10] or need_w)
     need_w = need_w or need_clip
-    with _OnDevice(dev):
-        args = _lib.AlBackwardArgs()
-        ends = _lib.tile_ends_array(ctx.in_sizes)
-        args.tile_ends = ends
-        args.grad_out, args.x, args.xq, args.w_mod = _ptr(g), _ptr(x2d), _ptr(xq), _ptr(w_mod)
-        args.ir_rows, args.keep_mask = _ptr(ir_rows), _ptr(keep_mask)
-        grad_x = torch.empty(m, k, device=dev, dtype=dtype) if (need_x or need_ir) else None
-        grad_w = None
-        if need_w:
-            if settings.grad_w_alloc is not None and ctx.needs_input_grad[1] and not need_clip:
-                grad_w = settings.grad_w_alloc(ctx.weight_address, (n, k), dtype)
-            if grad_w is None:
-                grad_w = torch.empty(n, k, device=dev, dtype=dtype)
-        grad_b = torch.empty(n, device=dev, dtype=dtype) if need_b else None
-        grad_ir = torch.empty(t, device=dev, dtype=dtype) if need_ir else None
-        scratch = torch.empty(lib.al_backward_scratch_floats(m, k, n, t), device=dev, dtype=torch.float32)
-        args.grad_x, args.grad_w, args.grad_bias = _ptr(grad_x), _ptr(grad_w), _ptr(grad_b)
-        args.grad_input_range, args.reduce_scratch = _ptr(grad_ir), _ptr(scratch)
-        args.reduce_scratch_floats = scratch.numel()
-        g_planes = None
-        if codes16 is not None:
-            g_planes = torch.empty(lib.al_backward_plane_elems(desc, ends), device=dev, dtype=torch.bfloat16)
-            args.codes16, args.w_planes, args.g_planes = _ptr(codes16), _ptr(w_planes), _ptr(g_planes)
-            args.g_planes_elems = g_planes.numel()
-        elif desc.operand_pitch and (n % 8 or g.data_ptr() % 16):
-            g_planes = torch.empty(m * ((n + 7) // 8 * 8), device=dev, dtype=dtype)  # rows TMA can address
-            args.g_planes, args.g_planes_elems = _ptr(g_planes), g_planes.numel()
-        grad_clip = None
-        if need_clip:
-            grad_clip = torch.empty(t, n, device=dev, dtype=dtype)
-            args.w, args.learnable_weight_clip = _ptr(w_saved), _ptr(lwc)
-            args.grad_weight_clip = _ptr(grad_clip)
-        hook = settings.after_wgrad
-        if hook is not None and grad_w is not None and grad_x is not None:
-            # weight-side gradients first: their exchange between replicas can then run while the
-            # input gradient is still being computed
-            args.grad_x = args.grad_input_range = None
-            if settings.comm_sms_wgrad > 0:
-                lib.al_reserve_sms(int(settings.comm_sms_wgrad))
-                try:
-                    _lib.check(lib.al_backward(desc, args, _stream(dev)))
-                finally:
-                    lib.al_reserve_sms(0)
-            else:
-                _lib.check(lib.al_backward(desc, args, _stream(dev)))
+    ends = _lib.tile_ends_array(ctx.in_sizes)
+    grad_w = None
+    if need_w and settings.grad_w_alloc is not None and ctx.needs_input_grad[1] and not need_clip:
+        grad_w = settings.grad_w_alloc(ctx.weight_address, (n, k), dtype)
+    call = _lib.host().backward
+    saved = (desc, ends, g, x2d, xq, w_mod, ir_rows, keep_mask, w_saved, lwc, codes16, w_planes)
+    hook = settings.after_wgrad
+    if hook is not None and need_w and (need_x or need_ir):
+        # weight-side gradients first: their exchange between replicas can then run while the
+        # input gradient is still being computed
+        with _reserved_sms(settings.comm_sms_wgrad):
+            status, _, grad_w, grad_b, _, grad_clip = call(*saved, False, grad_w, True, need_b, False, need_clip)
+        _lib.check(status)
+        hook(grad_w)
+        with _reserved_sms(settings.comm_sms):
+            status, grad_x, _, _, grad_ir, _ = call(*saved, True, None, False, False, need_ir, False)
+        _lib.check(status)
+    else:
+        status, grad_x, grad_w, grad_b, grad_ir, grad_clip = call(*saved, need_x or need_ir, grad_w, need_w, need_b, need_ir,
+                                                                  need_clip)
+        _lib.check(status)
+        if hook is not None and grad_w is not None:
             hook(grad_w)
-            args.grad_x, args.grad_input_range = _ptr(grad_x), _ptr(grad_ir)
-            args.grad_w = args.grad_bias = args.grad_weight_clip = None
-            if settings.comm_sms > 0:
-                lib.al_reserve_sms(int(settings.comm_sms))
-                try:
-                    _lib.check(lib.al_backward(desc, args, _stream(dev)))
-                finally:
-                    lib.al_reserve_sms(0)
-            else:
-                _lib.check(lib.al_backward(desc, args, _stream(dev)))
-        else:
-            _lib.check(lib.al_backward(desc, args, _stream(dev)))
-            if hook is not None and grad_w is not None:
-                hook(grad_w)
     if grad_x is not None:
         grad_x = grad_x.view(ctx.shape) if need_x else None
     if not ctx.needs_input_grad[1]:

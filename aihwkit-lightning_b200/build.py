@@ -1,9 +1,8 @@
-"""Build libanalog_b200.so (sm_100a) in-tree with nvcc.
+"""Build libanalog_b200.so (sm_100a, nvcc) and the Python extension that calls it (g++) in-tree.
 
     python aihwkit-lightning_b200/build.py [--force]
 
-The library lands in ``aihwkit_lightning_b200/lib/`` next to the Python package that loads it
-with ctypes.  nvcc cross-compiles without a GPU.
+Both land in ``aihwkit_lightning_b200/lib/`` next to the Python package that loads them.  nvcc cross-compiles without a GPU.
 """
 import os
 import subprocess
@@ -13,6 +12,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT_DIR = os.path.join(HERE, "aihwkit_lightning_b200", "lib")
 OUT = os.path.join(OUT_DIR, "libanalog_b200.so")
+HOST_OUT = os.path.join(OUT_DIR, "_host_calls.so")
 SOURCES = [
     "api.cu",
     "reduce_kernels.cu",
@@ -36,10 +36,25 @@ NVCC_FLAGS = [
 ]
 
 
+def _host_command():
+    """g++ command of the extension: torch's headers, linked against the library next to it."""
+    import sysconfig
+
+    from torch._C import _GLIBCXX_USE_CXX11_ABI
+    from torch.utils.cpp_extension import include_paths, library_paths
+
+    cuda = os.path.dirname(os.path.dirname(os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")))
+    includes = [*include_paths(), sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
+    return ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={int(_GLIBCXX_USE_CXX11_ABI)}",
+            *[f"-isystem{p}" for p in includes], os.path.join(CSRC, "host_calls.cpp"), "-o", HOST_OUT,
+            *[f"-L{p}" for p in library_paths()], "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python",
+            f"-L{OUT_DIR}", "-l:libanalog_b200.so", "-Wl,-rpath,$ORIGIN"]
+
+
 def _stale() -> bool:
-    if not os.path.exists(OUT):
+    if not os.path.exists(OUT) or not os.path.exists(HOST_OUT):
         return True
-    built = os.path.getmtime(OUT)
+    built = min(os.path.getmtime(OUT), os.path.getmtime(HOST_OUT))
     deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)]
     deps.append(os.path.join(HERE, "..", "include", "analog_b200.h"))
     return any(os.path.getmtime(p) > built for p in deps)
@@ -71,6 +86,10 @@ def build(force: bool = False, verbose: bool = False) -> str:
     if res.returncode != 0:
         sys.stderr.write(res.stdout)
         raise RuntimeError("link failed")
+    res = subprocess.run(_host_command(), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if res.returncode != 0:
+        sys.stderr.write(res.stdout)
+        raise RuntimeError("g++ failed on host_calls.cpp")
     if verbose:
         print("\n".join(log))
     return OUT

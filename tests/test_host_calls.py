@@ -1,0 +1,35 @@
+"""The extension behind ``nn.functional``: arguments it refuses before anything is launched (no GPU needed)."""
+import ctypes
+
+import pytest
+import torch
+
+
+def test_arguments_are_checked():
+    from aihwkit_lightning_b200 import _lib
+
+    host = _lib.host()
+    for fn, count in ((host.forward, 26), (host.backward, 18)):
+        with pytest.raises(ValueError):
+            fn()
+        with pytest.raises(TypeError):  # no descriptor
+            fn(*[None] * count)
+        with pytest.raises(ValueError):  # a descriptor that is too small
+            fn((ctypes.c_int32 * 1)(), (ctypes.c_int32 * 1)(), *[None] * (count - 2))
+        desc, ends = _lib.AlDesc(), (ctypes.c_int32 * 1)(8)
+        desc.M, desc.K, desc.N, desc.T = 4, 8, 8, 2
+        with pytest.raises(ValueError):  # two tiles announced, one end given
+            fn(desc, ends, *[None] * (count - 2))
+        desc.T = 1
+        with pytest.raises(TypeError):  # weights / gradient missing
+            fn(desc, ends, *[None] * (count - 2))
+        with pytest.raises(TypeError):  # not a tensor
+            fn(desc, ends, 1.5, 1.5, *[None] * (count - 4))
+
+
+def test_layer_refuses_cpu_tensors():
+    from aihwkit_lightning_b200.nn import AnalogLinear
+    from aihwkit_lightning_b200.simulator.configs import TorchInferenceRPUConfig
+
+    with pytest.raises(ValueError):
+        AnalogLinear(8, 8, rpu_config=TorchInferenceRPUConfig())(torch.zeros(2, 8))
