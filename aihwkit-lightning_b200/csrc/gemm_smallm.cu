@@ -1,203 +1,224 @@
-// Forward path for a handful of rows (M <= 16, e.g. single-token decoding): the layer is bound by
-// streaming the weights from HBM once, so one kernel reads every (8 output channels x analog
-// tile) block of W exactly once and takes from it both what the model needs of the weights --
-// the per-channel abs-max and the tile maximum -- and the 16 x 8 block of tile dot products
-// (mma.sync m16n8k16, bf16 in, fp32 accumulate; the tensor throughput is irrelevant here, the
-// instruction only saves the CUDA cores the 16 x 8 x k multiply-adds).  The per-tile output stage
-// needs the tile maximum over ALL channels, which is known only when the whole tile has been
-// streamed, so it runs in a second, tiny kernel over the [T, 16, N] fp32 partial results.
+// Forward path for a handful of rows (M <= 16, e.g. single-token decoding): the layer is bound by streaming the weights
+// from HBM once, so one kernel reads every weight exactly once and takes from it both what the model needs of the
+// weights -- the per-channel abs-max and the tile maximum -- and the tile dot products.  The per-tile output stage
+// needs the tile maximum over ALL channels, which is known only when the whole tile has been streamed, so it runs in a
+// second, tiny kernel over the [T, 16, N] fp32 partial results.
 //
-// The DAC runs inside the same kernel: every CTA stages the 16 x tile_w slice of the raw inputs it
-// multiplies with, takes the per-row range of the slice (dynamic input range) and quantises it in
-// shared memory with the arithmetic of the stand-alone DAC pass, so a call of this path has no
-// input pre-pass and no quantised copy of the inputs in HBM.
-//
-// Preconditions (checked by the caller): bf16, equally wide tiles with 16-byte aligned starts,
-// no weight modifier active in this call (the GEMM reads `w` itself) and no output noise.
+// Preconditions (checked by the caller): bf16, equally wide tiles with 16-byte aligned starts, no weight modifier active
+// in this call (the GEMM reads `w` itself) and no output noise.
 #include <cuda_bf16.h>
 
-#include "analog_math.cuh"
-#include "device_fast.cuh"
-#include "internal.h"
+#include "tcgen05_common.cuh"
 
 namespace al {
 
 namespace {
 
-constexpr int kRows = 16;       // rows of one MMA; rows >= M are zero
-constexpr int kWarps = 8;       // warps per CTA, each owns 8 output channels
-constexpr int kChanPerWarp = 8;
+constexpr int kRows = 16;  // columns of one MMA, rows of the layer's input; rows >= M are zero
 
-__device__ __forceinline__ void mma_16x8x16(float c[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                            uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
-      "{%0, %1, %2, %3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
+// A resident CTA per SM walks the (128 channels, analog tile) items with eleven stages of 64 k in flight across item
+// boundaries; the weights are the 128-row operand of tcgen05.mma and the quantised inputs its 16 columns, and eight
+// warps read the same stage once more from shared memory for the abs-max of its channels.  A CTA per (64 channels,
+// tile) with mma.sync, which staged (and quantised) its 16 KiB of inputs for 64 KiB of weights before its first product
+// and left its last wave mostly empty, was slower at every size, calls replayed from a graph, in us (then -> now):
+//   1 x 512 x 512 10.4 -> 8.0, 1 x 4096 x 4096 20.9 -> 16.1, 16 x 8192 x 3072 35.0 -> 25.8, 16 x 3072 x 16384 42.8 -> 33.1.
+// Results differ from 64 bits by the same 1.664e-3 (bf16 outputs) as before.
+constexpr int S_CH = 128;                                  // channels of an item: rows of the MMA
+constexpr int S_W_BYTES = S_CH * BK * 2, S_X_BYTES = kRows * BK * 2;
+constexpr int S_STAGE_BYTES = S_W_BYTES + S_X_BYTES;       // 18 KiB
+constexpr int S_STAGES = 11;
+constexpr int S_CONSUMERS = 256, S_THREADS = 128 + S_CONSUMERS;
+constexpr int S_TMEM_COLS = 32;                            // two accumulators of 16 columns
 
-// pitch of a staged input row in bf16 elements: a multiple of 64 plus 32, so that consecutive rows
-// are 64 bytes apart modulo 128 and the 16-byte reads of a quarter-warp (two rows x four
-// k-chunks) fall on distinct banks
-__host__ __device__ inline int x_pitch(int tile_w) { return ((tile_w + 63) / 64) * 64 + 32; }
+struct StreamBarriers {
+  uint64_t full[S_STAGES], empty[S_STAGES];
+  uint64_t acc_full[2], acc_empty[2];
+  uint64_t mma_done;
+  uint32_t tmem_slot, abort_flag;
+  float amax[S_CH];
+};
+constexpr int S_SMEM = S_STAGES * S_STAGE_BYTES + (int)sizeof(StreamBarriers) + 1024;
 
-// What the in-kernel DAC needs (dac.on == 0: the inputs arrive quantised).
-struct SmallmDac {
-  int on;
-  int ir_mode;               // AL_IR_DYNAMIC or AL_IR_STATIC
-  const uint16_t* ir_static;  // [T] ranges of a static input range
-  float inp_res;
-  int no_rounding;
-  int small_codes;    // |code| stays far below 2^22: the add-based rint applies
-  uint16_t* ir_rows;  // [T][M]: the dynamic ranges, written by the first column of CTAs
+struct StreamParams {
+  int32_t M, N, T, ksteps, num_items;  // item i: channels [128 (i / T), +128) of tile i % T
+  float* acc;                          // [T][16][N]
+  uint16_t* w_amax;                    // [T][N]
+  float* tile_max;                     // [T], zeroed by the caller
 };
 
-// grid: (ceil(N / 64), T).  acc [T][16][N] fp32, w_amax [T][N] bf16, tile_max [T] (float bits,
-// zeroed by the caller).
-__global__ void __launch_bounds__(kWarps * 32)
-smallm_partial_kernel(const uint16_t* __restrict__ xq, int M, int K, const uint16_t* __restrict__ w, int N,
-                      int tile_w, float* __restrict__ acc, uint16_t* __restrict__ w_amax,
-                      float* __restrict__ tile_max, const SmallmDac dac) {
-  extern __shared__ __align__(16) uint16_t x_s[];  // [16][pitch]
-  const int t = blockIdx.y;
-  const int lo = t * tile_w;
-  const int pitch = x_pitch(tile_w);
-  const int vec_per_row = pitch / 8;
+__global__ void __launch_bounds__(S_THREADS, 1)
+smallm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
+                     const StreamParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* const stage_base = align_1024(smem_raw);
+  StreamBarriers* const bars = reinterpret_cast<StreamBarriers*>(stage_base + S_STAGES * S_STAGE_BYTES);
+  volatile uint32_t* const abort_flag = &bars->abort_flag;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int g = lane >> 2, tg = lane & 3;
-  const int n0 = (blockIdx.x * kWarps + warp) * kChanPerWarp;
-  const bool active = n0 < N;
-  const int n = active ? n0 + g : 0;  // the channel whose weights this thread streams (N is a multiple of 8)
-  const uint16_t* wrow = w + (int64_t)n * K + lo;
-  const int chunks = (tile_w + 31) / 32;  // 32 k per step: thread tg covers k = 32 kc + 8 tg .. + 7
-  constexpr int kUnroll = 8;              // 8 x 16 bytes in flight per thread
-  // the first batch of weight loads goes out before the inputs are staged, so that the two
-  // latencies overlap
-  uint4 wv[kUnroll];
-  auto load_batch = [&](int kc0) {
-#pragma unroll
-    for (int u = 0; u < kUnroll; ++u) {
-      const int k = (kc0 + u) * 32 + 8 * tg;
-      wv[u] = (active && kc0 + u < chunks && k < tile_w) ? __ldg(reinterpret_cast<const uint4*>(wrow + k))
-                                                         : make_uint4(0u, 0u, 0u, 0u);
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < S_STAGES; ++s) {
+      mbar_init(&bars->full[s], 1);
+      mbar_init(&bars->empty[s], 1 + S_CONSUMERS / 32);  // the MMAs' commit and the eight warps of the abs-max
     }
-  };
-  load_batch(0);
-  // stage the tile's slice of the inputs; rows >= M and the padding are zero
-  for (int idx = threadIdx.x; idx < kRows * vec_per_row; idx += blockDim.x) {
-    const int m = idx / vec_per_row, v = idx - m * vec_per_row;
-    uint4 val = make_uint4(0u, 0u, 0u, 0u);
-    if (m < M && v * 8 < tile_w) val = *reinterpret_cast<const uint4*>(xq + (int64_t)m * K + lo + v * 8);
-    *reinterpret_cast<uint4*>(x_s + m * pitch + v * 8) = val;
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&bars->acc_full[b], 1);
+      mbar_init(&bars->acc_empty[b], 4);
+    }
+    mbar_init(&bars->mma_done, 1);
+    bars->abort_flag = 0;
+    fence_mbar_init();
   }
+  if (warp == 1) tmem_alloc(&bars->tmem_slot, S_TMEM_COLS);
+  tc_fence_before();
   __syncthreads();
-  if (dac.on) {
-    // DAC of the staged slice by all threads, one 16-byte vector at a time: range of every (row,
-    // tile) segment first, then the element-wise chain of the stand-alone pass (dac_prepare /
-    // dac_apply; its packed bf16 form when rounding is on and the codes are small)
-    __shared__ unsigned int row_bits[kRows];
-    __shared__ QuantSeg row_q[kRows];
-    const int vecs = tile_w / 8, total = M * vecs;
-    if (dac.ir_mode == AL_IR_DYNAMIC) {
-      if (threadIdx.x < kRows) row_bits[threadIdx.x] = 0u;
-      __syncthreads();
-      for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
-        const int m = idx / vecs, v = idx - m * vecs;
-        const uint4 raw = *reinterpret_cast<const uint4*>(x_s + m * pitch + v * 8);
-        __nv_bfloat162 a2 = __hmax2(__habs2(as_bf162(raw.x)), __habs2(as_bf162(raw.y)));
-        a2 = __hmax2(a2, __hmax2(__habs2(as_bf162(raw.z)), __habs2(as_bf162(raw.w))));
-        // non-negative floats order like their bit patterns
-        atomicMax(&row_bits[m], __float_as_uint(fmaxf(__low2float(a2), __high2float(a2))));
-      }
-      __syncthreads();
-    }
-    if (threadIdx.x < M) {
-      float ir;
-      bool clampit = false;
-      if (dac.ir_mode == AL_IR_DYNAMIC) {
-        ir = __uint_as_float(row_bits[threadIdx.x]);
-        if (blockIdx.x == 0) dac.ir_rows[(int64_t)t * M + threadIdx.x] = f32_to_bf16_bits(ir);
-      } else {
-        ir = bf16_bits_to_f32(dac.ir_static[t]);
-        clampit = true;
-      }
-      row_q[threadIdx.x] = dac_prepare<kBF16>(ir, dac.inp_res, clampit, dac.no_rounding != 0);
-    }
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
-      const int m = idx / vecs, v = idx - m * vecs;
-      const QuantSeg q = row_q[m];
-      uint4* slot = reinterpret_cast<uint4*>(x_s + m * pitch + v * 8);
-      const uint4 raw = *slot;
-      uint32_t wd[4] = {raw.x, raw.y, raw.z, raw.w};
-      if (q.quantise && !q.no_rounding && dac.small_codes) {
-        const __nv_bfloat162 b2 = __float2bfloat162_rn(q.bound), nb2 = __float2bfloat162_rn(-q.bound);
-        const __nv_bfloat162 step2 = __float2bfloat162_rn(q.step);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          __nv_bfloat162 x2 = as_bf162(wd[i]);
-          if (q.clampit) x2 = __hmin2_nan(__hmax2_nan(x2, nb2), b2);
-          const __nv_bfloat162 q2 = __floats2bfloat162_rn(fdiv_rcp(__low2float(x2), q.stepc, q.rstep),
-                                                          fdiv_rcp(__high2float(x2), q.stepc, q.rstep));
-          const float c_lo = rint_small(__low2float(q2)), c_hi = rint_small(__high2float(q2));
-          const uint32_t c2 = (__float_as_uint(c_lo) >> 16) | (__float_as_uint(c_hi) & 0xffff0000u);
-          wd[i] = as_u32(__hmul2_rn(as_bf162(c2), step2));
-        }
-      } else {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          float code;
-          const uint32_t lo16 = f32_to_bf16_bits(dac_apply<kBF16>(q, bf16_bits_to_f32((uint16_t)(wd[i] & 0xffffu)), &code));
-          const uint32_t hi16 = f32_to_bf16_bits(dac_apply<kBF16>(q, bf16_bits_to_f32((uint16_t)(wd[i] >> 16)), &code));
-          wd[i] = lo16 | (hi16 << 16);
-        }
-      }
-      *slot = make_uint4(wd[0], wd[1], wd[2], wd[3]);
-    }
-    __syncthreads();
-  }
-  if (!active) return;
+  tc_fence_after();
+  const uint32_t tmem_base = bars->tmem_slot;
 
-  const uint16_t* xa = x_s + g * pitch;
-  const uint16_t* xb = x_s + (g + 8) * pitch;
-  float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-  __nv_bfloat162 m2 = __float2bfloat162_rn(0.0f);
-  for (int kc0 = 0; kc0 < chunks; kc0 += kUnroll) {
-    if (kc0 > 0) load_batch(kc0);
-#pragma unroll
-    for (int u = 0; u < kUnroll; ++u) {
-      if (kc0 + u < chunks) {
-        const int k = (kc0 + u) * 32 + 8 * tg;
-        const uint4 a = *reinterpret_cast<const uint4*>(xa + k);
-        const uint4 b = *reinterpret_cast<const uint4*>(xb + k);
-        // The MMA's k index is a label: this thread supplies the same eight physical k to A and B.
-        mma_16x8x16(c, a.x, b.x, a.y, b.y, wv[u].x, wv[u].y);
-        mma_16x8x16(c, a.z, b.z, a.w, b.w, wv[u].z, wv[u].w);
-        m2 = __hmax2(m2, __habs2(as_bf162(wv[u].x)));
-        m2 = __hmax2(m2, __habs2(as_bf162(wv[u].y)));
-        m2 = __hmax2(m2, __habs2(as_bf162(wv[u].z)));
-        m2 = __hmax2(m2, __habs2(as_bf162(wv[u].w)));
+  if (warp == 0) {
+    // ---- TMA producer --------------------------------------------------------------------
+    if (elect_one()) {
+      tma_prefetch_desc(&map_w);
+      tma_prefetch_desc(&map_x);
+      uint32_t it = 0;
+      bool ok = true;
+      for (int item = blockIdx.x; item < p.num_items && ok; item += gridDim.x) {
+        const int nb = item / p.T, t = item - nb * p.T;
+        for (int ks = 0; ks < p.ksteps; ++ks, ++it) {
+          const int s = it % S_STAGES;
+          if (!mbar_wait(&bars->empty[s], ((it / S_STAGES) & 1u) ^ 1u, abort_flag)) {
+            raise_error(kErrProducer, abort_flag);
+            ok = false;
+            break;
+          }
+          uint8_t* const st = stage_base + s * S_STAGE_BYTES;
+          mbar_expect_tx(&bars->full[s], S_STAGE_BYTES);
+          tma_load_3d(st, &map_w, &bars->full[s], ks * BK, t, nb * S_CH);
+          tma_load_3d(st + S_W_BYTES, &map_x, &bars->full[s], ks * BK, t, 0);
+        }
+      }
+      const uint32_t n_back = it < (uint32_t)S_STAGES ? it : (uint32_t)S_STAGES;
+      for (uint32_t j = it - n_back; j < it; ++j) {  // the last copies must have landed before the CTA exits
+        const uint64_t t0 = globaltimer_ns();
+        while (!mbar_try(&bars->full[j % S_STAGES], (j / S_STAGES) & 1u)) {
+          if (globaltimer_ns() - t0 > wait_limit_ns()) {
+            raise_error(kErrDrain, abort_flag);
+            break;
+          }
+        }
       }
     }
-  }
-  // c0, c1: row g, channels n0 + 2 tg, + 1; c2, c3: row g + 8
-  float* arow = acc + ((int64_t)t * kRows + g) * N + n0 + 2 * tg;
-  *reinterpret_cast<float2*>(arow) = make_float2(c[0], c[1]);
-  *reinterpret_cast<float2*>(arow + (int64_t)8 * N) = make_float2(c[2], c[3]);
-  // abs-max of channel n: over this thread's values, then over the four threads of the channel
-  float amax = fmaxf(__low2float(m2), __high2float(m2));
-  amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-  amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-  if (tg == 0) w_amax[(int64_t)t * N + n] = f32_to_bf16_bits(amax);
-  float wmax = amax;
+  } else if (warp == 1) {
+    // ---- MMA issuer ----------------------------------------------------------------------
+    if (elect_one()) {
+      constexpr uint32_t idesc = make_idesc(S_CH, kRows, 0, 0);
+      uint32_t it = 0, acc_it = 0;
+      bool ok = true;
+      for (int item = blockIdx.x; item < p.num_items && ok; item += gridDim.x, ++acc_it) {
+        const int b = acc_it & 1u;
+        if (!mbar_wait(&bars->acc_empty[b], ((acc_it >> 1) & 1u) ^ 1u, abort_flag)) {
+          raise_error(kErrMma, abort_flag);
+          break;
+        }
+        tc_fence_after();
+        for (int ks = 0; ks < p.ksteps; ++ks, ++it) {
+          const int s = it % S_STAGES;
+          if (!mbar_wait(&bars->full[s], (it / S_STAGES) & 1u, abort_flag)) {
+            raise_error(kErrMma, abort_flag);
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t st = smem_u32(stage_base + s * S_STAGE_BYTES);
+          const uint64_t dw = desc_k_major(st), dx = desc_k_major(st + S_W_BYTES);
 #pragma unroll
-  for (int o = 4; o < 32; o <<= 1) wmax = fmaxf(wmax, __shfl_xor_sync(0xffffffffu, wmax, o));
-  if (lane == 0) {
-    unsigned int* slot = reinterpret_cast<unsigned int*>(tile_max) + t;
-    const unsigned int bits = __float_as_uint(wmax);
-    if (bits > *reinterpret_cast<volatile unsigned int*>(slot)) atomicMax(slot, bits);
+          for (int k4 = 0; k4 < BK / 16; ++k4)
+            umma_bf16(tmem_base + (uint32_t)(b * kRows), dw + (uint64_t)(k4 * 2), dx + (uint64_t)(k4 * 2), idesc,
+                      (ks | k4) != 0 ? 1u : 0u);
+          umma_commit(&bars->empty[s]);
+        }
+        if (ok) umma_commit(&bars->acc_full[b]);
+      }
+      umma_commit(&bars->mma_done);  // retired before the tensor memory is freed
+      const uint64_t t0 = globaltimer_ns();
+      while (!mbar_try(&bars->mma_done, 0)) {
+        if (globaltimer_ns() - t0 > wait_limit_ns()) {
+          raise_error(kErrDrain, abort_flag);
+          break;
+        }
+      }
+    }
+  } else if (warp >= 4) {
+    // ---- abs-max of the channels (all eight warps), accumulators to memory (four of them per item, in turn) ------
+    const int ct = threadIdx.x - 128, row = ct & (S_CH - 1), half = ct >> 7;  // half: 64 of a row's 128 bytes
+    uint32_t it = 0, acc_it = 0;
+    bool ok = true;
+    for (int item = blockIdx.x; item < p.num_items; item += gridDim.x, ++acc_it) {
+      const int nb = item / p.T, t = item - nb * p.T;
+      const int n = nb * S_CH + row;
+      __nv_bfloat162 m2 = __float2bfloat162_rn(0.0f);
+      for (int ks = 0; ks < p.ksteps && ok; ++ks, ++it) {
+        const int s = it % S_STAGES;
+        if (!mbar_wait(&bars->full[s], (it / S_STAGES) & 1u, abort_flag)) {
+          if (lane == 0) raise_error(kErrTransform, abort_flag);
+          ok = false;
+          break;
+        }
+        const uint32_t row_addr = smem_u32(stage_base + s * S_STAGE_BYTES) + (uint32_t)row * 128u;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {  // 16-byte chunk j of a row sits at j ^ (row & 7)
+          uint32_t v[4];
+          asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                       : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+                       : "r"(row_addr + (uint32_t)(((half * 4 + c) ^ (row & 7)) << 4))
+                       : "memory");
+#pragma unroll
+          for (int e = 0; e < 4; ++e) m2 = __hmax2(m2, __habs2(as_bf162(v[e])));
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars->empty[s]);
+      }
+      // the two halves of a row meet in the group whose turn it is to store this item
+      const int b = acc_it & 1u;
+      float amax = fmaxf(__low2float(m2), __high2float(m2));
+      if (half != b) bars->amax[row] = amax;
+      asm volatile("bar.sync 1, %0;" ::"n"(S_CONSUMERS) : "memory");
+      if (half == b) {
+        amax = fmaxf(amax, bars->amax[row]);
+        if (ok && n < p.N) p.w_amax[(int64_t)t * p.N + n] = f32_to_bf16_bits(amax);
+        float wmax = amax;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) wmax = fmaxf(wmax, __shfl_xor_sync(0xffffffffu, wmax, o));
+        if (lane == 0 && ok) {
+          unsigned int* const slot = reinterpret_cast<unsigned int*>(p.tile_max) + t;
+          const unsigned int bits = __float_as_uint(wmax);
+          if (bits > *reinterpret_cast<volatile unsigned int*>(slot)) atomicMax(slot, bits);
+        }
+        if (ok && !mbar_wait(&bars->acc_full[b], (acc_it >> 1) & 1u, abort_flag)) {
+          if (lane == 0) raise_error(kErrEpilogue, abort_flag);
+          ok = false;
+        }
+        if (ok) {
+          tc_fence_after();
+          uint32_t r[kRows];
+          tmem_ld16(tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(b * kRows), r);
+          tmem_wait_ld();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bars->acc_empty[b]);
+          if (n < p.N) {
+            float* const dst = p.acc + (int64_t)t * kRows * p.N + n;
+#pragma unroll
+            for (int m = 0; m < kRows; ++m)
+              if (m < p.M) dst[(int64_t)m * p.N] = __uint_as_float(r[m]);
+          }
+        }
+      }
+      asm volatile("bar.sync 1, %0;" ::"n"(S_CONSUMERS) : "memory");  // amax[] may be written again
+    }
   }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  if (warp == 1) tmem_dealloc(tmem_base, S_TMEM_COLS);
 }
 
 // out[m, n] = sum_t stage_t(acc[t, m, n]) + bias[n]; one thread per output
@@ -232,40 +253,39 @@ int64_t smallm_scratch_floats(int N, int T) { return (int64_t)T * kRows * N; }
 
 bool smallm_forward_supported(int M, int K, int N, const TileTable& tt) {
   if (M < 1 || M > kRows || K % 8 != 0 || N % 8 != 0) return false;
-  const int w = tt.hi(0);
-  for (int t = 1; t < tt.T; ++t)
-    if (tt.hi(t) - tt.lo(t) != w) return false;
-  return w % 8 == 0 && (size_t)kRows * x_pitch(w) * 2 <= 200 * 1024;
+  int w = 0;
+  return uniform_tiles(tt, &w) && w % 8 == 0;
 }
 
 int launch_fwd_smallm(int round_dt, const void* xq, const void* w, int K, const TileTable& tt,
                       const FwdEpilogueParams& ep, void* w_amax, float* tile_max, float* scratch, void* out,
-                      cudaStream_t s, int dac_in_kernel, const void* ir_static, float inp_res, int no_rounding) {
+                      cudaStream_t s, bool tile_max_zeroed) {
   ProfScope prof(AL_K_FWD_GEMM, s, 2);
   const int tile_w = tt.hi(0);
-  const int smem = kRows * x_pitch(tile_w) * 2;
-  cudaError_t e = cudaFuncSetAttribute(smallm_partial_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e == cudaSuccess) e = cudaMemsetAsync(tile_max, 0, sizeof(float) * tt.T, s);
+  int rc = ensure_smem(smallm_stream_kernel, S_SMEM);
+  if (rc) return rc;
+  cudaError_t e = tile_max_zeroed ? cudaSuccess : cudaMemsetAsync(tile_max, 0, sizeof(float) * tt.T, s);
   if (e != cudaSuccess) {
     set_error("fwd_smallm: %s", cudaGetErrorString(e));
     return AL_ERR_CUDA;
   }
-  dim3 grid((ep.N + kWarps * kChanPerWarp - 1) / (kWarps * kChanPerWarp), tt.T);
-  SmallmDac dac;
-  dac.on = dac_in_kernel;
-  dac.ir_mode = ep.ir_mode;
-  dac.ir_static = reinterpret_cast<const uint16_t*>(ir_static);
-  dac.inp_res = inp_res;
-  dac.no_rounding = no_rounding;
-  {
-    const float states = inp_res > 0.0f ? (inp_res > 1.0f ? inp_res : 1.0f / inp_res) : 0.0f;
-    dac.small_codes = states < 4.0e6f;
+  StreamParams p;
+  p.M = ep.M; p.N = ep.N; p.T = tt.T;
+  p.ksteps = (tile_w + BK - 1) / BK;
+  p.num_items = (ep.N + S_CH - 1) / S_CH * tt.T;
+  p.acc = scratch;
+  p.w_amax = reinterpret_cast<uint16_t*>(w_amax);
+  p.tile_max = tile_max;
+  CUtensorMap map_w, map_x;
+  for (int b = 0; b < 2; ++b) {
+    uint64_t dims[3] = {(uint64_t)tile_w, (uint64_t)tt.T, (uint64_t)(b ? ep.M : ep.N)};
+    uint64_t strides[2] = {(uint64_t)tile_w * 2, (uint64_t)K * 2};
+    uint32_t box[3] = {BK, 1, (uint32_t)(b ? kRows : S_CH)};
+    rc = make_map(b ? &map_x : &map_w, b ? xq : w, 3, dims, strides, box);
+    if (rc) return rc;
   }
-  dac.ir_rows = reinterpret_cast<uint16_t*>(const_cast<void*>(ep.ir_rows));
-  smallm_partial_kernel<<<grid, kWarps * 32, smem, s>>>(
-      reinterpret_cast<const uint16_t*>(xq), ep.M, K, reinterpret_cast<const uint16_t*>(w), ep.N, tile_w, scratch,
-      reinterpret_cast<uint16_t*>(w_amax), tile_max, dac);
-  int rc = check_launch("smallm_partial");
+  smallm_stream_kernel<<<p.num_items < sm_count() ? p.num_items : sm_count(), S_THREADS, S_SMEM, s>>>(map_w, map_x, p);
+  rc = check_launch("smallm_stream");
   if (rc) return rc;
   FwdEpilogueParams e2 = ep;
   e2.w_amax = w_amax;
@@ -275,5 +295,8 @@ int launch_fwd_smallm(int round_dt, const void* xq, const void* w, int K, const 
   else smallm_epilogue_kernel<kF32><<<grid2, 256, 0, s>>>(scratch, e2, out);
   return check_launch("smallm_epilogue");
 }
+
+cudaError_t tc_small_take_error_word(uint32_t* code) { return take_error_word(code); }
+cudaError_t tc_small_set_wait_limit(unsigned long long ns) { return set_wait_limit(ns); }
 
 }  // namespace al

@@ -1056,6 +1056,7 @@ int launch_wgrad_tc_f32(const void* g_planes, int sets, const void* codes16, int
 int tc_set_wait_limit(unsigned long long ns) {
   cudaError_t e = set_wait_limit(ns);
   if (e == cudaSuccess) e = tc_fwd_set_wait_limit(ns);
+  if (e == cudaSuccess) e = tc_small_set_wait_limit(ns);
   if (e != cudaSuccess) {
     set_error("al_set_device_wait_limit_ns: %s", cudaGetErrorString(e));
     return AL_ERR_CUDA;
@@ -1065,15 +1066,16 @@ int tc_set_wait_limit(unsigned long long ns) {
 
 int tc_read_device_error(cudaStream_t s, uint32_t* code) {
   cudaError_t e = cudaStreamSynchronize(s);
-  uint32_t fwd_code = 0;
+  uint32_t fwd_code = 0, small_code = 0;
   *code = 0;
   if (e == cudaSuccess) e = take_error_word(code);
   if (e == cudaSuccess) e = tc_fwd_take_error_word(&fwd_code);
+  if (e == cudaSuccess) e = tc_small_take_error_word(&small_code);
   if (e != cudaSuccess) {
     set_error("al_read_device_error: %s", cudaGetErrorString(e));
     return AL_ERR_CUDA;
   }
-  *code |= fwd_code;
+  *code |= fwd_code | small_code;
   if (*code != 0) {
     set_error("a device-side wait of the tcgen05 kernels gave up (role mask 0x%x)", *code);
     return AL_ERR_DEVICE_TIMEOUT;

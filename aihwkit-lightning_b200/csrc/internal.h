@@ -180,7 +180,7 @@ int64_t smallm_scratch_floats(int N, int T);
 bool smallm_forward_supported(int M, int K, int N, const TileTable& tt);
 int launch_fwd_smallm(int round_dt, const void* xq, const void* w, int K, const TileTable& tt,
                       const FwdEpilogueParams& ep, void* w_amax, float* tile_max, float* scratch, void* out,
-                      cudaStream_t s, int dac_in_kernel, const void* ir_static, float inp_res, int no_rounding);
+                      cudaStream_t s, bool tile_max_zeroed);
 
 // ---- tcgen05 GEMMs (gemm_tcgen05_fwd.cu, gemm_tcgen05_bwd.cu) -----------------------------
 bool tc_forward_supported(const AlDesc& d, const TileTable& tt);
@@ -215,6 +215,9 @@ int tc_read_device_error(cudaStream_t s, uint32_t* code);
 // limit of the device-side waits of all tcgen05 kernels (both translation units)
 int tc_set_wait_limit(unsigned long long ns);
 cudaError_t tc_fwd_set_wait_limit(unsigned long long ns);
+// the few-rows translation unit's own limit and error word
+cudaError_t tc_small_set_wait_limit(unsigned long long ns);
+cudaError_t tc_small_take_error_word(uint32_t* code);
 // test aid: the forward kernel's MMA issuer withholds its "accumulator full" signal
 cudaError_t tc_fwd_set_withhold_acc_signal(uint32_t on);
 // the forward translation unit's own error word (read and cleared); the stream must be idle

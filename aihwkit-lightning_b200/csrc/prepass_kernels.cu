@@ -111,7 +111,9 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 dac_kernel(const void* __restrict__ x, int M, int K, TileTable tt, int ir_mode,
            const void* __restrict__ ir_static, float inp_res, int no_rounding,
            void* __restrict__ xq, void* __restrict__ ir_rows, void* __restrict__ codes,
-           uint16_t* __restrict__ codes16, int aligned_base, int small_codes) {
+           uint16_t* __restrict__ codes16, int aligned_base, int small_codes, uint32_t* __restrict__ zero_words,
+           int zero_count) {
+  if (blockIdx.x == 0 && (int)threadIdx.x < zero_count) zero_words[threadIdx.x] = 0u;  // see dac_batched_kernel
   constexpr int VN = Pack<DT>::N;
   constexpr int ES = 16 / VN;
   const unsigned seg = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);  // rows * T < 2^31 (checked by the host)
@@ -522,6 +524,9 @@ int launch_dac(int dtype, const void* x, int M, int K, const TileTable& tt, int 
   float states = inp_res > 0.0f ? (inp_res > 1.0f ? inp_res : 1.0f / inp_res) : 0.0f;
   int small_codes = states < 4.0e6f;
   const int q = batched_q(tt, K);
+  uint32_t* zw = reinterpret_cast<uint32_t*>(zero_words);
+  if (zw == nullptr || zero_count > kWarpsPerBlock * 32) zero_count = 0;
+  if (zeroed) *zeroed = zero_count > 0;
   if (dtype == AL_BF16 && q > 0 && aligned && codes == nullptr && inp_res > 0.0f && !no_rounding && small_codes &&
       (ir_mode == AL_IR_DYNAMIC || ir_mode == AL_IR_STATIC) && aligned16(ir_rows)) {
     const int64_t warps = (int64_t)M * ((tt.T + kBatchVecs / q - 1) / (kBatchVecs / q));
@@ -530,9 +535,6 @@ int launch_dac(int dtype, const void* x, int M, int K, const TileTable& tt, int 
     const uint16_t* irs = reinterpret_cast<const uint16_t*>(ir_static);
     uint16_t* xqs = reinterpret_cast<uint16_t*>(xq);
     uint16_t* irr = reinterpret_cast<uint16_t*>(ir_rows);
-    uint32_t* zw = reinterpret_cast<uint32_t*>(zero_words);
-    if (zw == nullptr || zero_count > kWarpsPerBlock * 32) zero_count = 0;
-    if (zeroed) *zeroed = zero_count > 0;
     switch (q) {
       case 1: dac_batched_kernel<1><<<blocks, kWarpsPerBlock * 32, 0, s>>>(xs, M, K, tt.T, ir_mode, irs, inp_res, xqs, irr, zw, zero_count); break;
       case 2: dac_batched_kernel<2><<<blocks, kWarpsPerBlock * 32, 0, s>>>(xs, M, K, tt.T, ir_mode, irs, inp_res, xqs, irr, zw, zero_count); break;
@@ -542,9 +544,9 @@ int launch_dac(int dtype, const void* x, int M, int K, const TileTable& tt, int 
     return check_launch("dac_batched");
   }
   if (dtype == AL_F32)
-    dac_kernel<kF32><<<seg_blocks(segs), kWarpsPerBlock * 32, 0, s>>>(x, M, K, tt, ir_mode, ir_static, inp_res, no_rounding, xq, ir_rows, codes, static_cast<uint16_t*>(codes16), aligned, small_codes);
+    dac_kernel<kF32><<<seg_blocks(segs), kWarpsPerBlock * 32, 0, s>>>(x, M, K, tt, ir_mode, ir_static, inp_res, no_rounding, xq, ir_rows, codes, static_cast<uint16_t*>(codes16), aligned, small_codes, zw, zero_count);
   else
-    dac_kernel<kBF16><<<seg_blocks(segs), kWarpsPerBlock * 32, 0, s>>>(x, M, K, tt, ir_mode, ir_static, inp_res, no_rounding, xq, ir_rows, codes, nullptr, aligned, small_codes);
+    dac_kernel<kBF16><<<seg_blocks(segs), kWarpsPerBlock * 32, 0, s>>>(x, M, K, tt, ir_mode, ir_static, inp_res, no_rounding, xq, ir_rows, codes, nullptr, aligned, small_codes, zw, zero_count);
   return check_launch("dac");
 }
 
