@@ -403,6 +403,12 @@ int al_forward(const AlDesc* desc, const AlForwardArgs* a, void* stream) {
                       dv.weight_quant == AL_QUANT_NONE && dv.weight_noise == AL_NOISE_NONE &&
                       d.clip_type != AL_CLIP_LEARNABLE_PER_CHANNEL && !d.save_for_backward && a->w_amax &&
                       a->w_tile_max && smallm_forward_supported(d.M, d.K, d.N, tt) && ((uintptr_t)a->w % 16) == 0;
+  // fp32 layer on the tensor cores whose weights need no separate modifier pass: straight to planes
+  const bool weight_planes = tc_f32 && needs_wmax(dv) && dv.weight_quant == AL_QUANT_NONE && !a->w_noise &&
+                             dv.weight_noise != AL_NOISE_ADD_NORMAL && d.clip_type != AL_CLIP_LEARNABLE_PER_CHANNEL &&
+                             a->w_amax && a->w_tile_max && ((uintptr_t)a->w % 16) == 0 && ((uintptr_t)a->w_planes % 16) == 0 &&
+                             ((uintptr_t)a->w_mod % 16) == 0;
+
   // 2. DAC: x -> xq (+ per-row ranges in dynamic mode)
   const void* xq = a->x;
   bool tile_max_zeroed = false;
@@ -419,7 +425,9 @@ int al_forward(const AlDesc* desc, const AlForwardArgs* a, void* stream) {
     if (rc) return rc;
     xq = a->xq;
   } else if (d.ir_mode != AL_IR_OFF) {
-    if (!a->xq || (d.ir_mode == AL_IR_DYNAMIC && !a->ir_rows)) {
+    // fp32 on the tensor cores: without xq only the codes are written
+    const bool codes_only = tc_f32 && !a->xq && !a->codes && ((uintptr_t)a->x % 16) == 0 && ((uintptr_t)a->codes16 % 16) == 0;
+    if ((!a->xq && !codes_only) || (d.ir_mode == AL_IR_DYNAMIC && !a->ir_rows)) {
       set_error("al_forward: xq / ir_rows workspace missing");
       return AL_ERR_BAD_ARGUMENT;
     }
@@ -429,14 +437,20 @@ int al_forward(const AlDesc* desc, const AlForwardArgs* a, void* stream) {
                               dv.weight_quant == AL_QUANT_NONE && dv.weight_noise != AL_NOISE_ADD_NORMAL &&
                               a->w_amax && a->w_tile_max;
     if (fused_weights_next && !smallm && (int64_t)d.M * d.K >= kOverlapMinElems && (int64_t)d.N * d.K >= kOverlapMinElems &&
-        a->w_mod && a->w_mod != a->w) {
+        (weight_planes || (a->w_mod && a->w_mod != a->w))) {
       side = side_stream();
       if (side && cudaEventRecord(side->fork, s) == cudaSuccess && cudaStreamWaitEvent(side->stream, side->fork, 0) == cudaSuccess)
         fused_weights_next = false;  // the weight pass clears its own words: it no longer runs behind the DAC kernel
       else
         side = nullptr;
     }
-    rc = launch_dac(d.dtype, a->x, d.M, d.K, tt, d.ir_mode == AL_IR_FAST ? AL_IR_STATIC : d.ir_mode, ir_static, dv.has_dac ? dv.inp_res : -1.0f,
+    if (codes_only)
+      rc = launch_dac_codes(static_cast<const float*>(a->x), d.M, d.K, tt,
+                            d.ir_mode == AL_IR_FAST ? AL_IR_STATIC : d.ir_mode, static_cast<const float*>(ir_static),
+                            dv.inp_res, a->codes16, static_cast<float*>(a->ir_rows), s,
+                            fused_weights_next ? a->w_tile_max : nullptr, 2 * d.T, &tile_max_zeroed);
+    else
+      rc = launch_dac(d.dtype, a->x, d.M, d.K, tt, d.ir_mode == AL_IR_FAST ? AL_IR_STATIC : d.ir_mode, ir_static, dv.has_dac ? dv.inp_res : -1.0f,
                     d.no_rounding, a->xq, a->ir_rows, a->codes, s, tc_f32 ? a->codes16 : nullptr,
                     fused_weights_next ? a->w_tile_max : nullptr, 2 * d.T, &tile_max_zeroed);
     if (rc) return rc;
@@ -497,13 +511,18 @@ int al_forward(const AlDesc* desc, const AlForwardArgs* a, void* stream) {
     tile_max = (float*)a->w_tile_max;
     int32_t* flags = (int32_t*)(tile_max + d.T);
     const bool modifies = dv.weight_quant != AL_QUANT_NONE || dv.weight_noise != AL_NOISE_NONE;
-    if (modifies && (!a->w_mod || a->w_mod == a->w)) {
+    if (modifies && !weight_planes && (!a->w_mod || a->w_mod == a->w)) {
       set_error("al_forward: w_mod workspace missing (the modifier never writes into w)");
       return AL_ERR_BAD_ARGUMENT;
     }
     if (dv.weight_quant == AL_QUANT_NONE && dv.weight_noise != AL_NOISE_ADD_NORMAL) {
       // every scale the modifier needs is the segment's own abs-max: one sweep over w
-      rc = pitched ? launch_weight_ragged(true, a->w, d.N, d.K, rt, a->w_amax, tile_max, nullptr, AL_QUANT_NONE, 1.0f,
+      rc = weight_planes
+               ? launch_weight_planes(static_cast<const float*>(a->w), d.N, d.K, tt, static_cast<float*>(a->w_amax), tile_max,
+                                      dv.weight_noise, dv.std_dev, a->seed, a->offset, a->offset_base, a->w_planes,
+                                      modifies && a->w_mod != a->w ? static_cast<float*>(a->w_mod) : nullptr,
+                                      side ? side->stream : s, tile_max_zeroed)
+           : pitched ? launch_weight_ragged(true, a->w, d.N, d.K, rt, a->w_amax, tile_max, nullptr, AL_QUANT_NONE, 1.0f,
                                           1.0f, dv.weight_noise, dv.std_dev, a->seed, a->offset, 0, a->w_mod, s,
                                           a->offset_base)
                    : launch_weight_fused(d.dtype, a->w, d.N, d.K, tt, a->w_amax, tile_max, dv.weight_noise,
@@ -566,8 +585,10 @@ int al_forward(const AlDesc* desc, const AlForwardArgs* a, void* stream) {
   ep.offset_base = a->offset_base;
 
   if (tc_f32) {
-    rc = launch_split_planes(static_cast<const float*>(w_mod), (int64_t)d.N * d.K, a->w_planes, s);
-    if (rc) return rc;
+    if (!weight_planes) {
+      rc = launch_split_planes(static_cast<const float*>(w_mod), (int64_t)d.N * d.K, a->w_planes, s);
+      if (rc) return rc;
+    }
     return launch_fwd_tc_f32(a->codes16, a->w_planes, d.K, tt, ep, dv.inp_res, a->out, s);
   }
   if (ragged) return launch_fwd_tc_ragged(dv.round_dt, xq, w_mod, rt, ep, a->out, s);

@@ -147,11 +147,16 @@ PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   // with bf16 planes the backward GEMMs read those: the fp32 copies are kept only for the CUDA-core input gradient
   // of a layer with fewer than 64 channels
   const bool keep_xq = capture || (keep && !planes), keep_wmod = capture || (keep && !(planes && n >= 64));
+  // such a layer writes neither fp32 copy at all where nothing reads it (al_forward: codes_only, weight_planes)
+  const bool codes_only = planes && !capture && !prequant && (uintptr_t)args.x % 16 == 0;
+  const bool planes_only = planes && !capture && !replay && n >= 64 && d.quant_type == AL_QUANT_NONE &&
+                           !(d.training && d.noise_type == AL_NOISE_ADD_NORMAL) &&
+                           d.clip_type != AL_CLIP_LEARNABLE_PER_CHANNEL && (uintptr_t)args.w % 16 == 0;
   if (prequant) {
     args.xq = ptr_of(tensor_or_null(a[F_PRE_XQ]));
     args.ir_rows = ptr_of(tensor_or_null(a[F_PRE_IR]));
   } else if (d.ir_mode != AL_IR_OFF || pitched) {
-    place(keep_xq, &xq, &args.xq, {m, k_rows}, type);
+    if (!codes_only) place(keep_xq, &xq, &args.xq, {m, k_rows}, type);
     if (is_static) place(keep || capture, &ir_rows, &args.ir_rows, {t}, type);
     else place(keep || capture, &ir_rows, &args.ir_rows, {t, m}, type);
   } else {
@@ -159,7 +164,8 @@ PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   }
   place(capture, &w_amax, &args.w_amax, {t, n}, type);
   place(capture, &w_tile_max, &args.w_tile_max, {2 * t}, at::kFloat);
-  if (modifies || pitched) place(keep_wmod, &w_mod, &args.w_mod, {n, k_rows}, type);
+  if (modifies && planes_only) args.w_mod = nullptr;
+  else if (modifies || pitched) place(keep_wmod, &w_mod, &args.w_mod, {n, k_rows}, type);
   else args.w_mod = const_cast<void*>(args.w);
   if (d.out_bound > 0 && keep) place(true, &keep_mask, reinterpret_cast<void**>(&args.keep_mask), {t, (n + 31) / 32, m}, at::kInt);
   if (need_std) arena.add(reinterpret_cast<void**>(&args.std_scratch), al_std_scratch_floats(d.M, d.T) * 4);

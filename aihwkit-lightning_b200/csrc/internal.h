@@ -111,6 +111,13 @@ int launch_dac(int dtype, const void* x, int M, int K, const TileTable& tt, int 
 // GEMM inside the 1e-5 relative bar of fp32 layers at two (one exact operand) or three (both split)
 // plane products.
 constexpr int kPlanes = 2;
+// DAC of such a layer: the integer codes as bf16 and, with dynamic ranges, the ranges (launch_dac without xq)
+int launch_dac_codes(const float* x, int M, int K, const TileTable& tt, int ir_mode, const float* ir_static, float inp_res,
+                     void* codes16, float* ir_rows, cudaStream_t s, void* zero_words, int zero_count, bool* zeroed);
+// launch_weight_fused + launch_split_planes in one pass (internal noise only); w_mod may be null
+int launch_weight_planes(const float* w, int N, int K, const TileTable& tt, float* w_amax, float* tile_max, int noise_type,
+                         float std_dev, uint64_t seed, uint64_t offset, const uint64_t* offset_base, void* planes,
+                         float* w_mod, cudaStream_t s, bool tile_max_zeroed);
 // planes [kPlanes][count] bf16 (count % 4 == 0)
 int launch_split_planes(const float* src, int64_t count, void* planes, cudaStream_t s);
 // planes [sets][kPlanes][M][N] of g * keep_t * step(row, tile t): keep_mask null = nothing masked (sets

@@ -118,13 +118,17 @@ typedef struct AlForwardArgs {
   void* out;                 /* [M,N] dtype                                                 */
   /* saved for backward / intermediates (caller-allocated workspace) */
   void* xq;                  /* [M,K] dtype: DAC output fed to the GEMM. May equal x when
-                                 the input range and the DAC are both off                  */
+                                 the input range and the DAC are both off; may be null for an fp32
+                                 layer on the tensor cores (x and codes16 16-byte aligned), which
+                                 reads the codes only                                      */
   void* ir_rows;             /* [T,M] dtype (dynamic mode) or [T] dtype (static mode: the
                                  ranges actually used by this call)                        */
   void* w_amax;              /* [T,N] dtype per-tile per-channel abs-max of w               */
   void* w_tile_max;          /* [T] float  per-tile abs-max of w + [T] int32 flags behind it */
   void* w_mod;               /* [N,K] dtype modified weights; may equal w when the modifier
-                                 does nothing in this call                                  */
+                                 does nothing in this call; may be null for an fp32 layer on the
+                                 tensor cores without discretisation, per-tensor or replayed noise and
+                                 learned ranges (w and w_planes 16-byte aligned)             */
   uint32_t* keep_mask;       /* [T, ceil(N/32), M] word (t, n/32, m), bit n%32 = 1 where the
                                  ADC clamp of tile t passes the gradient of out[m, n];
                                  nullable if out_bound <= 0                                 */
