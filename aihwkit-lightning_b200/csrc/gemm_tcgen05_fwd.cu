@@ -56,7 +56,7 @@ __device__ __forceinline__ void normals16(uint64_t seed, uint64_t offset, uint64
 
 // MODE >= 0: the output stage is fixed at compile time (bit 0 output noise from the internal
 // generator, bit 1 ADC quantisation, bit 2 clamp; reference rounding, per-tile scalar scales,
-// rounding on, small ADC codes).  MODE < 0: every switch is read at run time.
+// rounding on, small ADC codes; fp32 layers: modes 0 and 1 only).  MODE < 0: every switch is read at run time.
 //
 // PAIR: launched as clusters of two CTAs that share one tcgen05.mma.cta_group::2 of 256 x 256
 // per k-step (an MMA that is 256 columns wide runs the tensor cores at their full rate, one of
@@ -69,6 +69,12 @@ __device__ __forceinline__ void normals16(uint64_t seed, uint64_t offset, uint64
 // `full` collects both CTAs' copies in the leader, `empty` and `acc_full` are signalled in both
 // CTAs by the leader's multicast commits, `acc_empty` collects both CTAs' epilogue warps in the
 // leader.
+//
+// fp32 layers run pairs with 256 x 128 blocks: two accumulators and the fp32 running sum (128 columns each) fit the
+// tensor memory, and a CTA stages 32 KiB per k-step for both planes where a single one stages 48 for the same products.
+// 4096^3 with output noise on eight tiles: 295 us on single CTAs, 275 us on pairs, 205 us with the output stage fixed
+// at compile time (MODE); 178 us with one tile, where the MMAs are the bound.  One 256-column MMA over both planes
+// side by side, with the running sum in shared memory, was slower (287 us; 180 us with one tile).
 //
 // IO: element type of the layer's tensors (input ranges, bias, replayed noise, per-channel scales,
 // outputs).  RAG: the row pitch of the outputs is no multiple of 8 (single CTAs, run-time output stage only): the
@@ -86,15 +92,16 @@ __global__ void __launch_bounds__(fwd_threads(PAIR, BN), 1)
 fwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
               const FwdTcParams p) {
   constexpr int kPlanesB = IO == kF32 ? kPlanes : 1;           // planes of the weights per stage
-  constexpr int kStages = PAIR ? FP_STAGES : fwd_stages(BN, kPlanesB);
+  constexpr bool kSumSmem = PAIR && IO == kBF16;               // running sum in shared memory, else in tensor memory
+  constexpr int kStages = kSumSmem ? FP_STAGES : fwd_stages(BN, kPlanesB);
   constexpr int kBRows = BN;                                   // weight rows this CTA stages
   constexpr int kPlaneBytes = kBRows * BK * 2;
   constexpr int kStageBytes = fwd_stage_bytes(BN, kPlanesB);
   constexpr int kEpiWarps = fwd_epi_warps(PAIR, BN);
-  static_assert(!PAIR || (BN == F_BN && IO == kBF16), "CTA pairs: 256 x 256 blocks of bf16 layers");
+  static_assert(!PAIR || BN == (IO == kBF16 ? 128 : 64), "CTA pairs: 256 x 256 blocks of bf16, 256 x 128 of fp32 layers");
   constexpr int kBlockRows = PAIR ? 2 * BM : BM;               // rows of the outputs per work item
   constexpr int kBN = PAIR ? 2 * BN : BN;                      // columns of the outputs per work item
-  constexpr int kSumBytes = PAIR ? FP_SUM_BYTES : 0;
+  constexpr int kSumBytes = kSumSmem ? FP_SUM_BYTES : 0;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* stage_base = align_1024(smem_raw);
   uint8_t* sum_base = stage_base + kStages * kStageBytes;      // PAIR: [128 rows][256 bf16], 16-byte chunks swizzled
@@ -159,7 +166,14 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
               if (leader) mbar_expect_tx(&bars->full[s], 2 * kStageBytes);
               const uint32_t bar = mapa_u32(smem_u32(&bars->full[s]), 0);
               tma_load_3d_pair(sa, &map_a, bar, ks * BK, t, mb * kBlockRows + row_off);
-              tma_load_3d_pair(sa + F_A_BYTES, &map_b, bar, ks * BK, t, nb * kBN + (int)rank * kBRows);
+              if (IO == kF32) {
+#pragma unroll
+                for (int plane = 0; plane < kPlanesB; ++plane)
+                  tma_load_4d_pair(sa + F_A_BYTES + plane * kPlaneBytes, &map_b, bar, ks * BK, t,
+                                   nb * kBN + (int)rank * kBRows, plane);
+              } else {
+                tma_load_3d_pair(sa + F_A_BYTES, &map_b, bar, ks * BK, t, nb * kBN + (int)rank * kBRows);
+              }
             } else {
               mbar_expect_tx(&bars->full[s], (uint32_t)(p.a_rows * BK * 2 + kPlanesB * kPlaneBytes));
               tma_load_3d(sa, &map_a, &bars->full[s], ks * BK, t, mb * BM);
@@ -271,7 +285,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
     // one draw per output at the last tile replaces T draws -- same distribution up to the bf16
     // rounding of the partial sums, an eighth of the generator work on an 8-tile layer.  Replayed
     // noise (parity runs) never takes this route: it is applied tile by tile as given.
-    constexpr bool kMergedNoise = kFixed && MODE == 1;
+    constexpr bool kMergedNoise = kFixed && MODE == 1 && IO == kBF16;
     float noise_var = 0.0f;
     TileEpilogueCfg cfg;
     cfg.has_noise = ep.has_noise; cfg.has_bound = ep.has_bound; cfg.has_adc = ep.has_adc;
@@ -351,7 +365,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
           uint32_t accr[16], sumr[16];
           tmem_ld16(tmem_base + lane_base + (uint32_t)(b * kBN + cc), accr);
           if (t > 0) {
-            if (PAIR) {
+            if (kSumSmem) {
 #pragma unroll
               for (int v = 0; v < 2; ++v) {
                 const uint32_t addr = sum_row + (uint32_t)((((cc >> 3) + v) ^ (srow & 7)) << 4);
@@ -360,9 +374,9 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
                              : "r"(addr) : "memory");
               }
             } else if (packed) {
-              tmem_ld8(tmem_base + lane_base + (uint32_t)(2 * BN + (cc >> 1)), sumr);
+              tmem_ld8(tmem_base + lane_base + (uint32_t)(2 * kBN + (cc >> 1)), sumr);
             } else {
-              tmem_ld16(tmem_base + lane_base + (uint32_t)(2 * BN + cc), sumr);
+              tmem_ld16(tmem_base + lane_base + (uint32_t)(2 * kBN + cc), sumr);
             }
           }
           tmem_wait_ld();
@@ -370,7 +384,23 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
 #pragma unroll
             for (int j = 0; j < 16; ++j) accr[j] = __float_as_uint(fmul(__uint_as_float(accr[j]), dac_step));
           }
-          if constexpr (kFixed) {
+          if constexpr (kFixed && IO == kF32) {
+            // ---- fp32 layer without ADC and clamp: noise and running sum --------------------------
+            float z[16];
+            if (has_noise) {
+#pragma unroll
+              for (int g8 = 0; g8 < 2; ++g8) {
+                const int nq = nh + g8 * 8;
+                normal8_keyed(p.noise, noise_ctr, row_group8 + (uint32_t)((nq < N ? nq : 0) >> 3), &z[g8 * 8]);
+              }
+            }
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+              float o = __uint_as_float(accr[j]);
+              if (has_noise) o = fadd(o, fmul(sc, z[j]));
+              sumr[j] = __float_as_uint(fadd(t == 0 ? 0.0f : __uint_as_float(sumr[j]), o));
+            }
+          } else if constexpr (kFixed) {
             // ---- output stage fixed at compile time: everything in packed bf16 arithmetic --------
             if (t == 0) {
 #pragma unroll
@@ -512,7 +542,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
           }
           }  // !kFixed
           if (t < T - 1) {
-            if (PAIR) {
+            if (kSumSmem) {
 #pragma unroll
               for (int v = 0; v < 2; ++v) {
                 const uint32_t addr = sum_row + (uint32_t)((((cc >> 3) + v) ^ (srow & 7)) << 4);
@@ -520,9 +550,9 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
                              "r"(sumr[4 * v + 1]), "r"(sumr[4 * v + 2]), "r"(sumr[4 * v + 3]) : "memory");
               }
             } else if (packed) {
-              tmem_st8(tmem_base + lane_base + (uint32_t)(2 * BN + (cc >> 1)), sumr);
+              tmem_st8(tmem_base + lane_base + (uint32_t)(2 * kBN + (cc >> 1)), sumr);
             } else {
-              tmem_st16(tmem_base + lane_base + (uint32_t)(2 * BN + cc), sumr);
+              tmem_st16(tmem_base + lane_base + (uint32_t)(2 * kBN + cc), sumr);
             }
           } else if (RAG) {
             // final (ragged outputs): bias, convert, transpose through this warp's staging buffer
@@ -653,10 +683,9 @@ static FwdKernel pick_fwd_kernel(int mode, int round_dt) {
 }
 
 // Columns of a single CTA's block (128, 64 or 32), or 0 when CTA pairs are the better choice
-static int fwd_block_columns(int M, int N, int n_pairs = 0) {
-  const int64_t pair_blocks = (int64_t)((M + 2 * BM - 1) / (2 * BM)) * ((N + 2 * F_BN - 1) / (2 * F_BN));
+static int fwd_block_columns(int M, int N, int n_pairs = 0, int64_t pair_blocks = 0, int planes = 1) {
   return pick_blocks(n_pairs, pair_blocks, sm_count(), 128, 32,
-                     [&](int bn) { return (int64_t)((M + BM - 1) / BM) * ((N + bn - 1) / bn); });
+                     [&](int bn) { return (int64_t)((M + BM - 1) / BM) * ((N + bn - 1) / bn); }, planes);
 }
 
 static int fwd_copy_rows(int M) { return M < BM ? (M + 7) / 8 * 8 : BM; }
@@ -676,7 +705,7 @@ static int max_fwd_pairs(FwdKernel kernel, int smem) {
   for (int i = 0; i < n_seen; ++i)
     if (seen[i] == kernel) return count[i];
   int clusters = 0;
-  PairLaunch pl(2 * sm_count(), fwd_threads(true, F_BN), smem, nullptr);
+  PairLaunch pl(2 * sm_count(), fwd_threads(true, F_BN), smem, nullptr);  // every pair kernel has that many threads
   if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &pl.cfg) != cudaSuccess) {
     cudaGetLastError();
     clusters = 0;
@@ -727,7 +756,7 @@ int launch_fwd_tc(int round_dt, const void* xq, const void* w_mod, int K, const 
     if (rc) return rc;
     pairs = max_fwd_pairs(kernel, pair_smem);
   }
-  const int columns = pairing > 0 && pairs > 0 ? 0 : fwd_block_columns(ep.M, ep.N, pairs);
+  const int columns = pairing > 0 && pairs > 0 ? 0 : fwd_block_columns(ep.M, ep.N, pairs, pair_tiles);
   const bool pair = columns == 0;
   const int bn = pair ? F_BN : columns;
   const int single_smem = fwd_smem(bn, 1);
@@ -840,9 +869,15 @@ bool tc_f32_supported(const AlDesc& d, const TileTable& tt) {
   return states <= 510.0;
 }
 
+template <bool PAIR, int BN>
+static FwdKernel pick_f32_kernel(int mode) {
+  return mode == 0   ? fwd_tc_kernel<kF32, 0, PAIR, kF32, false, BN>
+         : mode == 1 ? fwd_tc_kernel<kF32, 1, PAIR, kF32, false, BN>
+                     : fwd_tc_kernel<kF32, -1, PAIR, kF32, false, BN>;
+}
+
 // Forward of an fp32 layer on the tensor cores: A = DAC codes as bf16 [M,K], B = the bf16 planes of the
-// modified weights [kPlanes][N][K]; single CTAs (128 x 128 blocks, fp32 running sum in tensor memory), every
-// output-stage switch read at run time.
+// modified weights [kPlanes][N][K]; fp32 running sum in tensor memory.
 int launch_fwd_tc_f32(const void* codes16, const void* w_planes, int K, const TileTable& tt,
                       const FwdEpilogueParams& ep, float inp_res, void* out, cudaStream_t s) {
   ProfScope prof(AL_K_FWD_GEMM, s);
@@ -856,19 +891,34 @@ int launch_fwd_tc_f32(const void* codes16, const void* w_planes, int K, const Ti
   p.ksteps = (w + BK - 1) / BK;
   p.num_mb = (ep.M + BM - 1) / BM;
   p.a_rows = fwd_copy_rows(ep.M);
-  const int bn = fwd_block_columns(ep.M, ep.N);
-  p.num_nb = (ep.N + bn - 1) / bn;
+  const bool per_channel = ep.w_amax != nullptr && (ep.noise_pc || ep.bound_pc);
+  const bool fixed = !ep.has_adc && !ep.has_bound && !per_channel && ep.out_noise == nullptr;
+  const int mode = fixed ? (ep.has_noise ? 1 : 0) : -1;
+  FwdKernel kernel = pick_f32_kernel<true, 64>(mode);
+  int rc = ensure_smem(kernel, fwd_smem(64, kPlanes));
+  if (rc) return rc;
+  const int pairs = max_fwd_pairs(kernel, fwd_smem(64, kPlanes));
+  const int64_t pair_blocks = (int64_t)((ep.M + 2 * BM - 1) / (2 * BM)) * ((ep.N + BM - 1) / BM);
+  const int columns = fwd_block_columns(ep.M, ep.N, pairs, pair_blocks, kPlanes);
+  const bool pair = columns == 0;
+  const int bn = pair ? 64 : columns;  // weight rows a CTA stages
+  p.num_nb = pair ? (ep.N + BM - 1) / BM : (ep.N + bn - 1) / bn;
+  if (pair) {
+    p.num_mb = (ep.M + 2 * BM - 1) / (2 * BM);
+    p.a_rows = BM;
+  }
   p.ep = ep;
   p.noise = make_noise_keys(ep.seed, ep.offset, 1u, ep.offset_base);
   p.out = out;
   p.inp_res = inp_res;
   p.small_adc_codes = 0;  // fp32 accumulators: guarded rint
-  FwdKernel kernel = bn == 128  ? fwd_tc_kernel<kF32, -1, false, kF32, false, 128>
-                     : bn == 64 ? fwd_tc_kernel<kF32, -1, false, kF32, false, 64>
-                                : fwd_tc_kernel<kF32, -1, false, kF32, false, 32>;
   const int smem = fwd_smem(bn, kPlanes);
-  int rc = ensure_smem(kernel, smem);
-  if (rc) return rc;
+  if (!pair) {
+    kernel = bn == 128  ? pick_f32_kernel<false, 128>(mode)
+             : bn == 64 ? pick_f32_kernel<false, 64>(mode) : pick_f32_kernel<false, 32>(mode);
+    rc = ensure_smem(kernel, smem);
+    if (rc) return rc;
+  }
   CUtensorMap map_a, map_b;
   {
     uint64_t dims[3] = {(uint64_t)w, (uint64_t)tt.T, (uint64_t)ep.M};
@@ -885,6 +935,15 @@ int launch_fwd_tc_f32(const void* codes16, const void* w_planes, int K, const Ti
     if (rc) return rc;
   }
   const int tiles = p.num_mb * p.num_nb;
+  if (pair) {
+    PairLaunch pl(2 * (tiles < pairs ? tiles : pairs), fwd_threads(true, bn), smem, s);
+    const cudaError_t e = cudaLaunchKernelEx(&pl.cfg, kernel, map_a, map_b, p);
+    if (e != cudaSuccess) {
+      set_error("fwd_tc_f32 (pairs): %s", cudaGetErrorString(e));
+      return AL_ERR_CUDA;
+    }
+    return check_launch("fwd_tc_f32_pair");
+  }
   const int grid = tiles < sm_count() ? tiles : sm_count();
   kernel<<<grid, fwd_threads(false, bn), smem, s>>>(map_a, map_b, p);
   return check_launch("fwd_tc_f32");

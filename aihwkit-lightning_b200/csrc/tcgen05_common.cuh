@@ -255,6 +255,14 @@ __device__ __forceinline__ void tma_load_3d_pair(void* dst, const CUtensorMap* m
       ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(c0), "r"(c1), "r"(c2)
       : "memory");
 }
+__device__ __forceinline__ void tma_load_4d_pair(void* dst, const CUtensorMap* map, uint32_t bar_cluster_addr,
+                                                 int c0, int c1, int c2, int c3) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes "
+      "[%0], [%1, {%3, %4, %5, %6}], [%2];"
+      ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+      : "memory");
+}
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t* slot, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "r"(ncols)
                : "memory");
@@ -473,14 +481,14 @@ constexpr int bwd_smem(int bn) { return bwd_stages(bn) * bwd_stage_bytes(bn) + (
 // the copies, and CTA pairs are taken as soon as they save a round (64 pairs instead of 256 single blocks at 1024 x
 // 4096).  Against 128-wide (forward) and 128- or 256-wide (backward) blocks throughout: 1.12x (geometric mean of 41 sizes
 // from 17 x 1024 x 1024 to 4096^3), 512 x 1024 x 1024 training 39.8 -> 33.9 us, 2048^3 105 -> 82, none slower by over 1 %.
-// n_pairs: CTA pairs the device runs at once (0: none), pair_blocks their 256 x 256 blocks; blocks_of(bn): blocks of
-// 128 x bn columns.  Returns 0 for pairs, else the block width; the narrower of two that cost the same.
+// n_pairs: CTA pairs the device runs at once (0: none), pair_blocks their blocks (32 KiB per CTA and k-step);
+// blocks_of(bn): blocks of 128 x bn columns, which stage `planes` planes of their second operand.  Returns 0 for pairs, else the block width; the narrower of two that cost the same.
 template <class BlocksOf>
-int pick_blocks(int n_pairs, int64_t pair_blocks, int sms, int widest, int narrowest, BlocksOf blocks_of) {
+int pick_blocks(int n_pairs, int64_t pair_blocks, int sms, int widest, int narrowest, BlocksOf blocks_of, int planes = 1) {
   int best = 0;
   int64_t cost = n_pairs > 0 ? (pair_blocks + n_pairs - 1) / n_pairs * 32 : INT64_MAX;
   for (int bn = widest; bn >= narrowest; bn /= 2) {
-    const int64_t c = (blocks_of(bn) + sms - 1) / sms * (16 + bn / 8);
+    const int64_t c = (blocks_of(bn) + sms - 1) / sms * (16 + planes * bn / 8);
     if (c <= cost) {
       cost = c;
       best = bn;
@@ -491,13 +499,28 @@ int pick_blocks(int n_pairs, int64_t pair_blocks, int sms, int widest, int narro
 constexpr int P_SMEM = P_STAGES * P_STAGE_BYTES + (int)sizeof(Barriers) + 1024;
 constexpr int FP_SMEM = FP_STAGES * F_STAGE_BYTES + FP_SUM_BYTES + (int)sizeof(Barriers) + 1024;
 
+// Opts a kernel in to its dynamic shared memory, once per host thread and device (the attribute belongs to the device's
+// context; a kernel always asks for the same size).  The first call of a thread also binds the device's context to it.
 template <class Kernel>
 int ensure_smem(Kernel k, int bytes) {
+  struct Seen {
+    const void* kernel;
+    int device;
+  };
+  constexpr int kSeen = 64;  // more kernels than a translation unit has; beyond it the call is simply repeated
+  thread_local Seen seen[kSeen];
+  thread_local int n_seen = 0;
+  int device = -1;
+  if (cudaGetDevice(&device) != cudaSuccess) device = -1;
+  const void* const key = reinterpret_cast<const void*>(k);
+  for (int i = 0; i < n_seen; ++i)
+    if (seen[i].kernel == key && seen[i].device == device) return AL_OK;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   if (e != cudaSuccess) {
     set_error("cudaFuncSetAttribute(%d bytes): %s", bytes, cudaGetErrorString(e));
     return AL_ERR_CUDA;
   }
+  if (device >= 0 && n_seen < kSeen) seen[n_seen++] = Seen{key, device};
   return AL_OK;
 }
 
