@@ -85,6 +85,7 @@ SYMBOLS = {
     "al_f32_planes": (c_int32, []),
     "al_clip_weights": (c_int32, [c_int32, c_void_p, c_int32, c_int32, c_int32, c_float, c_void_p, c_void_p]),
     "al_unfold2d": (c_int32, [c_int32, c_void_p] + [c_int32] * 12 + [c_void_p, c_void_p]),
+    "al_transpose_images": (c_int32, [c_int32, c_void_p, c_int32, c_int32, c_int32, c_void_p, c_void_p]),
     "al_fold2d": (c_int32, [c_int32, c_void_p] + [c_int32] * 12 + [c_void_p, c_void_p]),
     "al_conv2d_input_grad_supported": (c_int32, [c_int32] * 14),
     "al_conv2d_input_grad": (c_int32, [c_int32, c_void_p, c_void_p] + [c_int32] * 13 + [c_void_p, c_void_p]),

@@ -542,15 +542,25 @@ def _direct_input_grad(ctx, grad_out):
     return grad_img
 
 
+def _transpose_images(src: Tensor, batch: int, rows: int, cols: int) -> Tensor:
+    """``[batch, rows, cols] -> [batch, cols, rows]``, both contiguous."""
+    out = torch.empty(batch, cols, rows, device=src.device, dtype=src.dtype)
+    with _OnDevice(src.device):
+        _lib.check(_lib.load().al_transpose_images(_DTYPE[src.dtype], src.data_ptr(), batch, rows, cols, out.data_ptr(),
+                                                   _stream(src.device)))
+    return out
+
+
 class AnalogConv2dFunction(torch.autograd.Function):
     """Analog convolution with a dynamic input range as ONE operator: the patch extraction quantises on
     the way (``al_unfold2d_dac``), the tiled GEMM consumes the quantised patches, and the backward folds
     the patch gradients back into the image.  Same values as ``unfold2d`` followed by ``analog_linear``;
-    the unquantised patch matrix is never written.  Returns ``[B * Ho * Wo, out_channels]``."""
+    the unquantised patch matrix is never written.  Returns images ``[B, out_channels, Ho, Wo]`` with
+    ``as_image`` (and takes their gradient), else rows ``[B * Ho * Wo, out_channels]``."""
 
     @staticmethod
     def forward(ctx, inp, weight, bias, input_range, input_range_update_idx, in_sizes, training, rpu_config,
-                x_min, x_max, learnable_weight_clip, grad_enabled, geometry):  # type: ignore[override]
+                x_min, x_max, learnable_weight_clip, grad_enabled, geometry, as_image=False):  # type: ignore[override]
         lib = _lib.load()
         xc = inp.contiguous()
         b, c, h, w = xc.shape
@@ -575,13 +585,17 @@ class AnalogConv2dFunction(torch.autograd.Function):
         if status == _lib.AL_ERR_UNSUPPORTED:
             raise _PatchTooLarge()
         _lib.check(status)
-        ctx.geom, ctx.dtype_code = geom, _DTYPE[xc.dtype]
-        return _analog_forward(ctx, xc, weight, bias, input_range, input_range_update_idx, in_sizes, training,
-                               rpu_config, x_min, x_max, learnable_weight_clip, grad_enabled,
-                               prequant=(xq, ir_rows, codes16, rows, k))
+        ctx.geom, ctx.dtype_code, ctx.as_image = geom, _DTYPE[xc.dtype], as_image
+        out = _analog_forward(ctx, xc, weight, bias, input_range, input_range_update_idx, in_sizes, training,
+                              rpu_config, x_min, x_max, learnable_weight_clip, grad_enabled,
+                              prequant=(xq, ir_rows, codes16, rows, k))
+        return _transpose_images(out, b, ho * wo, out.shape[1]).view(b, -1, ho, wo) if as_image else out
 
     @staticmethod
     def backward(ctx, grad_out):  # type: ignore[override]
+        if ctx.as_image:
+            b, n = grad_out.shape[:2]
+            grad_out = _transpose_images(grad_out.to(ctx.dtype).contiguous(), b, n, grad_out.shape[2] * grad_out.shape[3])
         direct = _direct_input_grad_applies(ctx)
         grads = _analog_backward(ctx, grad_out, skip_input_grad=direct)  # weight-side gradients first
         grad_img = _direct_input_grad(ctx, grad_out) if direct else None
@@ -592,7 +606,7 @@ class AnalogConv2dFunction(torch.autograd.Function):
             grad_img = torch.empty(b, c, h, w, device=gp.device, dtype=gp.dtype)
             with _OnDevice(gp.device):
                 _lib.check(lib.al_fold2d(ctx.dtype_code, gp.data_ptr(), *ctx.geom, grad_img.data_ptr(), _stream(gp.device)))
-        return (grad_img,) + tuple(grads[1:]) + (None,)
+        return (grad_img,) + tuple(grads[1:]) + (None, None)
 
 
 class _PatchTooLarge(Exception):
@@ -600,9 +614,11 @@ class _PatchTooLarge(Exception):
 
 
 def analog_conv2d_rows(inp: Tensor, weight2d: Tensor, bias, input_range, input_range_update_idx, in_sizes, training,
-                       rpu_config, x_min, x_max, learnable_weight_clip, kernel_size, dilation, padding, stride):
+                       rpu_config, x_min, x_max, learnable_weight_clip, kernel_size, dilation, padding, stride,
+                       as_image=False):
     """``[B, C, H, W] -> [B * Ho * Wo, out_channels]`` (or ``[Ho * Wo, out]`` for a 3-D input): patches through the
-    analog linear operator.  Dynamic input ranges with the DAC on take the fused operator."""
+    analog linear operator.  Dynamic input ranges with the DAC on take the fused operator, which with ``as_image``
+    returns images ``[B, out_channels, Ho, Wo]`` instead; the other routes return rows all the same."""
     irp = rpu_config.pre_post.input_range
     fused = (inp.dim() == 4 and inp.is_cuda and irp.enable and irp.dynamic and not irp.fast_mode
              and rpu_config.forward.inp_res > 0 and not settings.no_rounding and settings.capture is None
@@ -615,9 +631,9 @@ def analog_conv2d_rows(inp: Tensor, weight2d: Tensor, bias, input_range, input_r
                 ctx = _NoGradCtx()
                 return AnalogConv2dFunction.forward(ctx, inp, weight2d, bias, input_range, input_range_update_idx,
                                                     in_sizes, training, rpu_config, x_min, x_max, learnable_weight_clip,
-                                                    False, geometry)
+                                                    False, geometry, as_image)
             return AnalogConv2dFunction.apply(inp, weight2d, bias, input_range, input_range_update_idx, in_sizes,
-                                              training, rpu_config, x_min, x_max, learnable_weight_clip, grad, geometry)
+                                              training, rpu_config, x_min, x_max, learnable_weight_clip, grad, geometry, as_image)
         except _PatchTooLarge:
             pass
     patches = unfold2d(inp, kernel_size, dilation, padding, stride)

@@ -98,7 +98,9 @@ class _AnalogConvNd(AnalogLayerBase, _ConvNd):
                                    self.input_range, self.input_range_update_idx, self.in_sizes,
                                    self.training, self.rpu_config, self.x_min, self.x_max,
                                    self.learnable_weight_clip, self.kernel_size, self.dilation, self.padding,
-                                   self.stride)
+                                   self.stride, as_image=True)
+        if out.dim() == 4:  # the fused operator
+            return out
         out_size = (im_shape[-2] + 2 * self.padding[0] - self.dilation[0] * (self.kernel_size[0] - 1) - 1
                     ) // self.stride[0] + 1
         if len(im_shape) == 3:

@@ -286,6 +286,9 @@ int al_unfold2d_dac(int32_t dtype, const void* x, int32_t B, int32_t C, int32_t 
                     int32_t sh, int32_t sw, int32_t ph, int32_t pw, int32_t dh, int32_t dw,
                     const int32_t* tile_ends_host, int32_t T, double inp_res, void* xq, void* ir_rows, void* codes16,
                     void* stream);
+/* dst[b, c, r] = src[b, r, c] for B matrices of rows x cols: the outputs of a convolution's GEMM (one row per pixel) to
+ * images and back (`transpose(-1, -2).contiguous()` in P/conv.py:312-345). */
+int al_transpose_images(int32_t dtype, const void* src, int32_t B, int32_t rows, int32_t cols, void* dst, void* stream);
 int al_fold2d(int32_t dtype, const void* grad_patches, int32_t B, int32_t C, int32_t H, int32_t W, int32_t kh,
               int32_t kw, int32_t sh, int32_t sw, int32_t ph, int32_t pw, int32_t dh, int32_t dw, void* grad_x,
               void* stream);

@@ -33,3 +33,13 @@ def test_layer_refuses_cpu_tensors():
 
     with pytest.raises(ValueError):
         AnalogLinear(8, 8, rpu_config=TorchInferenceRPUConfig())(torch.zeros(2, 8))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("shape", [(3, 1024, 16), (3, 16, 1024), (2, 65, 33), (2, 33, 65), (1, 1, 1), (5, 64, 64), (2, 130, 3), (1, 7, 2049)])
+def test_transpose_images(shape, dtype):
+    from aihwkit_lightning_b200.nn import functional as F
+
+    src = torch.randn(*shape, device="cuda").to(dtype)
+    assert torch.equal(F._transpose_images(src, *shape), src.transpose(-1, -2).contiguous())
