@@ -148,11 +148,10 @@ static bool needs_wmax(const Derived& dv) {
 }
 static size_t elem_size(int dtype) { return dtype == AL_BF16 ? 2 : 4; }
 
-// the pitched layout the caller announced must be the one the kernels assume
 static int check_ragged(const AlDesc& d, const TileTable& tt, RaggedTiles* rt) {
-  if (tc_ragged_supported(d, tt, rt) && d.operand_pitch == rt->T * rt->pitch) return AL_OK;
-  set_error("operand_pitch = %d is not al_operand_pitch() of this layer", d.operand_pitch);
-  return AL_ERR_BAD_ARGUMENT;
+  if (tc_ragged_supported(d, tt, rt)) return AL_OK;
+  set_error("pitched operands announced for a layer without al_operand_pitch()");
+  return AL_ERR_UNSUPPORTED;
 }
 
 static bool pick_tc(const AlDesc& d, const TileTable& tt, bool backward) {
@@ -325,15 +324,16 @@ int al_forward(const AlDesc* desc, const AlForwardArgs* a, void* stream) {
 
   // ragged layer on the tensor cores: xq and w_mod in the pitched layout
   RaggedTiles rt;
-  const bool ragged = d.operand_pitch != 0;
-  // the pitched layout of a layer with only N ragged is the dense one: its operands come from the dense pre-passes
-  const bool pitched = ragged && d.operand_pitch != d.K;
+  const bool ragged = d.engine == AL_ENGINE_PITCHED;
+  bool pitched = false;
   if (ragged) {
     rc = check_ragged(d, tt, &rt);
     if (rc) return rc;
+    // the pitched layout of a layer with only N ragged is the dense one: its operands come from the dense pre-passes
+    pitched = rt.T * rt.pitch != d.K;
     if (prequantised || a->w_noise || a->out_noise || a->codes ||
         (pitched && (!a->xq || !a->w_mod || a->w_mod == a->w || a->xq == a->x))) {
-      set_error("al_forward: operand_pitch needs separate xq and w_mod; not with x_prequantised, replayed noise or codes");
+      set_error("al_forward: AL_ENGINE_PITCHED needs separate xq and w_mod; not with x_prequantised, replayed noise or codes");
       return AL_ERR_BAD_ARGUMENT;
     }
   }
@@ -690,13 +690,13 @@ int al_backward(const AlDesc* desc, const AlBackwardArgs* a, void* stream) {
               (long long)a->g_planes_elems, (long long)al_backward_plane_elems(desc, a->tile_ends));
     return AL_ERR_BAD_ARGUMENT;
   }
-  if (d.engine >= AL_ENGINE_TCGEN05 && !tc_f32 && !tc_backward_supported(d, tt)) {
+  const bool ragged = d.engine == AL_ENGINE_PITCHED;
+  if (d.engine >= AL_ENGINE_TCGEN05 && !ragged && !tc_f32 && !tc_backward_supported(d, tt)) {
     set_error("tcgen05 engine requested but the problem does not qualify");
     return AL_ERR_UNSUPPORTED;
   }
   bool tc = !tc_f32 && pick_tc(d, tt, true);
   RaggedTiles rt;
-  const bool ragged = d.operand_pitch != 0;
   const void* g_rows = a->grad_out;  // ragged: rows of a multiple of 8 elements, 16-byte aligned
   if (ragged) {
     rc = check_ragged(d, tt, &rt);

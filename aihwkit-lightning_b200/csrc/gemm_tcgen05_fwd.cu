@@ -811,7 +811,9 @@ int launch_fwd_tc(int round_dt, const void* xq, const void* w_mod, int K, const 
 // even as possible have no closed-form start (no module makes them); and the weight gradient here does not split its
 // reduction over the rows, so a layer of few output blocks leaves from 8192 rows on.
 bool tc_ragged_supported(const AlDesc& d, const TileTable& tt, RaggedTiles* rt) {
-  if (d.dtype != AL_BF16 || d.engine != AL_ENGINE_AUTO || tc_tiling_ok(d, tt) || !ragged_tiles(tt, rt)) return false;
+  if (d.dtype != AL_BF16 || (d.engine != AL_ENGINE_AUTO && d.engine != AL_ENGINE_PITCHED) || tc_tiling_ok(d, tt) ||
+      !ragged_tiles(tt, rt))
+    return false;
   const int64_t blocks = (int64_t)((d.N + BM - 1) / BM) * rt->T * ((rt->widest() + 255) / 256);
   if (rt->widest() < 8 || (d.M > 8192 && blocks < 37)) return false;
   return (int64_t)rt->T * rt->pitch < (1ll << 31);

@@ -121,12 +121,15 @@ PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
 
   // sizes that are no multiples of 8: the tensor-core route takes its operands in a pitched layout (a layer whose
   // pitch equals K reads x and w themselves where nothing modifies them: those must be aligned)
+  int64_t k_rows = k;
   if (d.dtype == AL_BF16 && !prequant && !capture && !replay &&
       (n % 8 || k % 8 || ends[0] % 8 || (t > 1 && (ends[t - 1] - ends[t - 2]) % 8))) {
     const int32_t pitch = al_operand_pitch(&d, ends);
-    if (pitch != k || !(((uintptr_t)args.x | (uintptr_t)args.w) % 16)) d.operand_pitch = pitch;
+    if (pitch != 0 && (pitch != k || !(((uintptr_t)args.x | (uintptr_t)args.w) % 16))) {
+      d.engine = AL_ENGINE_PITCHED;
+      k_rows = pitch;
+    }
   }
-  const int64_t k_rows = d.operand_pitch ? d.operand_pitch : k;
   const bool pitched = k_rows != k;
   // fp32 layer on the tensor cores: the GEMMs read the DAC codes and the weights as bf16 planes
   const bool planes = d.dtype == AL_F32 && al_uses_tcgen05(&d, ends);
@@ -257,7 +260,7 @@ PyObject* backward(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   args.reduce_scratch_floats = al_backward_scratch_floats(d.M, d.K, d.N, d.T);
   arena.add(reinterpret_cast<void**>(&args.reduce_scratch), args.reduce_scratch_floats * 4);
   if (args.codes16) args.g_planes_elems = al_backward_plane_elems(&d, ends);
-  else if (d.operand_pitch && (n % 8 || (uintptr_t)args.grad_out % 16)) args.g_planes_elems = m * round_up(n, 8);
+  else if (d.engine == AL_ENGINE_PITCHED && (n % 8 || (uintptr_t)args.grad_out % 16)) args.g_planes_elems = m * round_up(n, 8);
   if (args.g_planes_elems > 0) arena.add(&args.g_planes, args.g_planes_elems * 2);
   const at::Tensor workspace = arena.place(opt);
   const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(g.device().index()).stream();

@@ -54,10 +54,15 @@ enum AlInputRangeMode { AL_IR_OFF = 0, AL_IR_STATIC = 1, AL_IR_DYNAMIC = 2, AL_I
  * allow and the SIMT kernels otherwise; SIMT and TCGEN05 force one of them (tests).  The
  * tcgen05 backward GEMMs run on CTA pairs (cta_group::2) when the problem has a 256 x 256 block
  * per pair of SMs and on single CTAs otherwise; TCGEN05_PAIR / TCGEN05_SINGLE force that choice
- * as well (tests, comparisons). */
+ * as well (tests, comparisons).
+ * PITCHED is for a bf16 layer with al_operand_pitch() > 0, in the forward and the backward call alike: xq and
+ * w_mod hold al_operand_pitch() elements per row (separate from x and w unless that is K), the GEMMs run on the
+ * tensor cores, and the backward takes g_planes as a workspace of g_planes_elems >= M * (N rounded up to 8) bf16
+ * elements unless N is a multiple of 8 and grad_out 16-byte aligned.  Not with x_prequantised, replayed noise or
+ * `codes`. */
 enum AlEngine {
   AL_ENGINE_AUTO = 0, AL_ENGINE_SIMT = 1, AL_ENGINE_TCGEN05 = 2,
-  AL_ENGINE_TCGEN05_PAIR = 3, AL_ENGINE_TCGEN05_SINGLE = 4
+  AL_ENGINE_TCGEN05_PAIR = 3, AL_ENGINE_TCGEN05_SINGLE = 4, AL_ENGINE_PITCHED = 5
 };
 
 /*
@@ -92,12 +97,6 @@ typedef struct AlDesc {
   int32_t ref_rounding;      /* bf16: round to bf16 after every op like the reference does */
   int32_t engine;            /* AlEngine                                                    */
   int32_t save_for_backward; /* write `keep_mask` (forward) so that al_backward can run     */
-  int32_t operand_pitch;     /* 0: xq and w_mod are dense.  Otherwise al_operand_pitch() of the layer, the same
-                                 in the forward and the backward call: xq and w_mod hold that many
-                                 elements per row (separate from x and w unless the pitch is K), the GEMMs run
-                                 on the tensor cores, and the backward takes g_planes as a workspace of
-                                 g_planes_elems >= M * (N rounded up to 8) bf16 elements unless N is a
-                                 multiple of 8.  Not with x_prequantised, replayed noise or `codes` */
 } AlDesc;
 
 /*
@@ -256,7 +255,8 @@ int64_t al_backward_plane_elems(const AlDesc* desc, const int32_t* tile_ends_hos
 /* Number of bf16 planes an fp32 operand is split into for the tensor cores (first dimension of w_planes). */
 int32_t al_f32_planes(void);
 /* Elements per row of xq and w_mod with which a bf16 layer whose sizes are no multiples of 8 runs on the tensor
- * cores (every analog tile padded to a multiple of 8 columns); 0 when the layer takes the dense layout. */
+ * cores under AL_ENGINE_PITCHED (every analog tile padded to a multiple of 8 columns); 0 when the layer takes the
+ * dense layout. */
 int32_t al_operand_pitch(const AlDesc* desc, const int32_t* tile_ends_host);
 /* floats of AlForwardArgs.smallm_scratch; 0 when the problem has more than 16 rows */
 int64_t al_smallm_scratch_floats(int32_t M, int32_t N, int32_t T);

@@ -71,3 +71,23 @@ def test_bad_arguments_are_rejected_without_a_gpu():
     assert lib.al_forward(desc, args, None) == _lib.AL_ERR_BAD_ARGUMENT
     with pytest.raises(AssertionError):
         _lib.check(_lib.AL_ERR_BAD_ARGUMENT)
+
+
+def test_descriptor_has_the_layout_of_version_1():
+    """A caller built against the first header passes 148 bytes of fields and 4 of padding that it never wrote: nothing
+    of the call may depend on those."""
+    if not os.path.exists(_lib.LIB_PATH):
+        pytest.skip("library not built")
+    lib = _lib.load()
+    assert _lib.AlDesc.save_for_backward.offset == 144 and ctypes.sizeof(_lib.AlDesc) == 152
+    raw = (ctypes.c_ubyte * 152)()
+    desc = _lib.AlDesc.from_buffer(raw)
+    desc.M, desc.K, desc.N, desc.T = 4, 16, 8, 2
+    desc.dtype, desc.ir_mode, desc.inp_res = 1, 1, 254.0
+    args = _lib.AlForwardArgs()
+    args.x = args.w = args.out = 256
+    args.tile_ends = _lib.tile_ends_array([8, 8])
+    for fill in (0x00, 0xAB):
+        raw[148:152] = [fill] * 4
+        assert lib.al_forward(desc, args, None) == _lib.AL_ERR_BAD_ARGUMENT  # refused on the host: no ranges given
+        assert b"static input range needs input_range" in lib.al_last_error(), fill

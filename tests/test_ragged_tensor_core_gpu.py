@@ -138,9 +138,12 @@ def test_operand_pitch_is_checked_on_the_host():
     assert lib.al_operand_pitch(other, ends) == 0  # another engine: the dense layout
     tall = F.make_desc(layer.rpu_config, 8193, 1001, 515, 2, torch.bfloat16, False)
     assert lib.al_operand_pitch(tall, ends) == 0   # 5 x 4 blocks of the weight gradient, a long reduction
-    desc.operand_pitch = 1008 + 8
+    even = F.make_desc(layer.rpu_config, 130, 1024, 512, 2, torch.bfloat16, False)
+    ends = _lib.tile_ends_array([512, 512])
+    even.engine = _lib.AL_ENGINE_PITCHED  # announced for a layer that has no pitched layout
+    assert lib.al_operand_pitch(even, ends) == 0
     args = _lib.AlForwardArgs()
     buf = torch.zeros(4 << 20, device="cuda", dtype=torch.uint8)
     args.x = args.w = args.out = args.xq = args.w_mod = args.ir_rows = buf.data_ptr()
     args.tile_ends = ends
-    assert lib.al_forward(desc, args, None) != _lib.AL_OK
+    assert lib.al_forward(even, args, None) != _lib.AL_OK
