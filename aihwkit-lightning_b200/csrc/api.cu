@@ -274,7 +274,9 @@ int32_t al_f32_planes(void) { return kPlanes; }
 int al_uses_tcgen05(const AlDesc* desc, const int32_t* tile_ends_host) {
   if (!desc) return 0;
   TileTable tt;
+  RaggedTiles rt;
   if (make_tile_table(tile_ends_host, desc->T, desc->K, &tt)) return 0;
+  if (desc->engine == AL_ENGINE_PITCHED) return tc_ragged_supported(*desc, tt, &rt) ? 1 : 0;
   return (pick_tc(*desc, tt, false) || pick_tc_f32(*desc, tt)) ? 1 : 0;
 }
 

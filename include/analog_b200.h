@@ -343,7 +343,8 @@ int al_read_device_error(void* stream, uint32_t* out_code);
 int al_set_device_wait_limit_ns(uint64_t ns);
 int al_debug_withhold_forward_signal(int32_t on);
 
-/* 1 if the given problem would run on the tcgen05/TMA kernels under AL_ENGINE_AUTO. */
+/* 1 if the GEMMs of the given problem run on the tcgen05/TMA kernels with the engine of the descriptor.  A bf16 layer
+ * with al_operand_pitch() > 0: 1 under AL_ENGINE_PITCHED; 0 under AL_ENGINE_AUTO, where its operands are dense. */
 int al_uses_tcgen05(const AlDesc* desc, const int32_t* tile_ends_host);
 
 /* Launch accounting and optional per-kernel timing (no counterpart in the reference, whose

@@ -91,3 +91,19 @@ def test_descriptor_has_the_layout_of_version_1():
         raw[148:152] = [fill] * 4
         assert lib.al_forward(desc, args, None) == _lib.AL_ERR_BAD_ARGUMENT  # refused on the host: no ranges given
         assert b"static input range needs input_range" in lib.al_last_error(), fill
+
+
+def test_uses_tcgen05_speaks_for_the_engine_of_the_descriptor():
+    if not os.path.exists(_lib.LIB_PATH):
+        pytest.skip("library not built")
+    lib = _lib.load()
+    desc = _lib.AlDesc()
+    desc.M, desc.K, desc.N, desc.T = 64, 1000, 777, 2
+    desc.dtype, desc.ir_mode, desc.inp_res = 1, 2, 254.0
+    ends = _lib.tile_ends_array([500, 500])
+    assert lib.al_operand_pitch(desc, ends) == 1008
+    assert lib.al_uses_tcgen05(desc, ends) == 0  # dense operands: CUDA cores
+    desc.engine = _lib.AL_ENGINE_PITCHED
+    assert lib.al_uses_tcgen05(desc, ends) == 1
+    desc.N, desc.K = 776, 1008
+    assert lib.al_uses_tcgen05(desc, _lib.tile_ends_array([504, 504])) == 0  # no pitched layout to announce
