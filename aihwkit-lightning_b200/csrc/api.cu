@@ -610,10 +610,12 @@ int64_t al_smallm_scratch_floats(int32_t M, int32_t N, int32_t T) {
 }
 
 namespace {
+// range gradient: six floats per tile and block of eight or more rows
+int64_t range_partial_floats(int32_t M, int32_t T) { return 3 * (int64_t)T * (M < 2 ? 2 : M) + 16; }
 // reductions of the range / clip gradients, rounded up to 16 bytes; the partial sums of a split weight gradient
 // follow
 int64_t backward_reduce_floats(int32_t M, int32_t T) {
-  const int64_t n = 3 * (int64_t)T * M + 16 + 2 * (int64_t)T + 16;
+  const int64_t n = range_partial_floats(M, T) + 2 * (int64_t)T + 16;
   return (n + 3) / 4 * 4;
 }
 }  // namespace
@@ -803,7 +805,7 @@ int al_backward(const AlDesc* desc, const AlBackwardArgs* a, void* stream) {
                 "and reduce_scratch");
       return AL_ERR_BAD_ARGUMENT;
     }
-    float* tile_max = a->reduce_scratch + 3 * (int64_t)d.T * d.M + 16;
+    float* tile_max = a->reduce_scratch + range_partial_floats(d.M, d.T);
     int32_t* flags = (int32_t*)(tile_max + d.T);
     const int discretize = dv.weight_quant == AL_QUANT_DISCRETIZE_PER_CHANNEL;
     rc = launch_tile_max(d.dtype, a->learnable_weight_clip, d.N, tt, discretize ? dv.weight_quant : kQuantLearnClamp,

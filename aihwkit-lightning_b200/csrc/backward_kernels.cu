@@ -82,8 +82,10 @@ bias_grad_kernel(const void* __restrict__ g, int M, int N, void* __restrict__ gr
 }
 
 // Partial sums for the range gradient, then zero grad_x where the input was clipped and does not sit exactly on
-// the range.  A block takes `block_rows` consecutive rows of one tile and writes one triple of partial sums.  Bound by reading x and grad_x once.  VEC: every (row, tile) segment starts and ends on a 16-byte
-// boundary (the launcher checked), so a lane moves 16-byte vectors; single elements otherwise.
+// the range.  A block takes `block_rows` consecutive rows of one tile and writes three partial sums: fp32 within a lane's
+// share of one row, double beyond it (terms of both signs cancel in fast mode), kept as the sum of two floats because
+// the workspace is only known to be aligned for those.  Bound by reading x and grad_x once.  VEC: every (row, tile) segment starts and ends on a 16-byte boundary (the launcher
+// checked), so a lane moves 16-byte vectors; single elements otherwise.
 struct IrSums {
   float up, lo, cnt;
 };
@@ -108,13 +110,15 @@ __global__ void __launch_bounds__(256)
 static_ir_partial_kernel(const void* __restrict__ x, const void* __restrict__ ir_used,
                          void* __restrict__ grad_x, int M, int K, TileTable tt,
                          float* __restrict__ partial, int fast_mode, int block_rows) {
-  __shared__ float part[8][3];
+  __shared__ double part[8][3];
   const int t = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int lo = tt.lo(t), len = tt.hi(t) - lo;
   const float ir = Elem<DT>::load(ir_used, t);
-  IrSums s = {0.0f, 0.0f, 0.0f};
-  const int m_end = min(M, (int)(blockIdx.x + 1) * block_rows);
-  for (int m = (int)blockIdx.x * block_rows + warp; m < m_end; m += 8) {
+  double up = 0.0, down = 0.0;
+  IrSums s = {0.0f, 0.0f, 0.0f};  // up, lo: of the row at hand; cnt: of all rows (exact)
+  const unsigned m_first = blockIdx.x * (unsigned)block_rows, m_end = min((unsigned)M, m_first + (unsigned)block_rows);
+  for (unsigned m = m_first + warp; m < m_end; m += 8) {
+    s.up = s.lo = 0.0f;
     const int64_t start = (int64_t)m * K + lo;
     if (VEC) {
       constexpr int VN = DT == kF32 ? 4 : 8;
@@ -153,24 +157,29 @@ static_ir_partial_kernel(const void* __restrict__ x, const void* __restrict__ ir
         if (ir_element(Elem<DT>::load(x, start + i), Elem<DT>::load(grad_x, start + i), ir, fast_mode, s))
           Elem<DT>::store(grad_x, start + i, 0.0f);
     }
+    up += (double)s.up;
+    down += (double)s.lo;
   }
+  double cnt = (double)s.cnt;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
-    s.up += __shfl_xor_sync(0xffffffffu, s.up, o);
-    s.lo += __shfl_xor_sync(0xffffffffu, s.lo, o);
-    s.cnt += __shfl_xor_sync(0xffffffffu, s.cnt, o);
+    up += __shfl_xor_sync(0xffffffffu, up, o);
+    down += __shfl_xor_sync(0xffffffffu, down, o);
+    cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
   }
   if (lane == 0) {
-    part[warp][0] = s.up;
-    part[warp][1] = s.lo;
-    part[warp][2] = s.cnt;
+    part[warp][0] = up;
+    part[warp][1] = down;
+    part[warp][2] = cnt;
   }
   __syncthreads();
   if (threadIdx.x < 3) {
-    float sum = part[0][threadIdx.x];
+    double sum = part[0][threadIdx.x];
 #pragma unroll
     for (int w = 1; w < 8; ++w) sum += part[w][threadIdx.x];
-    partial[((int64_t)t * gridDim.x + blockIdx.x) * 3 + threadIdx.x] = sum;
+    float* const p = partial + (((int64_t)t * gridDim.x + blockIdx.x) * 3 + threadIdx.x) * 2;
+    p[0] = (float)sum;
+    p[1] = (float)(sum - (double)p[0]);
   }
 }
 
@@ -183,10 +192,10 @@ __global__ void static_ir_final_kernel(const float* __restrict__ partial,
   int t = blockIdx.x;
   double a = 0.0, b = 0.0, c = 0.0;
   for (int i = threadIdx.x; i < n_partials; i += blockDim.x) {
-    const float* p = partial + ((int64_t)t * n_partials + i) * 3;
-    a += (double)p[0];
-    b += (double)p[1];
-    c += (double)p[2];
+    const float* p = partial + ((int64_t)t * n_partials + i) * 6;
+    a += (double)p[0] + (double)p[1];
+    b += (double)p[2] + (double)p[3];
+    c += (double)p[4] + (double)p[5];
   }
   sm[0][threadIdx.x] = a;
   sm[1][threadIdx.x] = b;

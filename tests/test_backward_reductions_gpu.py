@@ -61,3 +61,32 @@ def test_static_range_gradient_and_clipped_inputs(dtype, m, k, tiles):
         scale = 1.5 * gx[clipped[:, cols]].abs().sum() + 1e-6
         assert abs(layer.input_range.grad[t].double() - want) <= tol * scale
         lo += size
+
+
+@pytest.mark.parametrize("m,rows", [(3, (0, 1, 2)), (18976, (0, 8, 16)), (18976, (0, 1, 18975)), (9, (0, 1, 8))],
+                         ids=["row_per_warp", "rows_of_a_warp", "two_blocks", "two_short_blocks"])
+def test_range_gradient_keeps_small_terms_between_large_ones(m, rows):
+    """Rows of 2^24, 1 and -2^24: fp32 sums over rows lose the 1, which the result consists of."""
+    from aihwkit_lightning_b200 import _lib
+
+    lib = _lib.load()
+    k = 32
+    x = torch.zeros(m, k, device="cuda")
+    g = torch.zeros(m, 1, device="cuda")
+    for row, v in zip(rows, (2.0 ** 24, 1.0, -(2.0 ** 24))):
+        x[row, 5], g[row, 0] = 2.0, v
+    w, ir = torch.ones(1, k, device="cuda"), torch.ones(1, device="cuda")
+    grad_x, grad_ir = torch.empty(m, k, device="cuda"), torch.empty(1, device="cuda")
+    scratch = torch.empty(lib.al_backward_scratch_floats(m, k, 1, 1), device="cuda")
+    desc = _lib.AlDesc()
+    desc.M, desc.K, desc.N, desc.T = m, k, 1, 1
+    desc.dtype, desc.ir_mode, desc.engine = _lib.AL_F32, _lib.AL_IR_FAST, _lib.AL_ENGINE_SIMT
+    desc.inp_res, desc.out_res, desc.out_bound = 254.0, -1.0, -1.0
+    args = _lib.AlBackwardArgs()
+    args.tile_ends = _lib.tile_ends_array([k])
+    args.grad_out, args.x, args.w_mod, args.ir_rows = g.data_ptr(), x.data_ptr(), w.data_ptr(), ir.data_ptr()
+    args.grad_x, args.grad_input_range = grad_x.data_ptr(), grad_ir.data_ptr()
+    args.reduce_scratch, args.reduce_scratch_floats = scratch.data_ptr(), scratch.numel()
+    _lib.check(lib.al_backward(desc, args, torch.cuda.current_stream().cuda_stream))
+    assert grad_ir.item() == 1.0
+    assert not bool(grad_x[x > 1].any())
