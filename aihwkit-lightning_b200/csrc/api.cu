@@ -817,7 +817,8 @@ int al_backward(const AlDesc* desc, const AlBackwardArgs* a, void* stream) {
     if (rc) return rc;
   }
   if (a->grad_bias) {
-    rc = launch_bias_grad(d.dtype, a->grad_out, d.M, d.N, a->grad_bias, s);
+    rc = launch_bias_grad(d.dtype, a->grad_out, d.M, d.N, a->grad_bias, a->reduce_scratch,
+                          a->reduce_scratch ? a->reduce_scratch_floats : 0, s);
     if (rc) return rc;
   }
   return AL_OK;

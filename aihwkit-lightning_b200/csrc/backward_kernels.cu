@@ -1,7 +1,7 @@
 // Element-wise and reduction parts of the backward pass: the bias gradient (column sums of
 // the upstream gradient) and, for learned/fixed input ranges, the input-range gradient with
 // its decay term followed by the straight-through zeroing of clipped inputs.  Both reduce in
-// two stages with a fixed order (no floating-point atomics).
+// a fixed order (no floating-point atomics).
 #include <cooperative_groups.h>
 
 #include "analog_math.cuh"
@@ -13,11 +13,23 @@ namespace al {
 
 namespace {
 
-// Column sums of g [M, N] in one launch.  A cluster of kBiasCluster CTAs owns 64 columns; each CTA adds every
-// kBiasCluster-th group of rows (a thread: VN columns of every (kBiasCluster * rows-per-pass)-th row, kBiasAhead
-// loads in flight), then the row groups are added in shared memory and the CTAs of the cluster through distributed
-// shared memory, always in the same order.  Bound by reading g once.
-constexpr int kBiasCluster = 8, kBiasCols = 64, kBiasThreads = 256, kBiasAhead = 8;
+// Column sums of g [M, N].  A cluster of kBiasCluster CTAs owns COLS columns of every `splits`-th run of rows; a thread
+// adds VN columns of its rows in runs of bias_ahead with their loads in flight, then the row groups are added in shared
+// memory and the CTAs of the cluster through distributed shared memory, always in the same order.
+// Reading g bounds it where the CTAs fill the chip (large N, or a split); otherwise what a few CTAs have in flight.
+// A run is summed by itself first: that keeps the chain of roundings shorter than one per 256 rows of the matrix.
+constexpr int kBiasCluster = 8, kBiasThreads = 256, kBiasMaxSplits = 32;
+// rows of a thread whose loads are in flight
+constexpr int bias_ahead(int vn, bool wide) { return wide && vn == 1 ? 16 : 8; }
+// Split from this many rows per thread on, and a quarter more for each column group: a second kernel costs about 1.5 us,
+// and groups bring CTAs of their own.  Unsplit -> split, fp32: 64 columns 4096 rows (32 per thread) 3.9 -> 4.1 us,
+// 8192 5.6 -> 5.1, 131072 57 -> 8.2; 65 columns 131072 100 -> 13; 1001 columns 4096 rows (128) 5.7 -> 6.4; 1000 columns
+// 65536 rows (512) 90 -> 43.
+constexpr int kBiasSplitRows = 64;
+// WIDE: the loads of a last short run are in flight together as well, which takes 51 registers instead of 40 -- for
+// grids that leave the SMs room for it.  333 x 777 fp32 3.0 -> 2.5 us, 8192 x 256 6.2 -> 5.2, but 64 x 16384 6.3 -> 10.0
+constexpr unsigned kBiasWideGroups = 4 * 148 / kBiasCluster;
+constexpr int kBiasCtas = 4 * 148;  // what a split fills the chip with: four of up to eight resident CTAs per SM
 template <int DT, int VN>
 __device__ __forceinline__ void load_cols(const void* p, int64_t idx, float v[VN]) {
   if (VN == 1) {
@@ -31,32 +43,49 @@ __device__ __forceinline__ void load_cols(const void* p, int64_t idx, float v[VN
     v[2] = __uint_as_float(u.y << 16); v[3] = __uint_as_float(u.y & 0xffff0000u);
   }
 }
-template <int DT, int VN>
+template <int DT, int VN, int COLS, bool WIDE, bool SPLIT>
 __global__ void __cluster_dims__(1, kBiasCluster, 1) __launch_bounds__(kBiasThreads)
-bias_grad_kernel(const void* __restrict__ g, int M, int N, void* __restrict__ grad_bias) {
-  constexpr int kColThreads = kBiasCols / VN, kRowThreads = kBiasThreads / kColThreads;
-  __shared__ float part[kRowThreads][kBiasCols];
-  __shared__ float total[kBiasCols];
+bias_grad_kernel(const void* __restrict__ g, int M, int N, int splits, float* __restrict__ partial,
+                 void* __restrict__ grad_bias) {
+  constexpr int kColThreads = COLS / VN, kRowThreads = kBiasThreads / kColThreads, kAhead = bias_ahead(VN, WIDE);
+  __shared__ float part[kRowThreads][COLS];
+  __shared__ float total[COLS];
   const int tc = threadIdx.x % kColThreads, tr = threadIdx.x / kColThreads;
-  const int n = blockIdx.x * kBiasCols + tc * VN;  // N % VN == 0
+  const int n = blockIdx.x * COLS + tc * VN;  // N % VN == 0
   float s[VN];
 #pragma unroll
   for (int i = 0; i < VN; ++i) s[i] = 0.0f;
-  constexpr int kStep = kRowThreads * kBiasCluster;
-  if (n < N) {
-    int m = (int)blockIdx.y * kRowThreads + tr;
-    for (; m + (kBiasAhead - 1) * kStep < M; m += kBiasAhead * kStep) {
-      float v[kBiasAhead][VN];
+  const int step = kRowThreads * kBiasCluster * (SPLIT ? splits : 1), first = (int)blockIdx.y * kRowThreads + tr;
+  if (n < N && first < M) {
+    const int count = (M - 1 - first) / step + 1;  // rows of this thread; no row index below goes beyond M
+    int r = 0;
+    for (; WIDE ? r < count : r + kAhead <= count; r += kAhead) {
+      float v[kAhead][VN];
+      if (!WIDE || r + kAhead <= count) {
 #pragma unroll
-      for (int u = 0; u < kBiasAhead; ++u) load_cols<DT, VN>(g, (int64_t)(m + u * kStep) * N + n, v[u]);
+        for (int u = 0; u < kAhead; ++u) load_cols<DT, VN>(g, (int64_t)(first + (r + u) * step) * N + n, v[u]);
+      } else {
 #pragma unroll
-      for (int u = 0; u < kBiasAhead; ++u)
+        for (int u = 0; u < kAhead; ++u) {
+          if (r + u < count) {
+            load_cols<DT, VN>(g, (int64_t)(first + (r + u) * step) * N + n, v[u]);
+          } else {
 #pragma unroll
-        for (int i = 0; i < VN; ++i) s[i] = fadd(s[i], v[u][i]);
+            for (int i = 0; i < VN; ++i) v[u][i] = 0.0f;
+          }
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < VN; ++i) {
+        float run = v[0][i];
+#pragma unroll
+        for (int u = 1; u < kAhead; ++u) run = fadd(run, v[u][i]);
+        s[i] = fadd(s[i], run);
+      }
     }
-    for (; m < M; m += kStep) {
+    for (; !WIDE && r < count; ++r) {
       float v[VN];
-      load_cols<DT, VN>(g, (int64_t)m * N + n, v);
+      load_cols<DT, VN>(g, (int64_t)(first + r * step) * N + n, v);
 #pragma unroll
       for (int i = 0; i < VN; ++i) s[i] = fadd(s[i], v[i]);
     }
@@ -64,7 +93,7 @@ bias_grad_kernel(const void* __restrict__ g, int M, int N, void* __restrict__ gr
 #pragma unroll
   for (int i = 0; i < VN; ++i) part[tr][tc * VN + i] = s[i];
   __syncthreads();
-  if (threadIdx.x < kBiasCols) {
+  if (threadIdx.x < COLS) {
     float sum = part[0][threadIdx.x];
 #pragma unroll
     for (int r = 1; r < kRowThreads; ++r) sum = fadd(sum, part[r][threadIdx.x]);
@@ -72,13 +101,24 @@ bias_grad_kernel(const void* __restrict__ g, int M, int N, void* __restrict__ gr
   }
   cg::cluster_group cluster = cg::this_cluster();
   cluster.sync();
-  if (blockIdx.y == 0 && threadIdx.x < kBiasCols && blockIdx.x * kBiasCols + threadIdx.x < N) {
+  const int col = blockIdx.x * COLS + threadIdx.x;
+  if (blockIdx.y % kBiasCluster == 0 && threadIdx.x < COLS && col < N) {
     float sum = total[threadIdx.x];
 #pragma unroll
     for (int c = 1; c < kBiasCluster; ++c) sum = fadd(sum, cluster.map_shared_rank(total, c)[threadIdx.x]);
-    Elem<DT>::store(grad_bias, blockIdx.x * kBiasCols + threadIdx.x, sum);
+    if (!SPLIT) Elem<DT>::store(grad_bias, col, sum);
+    else partial[(int64_t)(blockIdx.y / kBiasCluster) * N + col] = sum;
   }
   cluster.sync();  // no CTA leaves while another still reads its sums
+}
+template <int DT>
+__global__ void __launch_bounds__(kBiasThreads)
+bias_sum_kernel(const float* __restrict__ partial, int splits, int N, void* __restrict__ grad_bias) {
+  const int n = blockIdx.x * blockDim.x + threadIdx.x;
+  if (n >= N) return;
+  float sum = partial[n];
+  for (int c = 1; c < splits; ++c) sum = fadd(sum, partial[(int64_t)c * N + n]);
+  Elem<DT>::store(grad_bias, n, sum);
 }
 
 // Partial sums for the range gradient, then zero grad_x where the input was clipped and does not sit exactly on
@@ -302,18 +342,36 @@ int launch_learn_clip_backward(int dtype, const void* w, const void* clip, const
   return check_launch("learn_clip_backward");
 }
 
-int launch_bias_grad(int dtype, const void* g, int M, int N, void* grad_bias, cudaStream_t s) {
-  ProfScope prof(AL_K_BIAS_GRAD, s);
-  const dim3 grid((N + kBiasCols - 1) / kBiasCols, kBiasCluster);
+template <int DT, bool SPLIT>
+static void bias_grad_any(const void* g, int M, int N, bool vec, int cols, int splits, float* partial, void* grad_bias,
+                          cudaStream_t s) {
+  const dim3 grid((N + cols - 1) / cols, kBiasCluster * splits);
+  auto kernel = cols == 16 ? (vec ? bias_grad_kernel<DT, 4, 16, true, SPLIT> : bias_grad_kernel<DT, 1, 16, true, SPLIT>)
+                           : (vec ? bias_grad_kernel<DT, 4, 64, true, SPLIT> : bias_grad_kernel<DT, 1, 64, true, SPLIT>);
+  if (!SPLIT && grid.x > kBiasWideGroups)
+    kernel = vec ? bias_grad_kernel<DT, 4, 64, false, false> : bias_grad_kernel<DT, 1, 64, false, false>;
+  kernel<<<grid, kBiasThreads, 0, s>>>(g, M, N, splits, partial, grad_bias);
+  if (SPLIT) bias_sum_kernel<DT><<<(N + kBiasThreads - 1) / kBiasThreads, kBiasThreads, 0, s>>>(partial, splits, N, grad_bias);
+}
+
+int launch_bias_grad(int dtype, const void* g, int M, int N, void* grad_bias, float* scratch, int64_t scratch_floats,
+                     cudaStream_t s) {
   const uintptr_t align = dtype == AL_F32 ? 16 : 8;
   const bool vec = N % 4 == 0 && reinterpret_cast<uintptr_t>(g) % align == 0;
-  if (dtype == AL_F32) {
-    if (vec) bias_grad_kernel<kF32, 4><<<grid, kBiasThreads, 0, s>>>(g, M, N, grad_bias);
-    else bias_grad_kernel<kF32, 1><<<grid, kBiasThreads, 0, s>>>(g, M, N, grad_bias);
-  } else {
-    if (vec) bias_grad_kernel<kBF16, 4><<<grid, kBiasThreads, 0, s>>>(g, M, N, grad_bias);
-    else bias_grad_kernel<kBF16, 1><<<grid, kBiasThreads, 0, s>>>(g, M, N, grad_bias);
-  }
+  const int cols = N <= 16 ? 16 : 64, groups = (N + cols - 1) / cols;
+  // a tall gradient of few columns: several clusters per column group, while a thread keeps a run; their sums meet in the
+  // caller's scratch
+  const int ahead = bias_ahead(vec ? 4 : 1, true);
+  const int pass = kBiasThreads / (cols / (vec ? 4 : 1)) * kBiasCluster;  // rows a cluster reads at a time
+  int splits = kBiasCtas / (kBiasCluster * groups);
+  if (splits > kBiasMaxSplits) splits = kBiasMaxSplits;
+  if (splits > M / (pass * ahead)) splits = M / (pass * ahead);
+  if (M < pass * (kBiasSplitRows * (4 + groups) / 4) || scratch == nullptr || (int64_t)splits * N > scratch_floats) splits = 1;
+  if (splits < 1) splits = 1;
+  ProfScope prof(AL_K_BIAS_GRAD, s, splits > 1 ? 2 : 1);
+  auto run = dtype == AL_F32 ? (splits > 1 ? bias_grad_any<kF32, true> : bias_grad_any<kF32, false>)
+                             : (splits > 1 ? bias_grad_any<kBF16, true> : bias_grad_any<kBF16, false>);
+  run(g, M, N, vec, cols, splits, scratch, grad_bias, s);
   return check_launch("bias_grad");
 }
 

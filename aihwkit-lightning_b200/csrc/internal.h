@@ -172,7 +172,9 @@ int launch_wgrad_simt(int dtype, const void* g, const void* xq, const uint32_t* 
                       int64_t partial_capacity, void* grad_w, cudaStream_t s);
 
 // ---- backward element-wise parts (backward_kernels.cu) ------------------------------------
-int launch_bias_grad(int dtype, const void* g, int M, int N, void* grad_bias, cudaStream_t s);
+// scratch (nullable): up to 16 * N floats, used for tall and narrow gradients when it holds them
+int launch_bias_grad(int dtype, const void* g, int M, int N, void* grad_bias, float* scratch, int64_t scratch_floats,
+                     cudaStream_t s);
 // learned per-channel weight ranges: grad_w -> gradient of the unclipped weights (in place),
 // grad_clip [T,N]; all_gt1 = the per-tile flags launch_tile_max wrote for the ranges
 int launch_learn_clip_backward(int dtype, const void* w, const void* clip, const int32_t* all_gt1, int N,

@@ -90,3 +90,34 @@ def test_range_gradient_keeps_small_terms_between_large_ones(m, rows):
     _lib.check(lib.al_backward(desc, args, torch.cuda.current_stream().cuda_stream))
     assert grad_ir.item() == 1.0
     assert not bool(grad_x[x > 1].any())
+
+
+@pytest.mark.parametrize("m,n", [(262144, 16), (262144, 10), (262144, 65), (65537, 33), (16385, 64), (8191, 130), (255, 3)])
+def test_bias_gradient_of_tall_matrices(m, n):
+    """Against float64, to the error of a sum whose chain of roundings is one per 256 rows, then 256 partial sums (with and
+    without a workspace, which decides how the rows are split).  A rounding is uniform in half an ulp of the partial
+    sum at hand: its rms is 2^-24 / sqrt(3) of that sum at most, and the sum grows like the root of the rows in it, so
+    c roundings on the way to s leave at most 2^-24 / sqrt(3) * s * sqrt(c / 2) (rms over the columns)."""
+    from aihwkit_lightning_b200 import _lib
+
+    lib = _lib.load()
+    desc = _lib.AlDesc()
+    desc.M, desc.K, desc.N, desc.T = m, 8, n, 1
+    desc.dtype, desc.inp_res, desc.out_res, desc.out_bound = _lib.AL_F32, -1.0, -1.0, -1.0
+    args = _lib.AlBackwardArgs()
+    args.tile_ends = _lib.tile_ends_array([8])
+    scratch = torch.empty(lib.al_backward_scratch_floats(m, 8, n, 1), device="cuda")
+    for workspace in (False, True):
+        if workspace:
+            args.reduce_scratch, args.reduce_scratch_floats = scratch.data_ptr(), scratch.numel()
+        square, values = 0.0, 0
+        for seed in range(max(1, 256 // n)):  # a few hundred sums: the rms is known to some 5 %
+            gen = torch.Generator(device="cuda").manual_seed(seed)
+            g = torch.randn(m, n, device="cuda", generator=gen)
+            out = torch.empty(n, device="cuda")
+            args.grad_out, args.grad_bias = g.data_ptr(), out.data_ptr()
+            _lib.check(lib.al_backward(desc, args, torch.cuda.current_stream().cuda_stream))
+            square += ((out.double() - g.double().sum(0)) ** 2).sum().item()
+            values += n
+        chain = min(m, 256) + (m + 255) // 256
+        assert (square / values) ** 0.5 <= 2.0 ** -24 / 3 ** 0.5 * m ** 0.5 * (chain / 2) ** 0.5
