@@ -119,6 +119,16 @@ _lib = None
 _host = None
 
 
+def _check_torch(path):
+    """The extension is bound to the torch it was built against: its C++ types are laid out by those headers."""
+    import torch
+
+    with open(path, "rb") as fh:
+        if f"built for torch {torch.__version__};".encode() not in fh.read():
+            raise RuntimeError(f"{path} was built against another torch than {torch.__version__}: "
+                               "rebuild it with `python aihwkit-lightning_b200/build.py`")
+
+
 def host():
     """The extension that runs one analog call (``csrc/host_calls.cpp``); it needs torch to be imported."""
     global _host
@@ -127,6 +137,7 @@ def host():
         path = os.path.join(os.path.dirname(LIB_PATH), "_host_calls.so")
         if not os.path.exists(path):
             raise RuntimeError(f"{path} is missing: build it with `python aihwkit-lightning_b200/build.py`")
+        _check_torch(path)
         spec = importlib.util.spec_from_file_location("_host_calls", path)
         module = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(module)

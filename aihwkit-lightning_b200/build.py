@@ -3,6 +3,7 @@
     python aihwkit-lightning_b200/build.py [--force]
 
 Both land in ``aihwkit_lightning_b200/lib/`` next to the Python package that loads them.  nvcc cross-compiles without a GPU.
+Without torch or Python's headers only the C library is built: the extension is for the Python package, which needs both.
 """
 import os
 import subprocess
@@ -36,6 +37,17 @@ NVCC_FLAGS = [
 ]
 
 
+def _torch_version():
+    """Version of the installed torch, or None where the extension cannot be built."""
+    import sysconfig
+
+    try:
+        import torch
+    except ImportError:
+        return None
+    return torch.__version__ if os.path.exists(os.path.join(sysconfig.get_paths()["include"], "Python.h")) else None
+
+
 def _host_command():
     """g++ command of the extension: torch's headers, linked against the library next to it."""
     import sysconfig
@@ -45,19 +57,36 @@ def _host_command():
 
     cuda = os.path.dirname(os.path.dirname(os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")))
     includes = [*include_paths(), sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
-    return ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={int(_GLIBCXX_USE_CXX11_ABI)}",
+    return ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", f'-DAL_TORCH_VERSION="{_torch_version()}"',
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(_GLIBCXX_USE_CXX11_ABI)}",
             *[f"-isystem{p}" for p in includes], os.path.join(CSRC, "host_calls.cpp"), "-o", HOST_OUT,
             *[f"-L{p}" for p in library_paths()], "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python",
             f"-L{OUT_DIR}", "-l:libanalog_b200.so", "-Wl,-rpath,$ORIGIN"]
 
 
 def _stale() -> bool:
-    if not os.path.exists(OUT) or not os.path.exists(HOST_OUT):
+    version = _torch_version()
+    outputs = [OUT] if version is None else [OUT, HOST_OUT]
+    if not all(os.path.exists(p) for p in outputs):
         return True
-    built = min(os.path.getmtime(OUT), os.path.getmtime(HOST_OUT))
+    if version is not None and f"built for torch {version};".encode() not in open(HOST_OUT, "rb").read():
+        return True
+    built = min(os.path.getmtime(p) for p in outputs)
     deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)]
     deps.append(os.path.join(HERE, "..", "include", "analog_b200.h"))
     return any(os.path.getmtime(p) > built for p in deps)
+
+
+def build_host() -> None:
+    """The extension, or a line that says why there is none."""
+    version = _torch_version()
+    if version is None:
+        print("torch or Python.h not found: the C library was built, the extension of the Python package was not")
+        return
+    res = subprocess.run(_host_command(), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if res.returncode != 0:
+        sys.stderr.write(res.stdout)
+        raise RuntimeError("g++ failed on host_calls.cpp")
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -86,10 +115,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
     if res.returncode != 0:
         sys.stderr.write(res.stdout)
         raise RuntimeError("link failed")
-    res = subprocess.run(_host_command(), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
-    if res.returncode != 0:
-        sys.stderr.write(res.stdout)
-        raise RuntimeError("g++ failed on host_calls.cpp")
+    build_host()
     if verbose:
         print("\n".join(log))
     return OUT

@@ -17,6 +17,9 @@
 
 #include "../../include/analog_b200.h"
 
+// what the loader and the build look for in this file before they use it
+__attribute__((used)) extern const char al_host_built_for[] = "built for torch " AL_TORCH_VERSION ";";
+
 namespace {
 
 // a positional argument: a tensor, or None
