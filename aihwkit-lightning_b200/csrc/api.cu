@@ -586,19 +586,19 @@ int al_forward(const AlDesc* desc, const AlForwardArgs* a, void* stream) {
   ep.seed = a->seed; ep.offset = a->offset;
   ep.offset_base = a->offset_base;
 
+  const int pairing = d.engine == AL_ENGINE_TCGEN05_PAIR ? 1 : d.engine == AL_ENGINE_TCGEN05_SINGLE ? -1 : 0;
   if (tc_f32) {
     if (!weight_planes) {
       rc = launch_split_planes(static_cast<const float*>(w_mod), (int64_t)d.N * d.K, a->w_planes, s);
       if (rc) return rc;
     }
-    return launch_fwd_tc_f32(a->codes16, a->w_planes, d.K, tt, ep, dv.inp_res, a->out, s);
+    return launch_fwd_tc_f32(a->codes16, a->w_planes, d.K, tt, ep, dv.inp_res, pairing, a->out, s);
   }
   if (ragged) return launch_fwd_tc_ragged(dv.round_dt, xq, w_mod, rt, ep, a->out, s);
   if (d.engine >= AL_ENGINE_TCGEN05 && !tc_forward_supported(d, tt)) {
     set_error("tcgen05 engine requested but the problem does not qualify (bf16, 16-byte aligned tiles)");
     return AL_ERR_UNSUPPORTED;
   }
-  const int pairing = d.engine == AL_ENGINE_TCGEN05_PAIR ? 1 : d.engine == AL_ENGINE_TCGEN05_SINGLE ? -1 : 0;
   if (pick_tc(d, tt, false)) return launch_fwd_tc(dv.round_dt, xq, w_mod, d.K, tt, ep, pairing, a->out, s);
   return launch_fwd_simt(d.dtype, dv.round_dt, xq, w_mod, d.K, tt, ep, a->out, s);
 }

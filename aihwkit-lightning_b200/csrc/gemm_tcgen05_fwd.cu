@@ -881,7 +881,7 @@ static FwdKernel pick_f32_kernel(int mode) {
 // Forward of an fp32 layer on the tensor cores: A = DAC codes as bf16 [M,K], B = the bf16 planes of the
 // modified weights [kPlanes][N][K]; fp32 running sum in tensor memory.
 int launch_fwd_tc_f32(const void* codes16, const void* w_planes, int K, const TileTable& tt,
-                      const FwdEpilogueParams& ep, float inp_res, void* out, cudaStream_t s) {
+                      const FwdEpilogueParams& ep, float inp_res, int pairing, void* out, cudaStream_t s) {
   ProfScope prof(AL_K_FWD_GEMM, s);
   int w = 0;
   if (!uniform_tiles(tt, &w) || !aligned16(codes16) || !aligned16(w_planes) || !aligned16(out)) {
@@ -899,9 +899,9 @@ int launch_fwd_tc_f32(const void* codes16, const void* w_planes, int K, const Ti
   FwdKernel kernel = pick_f32_kernel<true, 64>(mode);
   int rc = ensure_smem(kernel, fwd_smem(64, kPlanes));
   if (rc) return rc;
-  const int pairs = max_fwd_pairs(kernel, fwd_smem(64, kPlanes));
+  const int pairs = pairing >= 0 ? max_fwd_pairs(kernel, fwd_smem(64, kPlanes)) : 0;
   const int64_t pair_blocks = (int64_t)((ep.M + 2 * BM - 1) / (2 * BM)) * ((ep.N + BM - 1) / BM);
-  const int columns = fwd_block_columns(ep.M, ep.N, pairs, pair_blocks, kPlanes);
+  const int columns = pairing > 0 && pairs > 0 ? 0 : fwd_block_columns(ep.M, ep.N, pairs, pair_blocks, kPlanes);
   const bool pair = columns == 0;
   const int bn = pair ? 64 : columns;  // weight rows a CTA stages
   p.num_nb = pair ? (ep.N + BM - 1) / BM : (ep.N + bn - 1) / bn;

@@ -214,7 +214,7 @@ int launch_wgrad_tc(const void* g, const void* xq, const uint32_t* keep_mask, in
 // fp32 layers on the tensor cores: operands as bf16 planes (split_kernels.cu)
 bool tc_f32_supported(const AlDesc& d, const TileTable& tt);
 int launch_fwd_tc_f32(const void* codes16, const void* w_planes, int K, const TileTable& tt,
-                      const FwdEpilogueParams& ep, float inp_res, void* out, cudaStream_t s);
+                      const FwdEpilogueParams& ep, float inp_res, int pairing, void* out, cudaStream_t s);
 int launch_dgrad_tc_f32(const void* g_planes, int sets, const void* w_planes, int M, int K, int N, const TileTable& tt,
                         int pairing, void* grad_x, cudaStream_t s);
 int launch_wgrad_tc_f32(const void* g_planes, int sets, const void* codes16, int M, int K, int N, const TileTable& tt,
