@@ -321,6 +321,8 @@ def _analog_forward(ctx, inp, weight, bias, input_range, input_range_update_idx,
         assert w_noise.shape == w.shape, "replayed weight noise must be [N,K]"
     if out_noise is not None:
         out_noise = out_noise.to(device=dev, dtype=dtype).contiguous()
+        if out_noise.data_ptr() % 16:
+            out_noise = out_noise.clone()  # read in 16-byte vectors
         assert out_noise.numel() == t * m * n, "replayed output noise must be [T,M,N]"
     capture = settings.capture is not None
     seed = offset = offset_base = 0

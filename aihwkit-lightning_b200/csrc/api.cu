@@ -587,6 +587,10 @@ int al_forward(const AlDesc* desc, const AlForwardArgs* a, void* stream) {
   ep.offset_base = a->offset_base;
 
   const int pairing = d.engine == AL_ENGINE_TCGEN05_PAIR ? 1 : d.engine == AL_ENGINE_TCGEN05_SINGLE ? -1 : 0;
+  if (a->out_noise && ((uintptr_t)a->out_noise % 16) != 0 && (tc_f32 || pick_tc(d, tt, false))) {
+    set_error("al_forward: replayed out_noise must be 16-byte aligned on the tensor cores");
+    return AL_ERR_BAD_ARGUMENT;
+  }
   if (tc_f32) {
     if (!weight_planes) {
       rc = launch_split_planes(static_cast<const float*>(w_mod), (int64_t)d.N * d.K, a->w_planes, s);

@@ -612,8 +612,10 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
                   for (int e = 0; e < 4; ++e) {
                     __nv_bfloat162 s2 = as_bf162(sumr[v * 4 + e]);
                     if (ep.bias) {
-                      const uint32_t b2 = *reinterpret_cast<const uint32_t*>(
-                          reinterpret_cast<const uint16_t*>(ep.bias) + nh + v * 8 + 2 * e);
+                      const uint16_t* const pb = reinterpret_cast<const uint16_t*>(ep.bias) + nh + v * 8 + 2 * e;
+                      const uint32_t b2 = (reinterpret_cast<uintptr_t>(ep.bias) & 2) == 0  // a view may start anywhere
+                                              ? *reinterpret_cast<const uint32_t*>(pb)
+                                              : (uint32_t)pb[0] | ((uint32_t)pb[1] << 16);
                       s2 = __hadd2_rn(s2, as_bf162(b2));
                     }
                     w4[e] = as_u32(s2);

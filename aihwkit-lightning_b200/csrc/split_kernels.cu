@@ -21,11 +21,18 @@ __device__ __forceinline__ void split_planes(float v, uint16_t b[kPlanes]) {
   }
 }
 
+// four floats from index 4 v on; `aligned`: the array starts on a 16-byte boundary
+__device__ __forceinline__ float4 load_four(const float* __restrict__ src, int64_t v, bool aligned) {
+  if (aligned) return reinterpret_cast<const float4*>(src)[v];
+  return make_float4(src[v * 4], src[v * 4 + 1], src[v * 4 + 2], src[v * 4 + 3]);
+}
+
 // planes[p][e] of src[e], e < count (count is a multiple of 4 on this path: K % 8 == 0)
 __global__ void __launch_bounds__(256)
-split_planes_kernel(const float* __restrict__ src, int64_t count4, uint16_t* __restrict__ planes, int64_t plane_stride) {
+split_planes_kernel(const float* __restrict__ src, int64_t count4, uint16_t* __restrict__ planes, int64_t plane_stride,
+                    bool aligned) {
   for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < count4; v += (int64_t)gridDim.x * blockDim.x) {
-    const float4 x = reinterpret_cast<const float4*>(src)[v];
+    const float4 x = load_four(src, v, aligned);
     const float in[4] = {x.x, x.y, x.z, x.w};
     uint16_t b[kPlanes][4];
 #pragma unroll
@@ -50,14 +57,14 @@ split_planes_kernel(const float* __restrict__ src, int64_t count4, uint16_t* __r
 // (N % 8 == 0), tiles in gridDim.y.
 __global__ void __launch_bounds__(256)
 split_planes_grad_kernel(const float* __restrict__ g, int M, int N, const uint32_t* __restrict__ keep_mask, int mask_words,
-                   const float* __restrict__ ir, int ir_per_row, float inp_res, uint16_t* __restrict__ planes) {
+                   const float* __restrict__ ir, int ir_per_row, float inp_res, uint16_t* __restrict__ planes, bool aligned) {
   const int t = blockIdx.y;
   const int64_t quads = (int64_t)M * (N / 4);
   const int64_t plane_stride = (int64_t)M * N;
   uint16_t* out = planes + (int64_t)t * kPlanes * plane_stride;
   for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < quads; v += (int64_t)gridDim.x * blockDim.x) {
     const int m = (int)(v / (N / 4)), n = (int)(v % (N / 4)) * 4;
-    const float4 x = reinterpret_cast<const float4*>(g)[v];
+    const float4 x = load_four(g, v, aligned);
     float in[4] = {x.x, x.y, x.z, x.w};
     float scale = 1.0f;
     if (ir != nullptr) scale = quant_step<kF32>(ir[ir_per_row ? (int64_t)t * M + m : t], inp_res);
@@ -212,6 +219,7 @@ weight_planes_kernel(const float* __restrict__ w, int N, int K, int T, int tile_
   for (int g = kHeld * 32 + lane; g < groups; g += 32) put(g, load_eight(w + start + g * 8, true));
 }
 
+bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 unsigned grid_for(int64_t work_items) {
   const int64_t blocks = (work_items + 255) / 256;
   return (unsigned)(blocks < 148 * 16 ? (blocks < 1 ? 1 : blocks) : 148 * 16);
@@ -249,7 +257,8 @@ int launch_weight_planes(const float* w, int N, int K, const TileTable& tt, floa
 
 int launch_split_planes(const float* src, int64_t count, void* planes, cudaStream_t s) {
   ProfScope prof(AL_K_WEIGHT_MODIFY, s);
-  split_planes_kernel<<<grid_for(count / 4), 256, 0, s>>>(src, count / 4, static_cast<uint16_t*>(planes), count);
+  split_planes_kernel<<<grid_for(count / 4), 256, 0, s>>>(src, count / 4, static_cast<uint16_t*>(planes), count,
+                                                         aligned16(src));
   return check_launch("split_planes");
 }
 
@@ -258,7 +267,7 @@ int launch_split_planes_grad(const float* g, int M, int N, const uint32_t* keep_
   ProfScope prof(AL_K_DAC, s);
   dim3 grid(grid_for((int64_t)M * (N / 4)), sets);
   split_planes_grad_kernel<<<grid, 256, 0, s>>>(g, M, N, keep_mask, mask_words, ir, ir_per_row, inp_res,
-                                          static_cast<uint16_t*>(planes));
+                                          static_cast<uint16_t*>(planes), aligned16(g));
   return check_launch("split_planes_grad");
 }
 

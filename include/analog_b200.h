@@ -150,7 +150,7 @@ typedef struct AlForwardArgs {
                                  w_mod to 2^-18 relative                                    */
   /* shared-noise parity mode: standard normals to use instead of the internal generator */
   const void* w_noise;       /* [N,K] dtype, nullable                                       */
-  const void* out_noise;     /* [T,M,N] dtype, nullable                                     */
+  const void* out_noise;     /* [T,M,N] dtype, nullable; 16-byte aligned on the tensor cores */
   /* optional debug output */
   void* codes;               /* [M,K] dtype integer DAC codes, nullable                     */
   uint64_t seed, offset;     /* counter-based generator: (seed, call counter)              */
