@@ -337,7 +337,7 @@ def _analog_forward(ctx, inp, weight, bias, input_range, input_range_update_idx,
         w_noise, out_noise, pre_xq, pre_ir, pre_codes, pre_kind, modifies, need_std, needs_grad, capture,
         capture and settings.capture_codes and desc.ir_mode != _lib.AL_IR_OFF, draw, seed, offset, offset_base)
     _lib.check(status)
-    if static and ir_data is not input_range.data:
+    if static and not input_range.is_contiguous():
         input_range.data.copy_(ir_data)
 
     if capture:

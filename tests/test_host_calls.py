@@ -43,3 +43,36 @@ def test_transpose_images(shape, dtype):
 
     src = torch.randn(*shape, device="cuda").to(dtype)
     assert torch.equal(F._transpose_images(src, *shape), src.transpose(-1, -2).contiguous())
+
+
+@pytest.mark.gpu
+def test_static_ranges_are_copied_back_only_where_they_were_copied():
+    """The library updates a contiguous range in place; a strided one goes through a copy and back."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    from aihwkit_lightning_b200.nn import AnalogLinear
+    from aihwkit_lightning_b200.simulator.configs import TorchInferenceRPUConfig
+
+    class Copies(TorchDispatchMode):
+        count = 0
+
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            self.count += func is torch.ops.aten.copy_.default
+            return func(*args, **(kwargs or {}))
+
+    rpu = TorchInferenceRPUConfig()
+    rpu.mapping.max_input_size, rpu.forward.inp_res = 16, 254.0
+    irp = rpu.pre_post.input_range
+    irp.enable, irp.learn_input_range, irp.init_value, irp.init_from_data = True, True, 3.0, 10
+    ranges = []
+    for strided in (False, True):
+        torch.manual_seed(0)
+        layer = AnalogLinear(64, 32, bias=False, rpu_config=rpu, device="cuda", dtype=torch.float32).train()
+        if strided:
+            layer.input_range.data = torch.full((8,), 3.0, device="cuda")[::2]
+            assert not layer.input_range.is_contiguous()
+        with Copies() as copies, torch.no_grad():
+            layer(torch.randn(40, 64, device="cuda"))
+        assert (copies.count > 0) == strided
+        ranges.append(layer.input_range.detach().clone())
+    assert torch.equal(*ranges) and not bool((ranges[0] == 3.0).any())  # updated from the data
