@@ -31,12 +31,16 @@ def build(dtype, k, n, max_in, adc):
     (torch.bfloat16, 256, 512, 256, 256, True),    # tcgen05 forward with noise + ADC, fused weight pre-pass
     (torch.bfloat16, 512, 1024, 512, 512, False),  # merged output noise
     (torch.float32, 128, 200, 48, 100, False),     # CUDA-core kernels, ragged tiles
-    (torch.float32, 256, 512, 256, 256, False),    # fp32 on the tensor cores
+    (torch.float32, 1024, 512, 256, 256, False),   # fp32 on the tensor cores
 ], ids=["bf16-adc", "bf16-merged-noise", "f32-simt", "f32-tensor-core"])
 def test_replays_draw_fresh_noise(dtype, m, k, n, max_in, adc):
+    from aihwkit_lightning_b200 import _lib
     from aihwkit_lightning_b200.nn import functional as F
 
     layer = build(dtype, k, n, max_in, adc)
+    desc = F.make_desc(layer.rpu_config, m, k, n, len(layer.in_sizes), dtype, True)
+    on_tensor_cores = bool(_lib.load().al_uses_tcgen05(desc, _lib.tile_ends_array(layer.in_sizes)))
+    assert on_tensor_cores == (k % 8 == 0 and max_in % 8 == 0)
     x = torch.randn(m, k, device="cuda").to(dtype).requires_grad_(True)
     g = torch.randn(m, n, device="cuda").to(dtype)
     noise = F.GraphNoise(x.device)
