@@ -68,17 +68,10 @@ __device__ __forceinline__ void store_c_ragged(void* c_out, int ld, int row0, in
   __syncwarp();
 }
 
-// r += the 32 columns of the cross-term accumulator at taddr (fp32, round to nearest)
+// r += 32 columns at taddr: the cross-term accumulator, or the running sum of a chunked item
 __device__ __forceinline__ void add_cross_terms(uint32_t taddr, uint32_t r[32]) {
-#pragma unroll
-  for (int half = 0; half < 2; ++half) {
-    uint32_t x[16];
-    tmem_ld16(taddr + (uint32_t)(half * 16), x);
-    tmem_wait_ld();
-#pragma unroll
-    for (int j = 0; j < 16; ++j)
-      r[half * 16 + j] = __float_as_uint(__fadd_rn(__uint_as_float(r[half * 16 + j]), __uint_as_float(x[j])));
-  }
+  add_tmem16(taddr, r);
+  add_tmem16(taddr + 16u, r + 16);
 }
 
 // 32 accumulator columns of one row -> C (bf16 or fp32), columns jc .. jc + 31 clipped at j_end
@@ -126,8 +119,9 @@ __device__ __forceinline__ void rewrite_row_masked(uint32_t row_addr, int sw, ui
   }
 }
 
-// BN: columns of a block (pick_blocks)
-template <bool WGRAD, bool RAG, int BN>
+// BN: columns of a block (pick_blocks).  CHUNK: sums of more than 64 * kRagChunkSteps terms (RAG only; a kernel of its own,
+// as a run-time switch it cost the others 2 %)
+template <bool WGRAD, bool RAG, int BN, bool CHUNK>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 bwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
               const BwdTcParams p) {
@@ -140,6 +134,8 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bool masked = p.keep_mask != nullptr;
   const bool split_acc = p.products > 1;
+  // both accumulators belong to one item, or the second holds its running sum
+  const bool one_acc = split_acc || (CHUNK && BN == 256);
   const int per_split = p.num_ib * p.T * p.num_jb;
   const int num_work = per_split * p.splits;  // item w: copy w / per_split of output block w % per_split
 
@@ -224,49 +220,53 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
       constexpr uint32_t idesc = make_idesc(BM, BN, WGRAD ? 1 : 0, 1);
       uint32_t it = 0, acc_it = 0;
       bool ok = true;
-      for (int w = blockIdx.x; w < num_work && ok; w += gridDim.x, ++acc_it) {
+      for (int w = blockIdx.x; w < num_work && ok; w += gridDim.x) {
         // plane products: the leading product accumulates in buffer 0 and the (much smaller) cross terms
         // in buffer 1 -- the tensor core truncates when it adds into an accumulator, and the truncation is
         // relative to the accumulator's size -- so an item holds both buffers and there is no overlap
-        const int b = split_acc ? 0 : (int)(acc_it & 1u);
-        const uint32_t aph = split_acc ? (acc_it & 1u) : ((acc_it >> 1) & 1u);
-        if (!mbar_wait(&bars->acc_empty[b], aph ^ 1u, abort_flag)) {
-          raise_error(kErrMma, abort_flag);
-          ok = false;
-          break;
-        }
-        tc_fence_after();
         const int sp = w / per_split;
         const int nls = min((sp + 1) * p.split_lsteps, p.lsteps) - sp * p.split_lsteps;  // this copy's l-steps
         const int steps = nls * p.products;  // every plane product runs over the whole range
-        for (int ls = 0; ls < steps; ++ls, ++it) {
-          const bool cross = split_acc && ls >= nls;
-          const uint32_t d_tmem = tmem_base + (uint32_t)((cross ? 1 : b) * BN);
-          const bool first = ls == 0 || (split_acc && ls == nls);
-          const int s = it % kStages;
-          const uint32_t ph = (it / kStages) & 1u;
-          // the transform warps vouch for a stage on `ready` before its copy has landed when
-          // the stage has nothing to zero, so both barriers gate the MMA
-          if (!mbar_wait(&bars->full[s], ph, abort_flag) ||
-              (masked && !mbar_wait(&bars->ready[s], ph, abort_flag))) {
+        const int chunk = CHUNK ? kRagChunkSteps : steps;
+        for (int ls0 = 0; ls0 < steps && ok; ls0 += chunk, ++acc_it) {
+          const int b = one_acc ? 0 : (int)(acc_it & 1u);
+          const uint32_t aph = one_acc ? (acc_it & 1u) : ((acc_it >> 1) & 1u);
+          if (!mbar_wait(&bars->acc_empty[b], aph ^ 1u, abort_flag)) {
             raise_error(kErrMma, abort_flag);
             ok = false;
             break;
           }
           tc_fence_after();
-          const uint32_t sa = smem_u32(stage_base + s * kStageBytes);
-          const uint32_t sb = sa + B_A_BYTES;
-          const uint64_t da = WGRAD ? desc_mn_major(sa, B_BOX_BYTES) : desc_k_major(sa);
-          const uint64_t db = desc_mn_major(sb, B_BOX_BYTES);
-          // one MMA consumes 16 k: 32 bytes along a K-major row, 16 rows (2048 bytes) of an MN-major box
-          constexpr uint64_t a_step = WGRAD ? (2048u >> 4) : (32u >> 4);
-          constexpr uint64_t b_step = 2048u >> 4;
+          const int ls1 = min(ls0 + chunk, steps);
+          for (int ls = ls0; ls < ls1; ++ls, ++it) {
+            const bool cross = split_acc && ls >= nls;
+            const uint32_t d_tmem = tmem_base + (uint32_t)((cross ? 1 : b) * BN);
+            const bool first = ls == ls0 || (split_acc && ls == nls);
+            const int s = it % kStages;
+            const uint32_t ph = (it / kStages) & 1u;
+            // the transform warps vouch for a stage on `ready` before its copy has landed when
+            // the stage has nothing to zero, so both barriers gate the MMA
+            if (!mbar_wait(&bars->full[s], ph, abort_flag) ||
+                (masked && !mbar_wait(&bars->ready[s], ph, abort_flag))) {
+              raise_error(kErrMma, abort_flag);
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+            const uint32_t sa = smem_u32(stage_base + s * kStageBytes);
+            const uint32_t sb = sa + B_A_BYTES;
+            const uint64_t da = WGRAD ? desc_mn_major(sa, B_BOX_BYTES) : desc_k_major(sa);
+            const uint64_t db = desc_mn_major(sb, B_BOX_BYTES);
+            // one MMA consumes 16 k: 32 bytes along a K-major row, 16 rows (2048 bytes) of an MN-major box
+            constexpr uint64_t a_step = WGRAD ? (2048u >> 4) : (32u >> 4);
+            constexpr uint64_t b_step = 2048u >> 4;
 #pragma unroll
-          for (int k4 = 0; k4 < BK / 16; ++k4)
-            umma_bf16(d_tmem, da + a_step * k4, db + b_step * k4, idesc, (first && k4 == 0) ? 0u : 1u);
-          umma_commit(&bars->empty[s]);
+            for (int k4 = 0; k4 < BK / 16; ++k4)
+              umma_bf16(d_tmem, da + a_step * k4, db + b_step * k4, idesc, (first && k4 == 0) ? 0u : 1u);
+            umma_commit(&bars->empty[s]);
+          }
+          if (ok) umma_commit(&bars->acc_full[b]);
         }
-        if (ok) umma_commit(&bars->acc_full[b]);
       }
       umma_commit(&bars->mma_done);
       uint64_t t0 = globaltimer_ns();
@@ -279,11 +279,13 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
     }
   } else if (warp >= 4 && warp < 8) {
     // ---- epilogue: TMEM -> bf16 -> global ------------------------------------------------
+    constexpr uint32_t kSumCol = BN == 256 ? 256 : 2 * BN;  // running sum of a chunked item
+    const int chunks = CHUNK ? (p.lsteps + kRagChunkSteps - 1) / kRagChunkSteps : 1;
     const int quad = warp & 3;
     const uint32_t lane_base = (uint32_t)(quad * 32) << 16;
     uint32_t acc_it = 0;
     bool ok = true;
-    for (int w = blockIdx.x; w < num_work && ok; w += gridDim.x, ++acc_it) {
+    for (int w = blockIdx.x; w < num_work && ok; w += gridDim.x) {
       const int sp = w / per_split, blk = w - sp * per_split;
       const int ib = blk / (p.T * p.num_jb);
       const int rem = blk % (p.T * p.num_jb);
@@ -293,31 +295,43 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
       const int i = ib * BM + quad * 32 + lane;
       void* const c_dst = p.splits > 1 ? static_cast<void*>(p.partial + (int64_t)sp * p.I * p.K) : p.c_out;
       const bool c_f32 = p.splits > 1 || p.f32_out != 0;
-      const int b = split_acc ? 0 : (int)(acc_it & 1u);
-      const uint32_t aph = split_acc ? (acc_it & 1u) : ((acc_it >> 1) & 1u);
-      if (!mbar_wait(&bars->acc_full[b], aph, abort_flag)) {
-        if (lane == 0) raise_error(kErrEpilogue, abort_flag);
-        ok = false;
-        break;
-      }
-      tc_fence_after();
-      const float c_scale = p.c_scale_ir != nullptr ? quant_step<kF32>(p.c_scale_ir[t], p.inp_res) : 1.0f;
+      for (int chunk = 0; chunk < chunks && ok; ++chunk, ++acc_it) {
+        const int b = one_acc ? 0 : (int)(acc_it & 1u);
+        const uint32_t aph = one_acc ? (acc_it & 1u) : ((acc_it >> 1) & 1u);
+        if (!mbar_wait(&bars->acc_full[b], aph, abort_flag)) {
+          if (lane == 0) raise_error(kErrEpilogue, abort_flag);
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        const float c_scale = p.c_scale_ir != nullptr ? quant_step<kF32>(p.c_scale_ir[t], p.inp_res) : 1.0f;
 #pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
-        const int jc = j0 + c * 32;
-        if (jc >= j_end) break;  // uniform across the warp
-        uint32_t r[32];
-        tmem_ld32(tmem_base + lane_base + (uint32_t)(b * BN + c * 32), r);
-        tmem_wait_ld();
-        if (split_acc) add_cross_terms(tmem_base + lane_base + (uint32_t)(BN + c * 32), r);
-        if (RAG)
-          store_c_ragged(c_dst, p.K, i - lane, p.I, p.rt.lo(t) + jc - t * p.tile_w, min(32, j_end - jc), r,
-                         reinterpret_cast<uint32_t*>(bars + 1) + quad * kRagStageWords, lane);
-        else if (i < p.I) store_c_row(c_dst, c_f32, p.K, i, jc, j_end, r, c_scale);
+        for (int c = 0; c < BN / 32; ++c) {
+          const int jc = j0 + c * 32;
+          if (jc >= j_end) break;  // uniform across the warp
+          uint32_t r[32];
+          tmem_ld32(tmem_base + lane_base + (uint32_t)(b * BN + c * 32), r);
+          tmem_wait_ld();
+          if (split_acc) add_cross_terms(tmem_base + lane_base + (uint32_t)(BN + c * 32), r);
+          if (CHUNK) {  // with 256 columns in place of the second accumulator
+            const uint32_t sum = tmem_base + lane_base + kSumCol + (uint32_t)(c * 32);
+            if (chunk > 0) add_cross_terms(sum, r);
+            if (chunk < chunks - 1) {
+              tmem_st16(sum, r);
+              tmem_st16(sum + 16, r + 16);
+              continue;
+            }
+          }
+          if (RAG)
+            store_c_ragged(c_dst, p.K, i - lane, p.I, p.rt.lo(t) + jc - t * p.tile_w, min(32, j_end - jc), r,
+                           reinterpret_cast<uint32_t*>(bars + 1) + quad * kRagStageWords, lane);
+          else if (i < p.I) store_c_row(c_dst, c_f32, p.K, i, jc, j_end, r, c_scale);
+        }
+        if (CHUNK) tmem_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars->acc_empty[b]);
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bars->acc_empty[b]);
     }
   } else if (warp >= 8 && masked && (int)blockIdx.x < num_work) {
     // ---- mask transform: zero the gradient entries the tile's ADC clamp blocked ---------
@@ -863,9 +877,10 @@ struct PlaneSpec {
 
 using BwdKernel = void (*)(const CUtensorMap, const CUtensorMap, const BwdTcParams);
 template <int BN>
-static BwdKernel pick_bwd_kernel(bool wgrad, bool ragged) {
-  if (ragged) return wgrad ? bwd_tc_kernel<true, true, BN> : bwd_tc_kernel<false, true, BN>;
-  return wgrad ? bwd_tc_kernel<true, false, BN> : bwd_tc_kernel<false, false, BN>;
+static BwdKernel pick_bwd_kernel(bool wgrad, bool ragged, bool chunked) {
+  if (chunked) return wgrad ? bwd_tc_kernel<true, true, BN, true> : bwd_tc_kernel<false, true, BN, true>;
+  if (ragged) return wgrad ? bwd_tc_kernel<true, true, BN, false> : bwd_tc_kernel<false, true, BN, false>;
+  return wgrad ? bwd_tc_kernel<true, false, BN, false> : bwd_tc_kernel<false, false, BN, false>;
 }
 
 static int launch_bwd_tc(bool wgrad, const void* g, const void* b_op, const uint32_t* keep_mask,
@@ -930,12 +945,13 @@ static int launch_bwd_tc(bool wgrad, const void* g, const void* b_op, const uint
   const bool pair = bn == 0;
   p.num_jb = (width + (pair ? P_BN : bn) - 1) / (pair ? P_BN : bn);
   if (pair) p.a_rows = BM;
+  const bool chunked = rt != nullptr && p.lsteps > kRagChunkSteps;
   // before the maps: this runtime call also binds the device's context to the calling thread (autograd's own threads),
   // which the driver entry point that encodes them needs
   const BwdKernel kernel = pair        ? (wgrad ? bwd_tc_pair_kernel<true> : bwd_tc_pair_kernel<false>)
-                           : bn == 256 ? pick_bwd_kernel<256>(wgrad, rt != nullptr)
-                           : bn == 128 ? pick_bwd_kernel<128>(wgrad, rt != nullptr)
-                                       : pick_bwd_kernel<64>(wgrad, rt != nullptr);
+                           : bn == 256 ? pick_bwd_kernel<256>(wgrad, rt != nullptr, chunked)
+                           : bn == 128 ? pick_bwd_kernel<128>(wgrad, rt != nullptr, chunked)
+                                       : pick_bwd_kernel<64>(wgrad, rt != nullptr, chunked);
   const int smem = pair ? P_SMEM : bwd_smem(bn) + (rt ? kRagStageBytes : 0);
   int rc = ensure_smem(kernel, smem);
   if (rc) return rc;

@@ -87,7 +87,9 @@ __device__ __forceinline__ void normals16(uint64_t seed, uint64_t offset, uint64
 //
 // BN: columns of a single CTA's block (pick_blocks; 256 x 4096 x 4096 with ADC: 27 us in 64 blocks of 128 columns, 15.8 us
 // in 128 of 64 issued by elected threads).  A copy of A brings no rows beyond M.
-template <int RD, int MODE, bool PAIR, int IO = kBF16, bool RAG = false, int BN = F_BN>
+// CHUNK: tiles of more than 64 * kRagChunkSteps columns (a kernel of its own: as a run-time switch it cost the others
+// registers).
+template <int RD, int MODE, bool PAIR, int IO = kBF16, bool RAG = false, int BN = F_BN, bool CHUNK = false>
 __global__ void __launch_bounds__(fwd_threads(PAIR, BN), 1)
 fwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
               const FwdTcParams p) {
@@ -111,6 +113,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const FwdEpilogueParams& ep = p.ep;
+  const int chunks = CHUNK ? (p.ksteps + kRagChunkSteps - 1) / kRagChunkSteps : 1;  // accumulators per analog tile
   const int T = ep.T;
   const int num_tiles = p.num_mb * p.num_nb;  // num_mb counts blocks of kBlockRows rows
   const uint32_t rank = PAIR ? cluster_ctarank() : 0u;
@@ -213,7 +216,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
       bool ok = true;
       const bool withhold = *(volatile uint32_t*)&g_tc_withhold_acc_signal != 0u;  // test aid, see its declaration
       for (int tile = worker; tile < num_tiles && ok; tile += n_workers) {
-        for (int t = 0; t < T && ok; ++t, ++acc_it) {
+        for (int part = 0; part < T * chunks && ok; ++part, ++acc_it) {  // chunk part % chunks of an analog tile
           const int b = acc_it & 1u;
           const uint32_t aph = (acc_it >> 1) & 1u;
           if (!mbar_wait(&bars->acc_empty[b], aph ^ 1u, abort_flag)) {
@@ -223,7 +226,9 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
           }
           tc_fence_after();
           const uint32_t d_tmem = tmem_base + (uint32_t)(b * kBN);
-          for (int ks = 0; ks < p.ksteps; ++ks, ++it) {
+          const int ks0 = CHUNK ? part % chunks * kRagChunkSteps : 0;
+          const int ks1 = CHUNK ? min(ks0 + kRagChunkSteps, p.ksteps) : p.ksteps;
+          for (int ks = ks0; ks < ks1; ++ks, ++it) {
             const int s = it % kStages;
             const uint32_t ph = (it / kStages) & 1u;
             if (!mbar_wait(&bars->full[s], ph, abort_flag)) {
@@ -239,7 +244,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
 #pragma unroll
               for (int k4 = 0; k4 < BK / 16; ++k4) {
                 const uint64_t dbp = db + (uint64_t)(plane * (kPlaneBytes >> 4) + k4 * 2);
-                const uint32_t acc = (ks | k4 | plane) != 0 ? 1u : 0u;
+                const uint32_t acc = ((ks - ks0) | k4 | plane) != 0 ? 1u : 0u;
                 if (PAIR) umma_bf16_pair(d_tmem, da + (uint64_t)(k4 * 2), dbp, idesc, acc);
                 else umma_bf16(d_tmem, da + (uint64_t)(k4 * 2), dbp, idesc, acc);
               }
@@ -299,6 +304,29 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
       const bool row_ok = m < M;
       const int n_first = nb * kBN + col0;
       for (int t = 0; t < T && ok; ++t, ++acc_it) {
+        // all but the last chunk of a wide tile: added up in tensor memory
+        for (int chunk = 0; CHUNK && chunk < chunks - 1 && ok; ++chunk, ++acc_it) {
+          if (!mbar_wait(&bars->acc_full[acc_it & 1u], (acc_it >> 1) & 1u, abort_flag)) {
+            if (lane == 0) raise_error(kErrEpilogue, abort_flag);
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+#pragma unroll 1
+          for (int h = 0; h < kCols / 16; ++h) {
+            uint32_t accr[16];
+            const uint32_t partial = tmem_base + lane_base + (uint32_t)(3 * kBN + col0 + h * 16);
+            tmem_ld16(tmem_base + lane_base + (acc_it & 1u) * (uint32_t)kBN + (uint32_t)(col0 + h * 16), accr);
+            tmem_wait_ld();
+            if (chunk > 0) add_tmem16(partial, accr);
+            tmem_st16(partial, accr);
+          }
+          tmem_wait_st();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bars->acc_empty[acc_it & 1u]);
+        }
+        if (CHUNK && !ok) break;
         const int b = acc_it & 1u;
         const uint32_t aph = (acc_it >> 1) & 1u;
         // constants of this (row, analog tile): fetched and derived before waiting for the
@@ -380,6 +408,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
             }
           }
           tmem_wait_ld();
+          if (CHUNK) add_tmem16(tmem_base + lane_base + (uint32_t)(3 * kBN + cc), accr);
           if (IO == kF32) {
 #pragma unroll
             for (int j = 0; j < 16; ++j) accr[j] = __float_as_uint(fmul(__uint_as_float(accr[j]), dac_step));
@@ -821,10 +850,10 @@ bool tc_ragged_supported(const AlDesc& d, const TileTable& tt, RaggedTiles* rt) 
   return (int64_t)rt->T * rt->pitch < (1ll << 31);
 }
 
-template <int BN>
+template <int BN, bool CHUNK = false>
 static FwdKernel pick_ragged_kernel(int round_dt) {
-  return round_dt == AL_BF16 ? fwd_tc_kernel<kBF16, -1, false, kBF16, true, BN>
-                             : fwd_tc_kernel<kF32, -1, false, kBF16, true, BN>;
+  return round_dt == AL_BF16 ? fwd_tc_kernel<kBF16, -1, false, kBF16, true, BN, CHUNK>
+                             : fwd_tc_kernel<kF32, -1, false, kBF16, true, BN, CHUNK>;
 }
 
 int launch_fwd_tc_ragged(int round_dt, const void* xq, const void* w_mod, const RaggedTiles& rt,
@@ -839,15 +868,18 @@ int launch_fwd_tc_ragged(int round_dt, const void* xq, const void* w_mod, const 
   p.ksteps = (p.tile_w + BK - 1) / BK;
   p.num_mb = (ep.M + BM - 1) / BM;
   p.a_rows = fwd_copy_rows(ep.M);
-  const int bn = fwd_block_columns(ep.M, ep.N);
+  const bool chunked = p.ksteps > kRagChunkSteps;
+  const int bn = chunked ? 64 : fwd_block_columns(ep.M, ep.N);
   p.num_nb = (ep.N + bn - 1) / bn;
   p.inp_res = 0.0f;
   p.ep = ep;
   p.noise = make_noise_keys(ep.seed, ep.offset, 1u, ep.offset_base);
   p.out = out;
   p.small_adc_codes = small_adc_codes(p.tile_w, ep);
-  FwdKernel kernel = bn == 128  ? pick_ragged_kernel<128>(round_dt)
-                     : bn == 64 ? pick_ragged_kernel<64>(round_dt) : pick_ragged_kernel<32>(round_dt);
+  FwdKernel kernel = chunked     ? pick_ragged_kernel<64, true>(round_dt)
+                     : bn == 128 ? pick_ragged_kernel<128>(round_dt)
+                     : bn == 64  ? pick_ragged_kernel<64>(round_dt)
+                                 : pick_ragged_kernel<32>(round_dt);
   const int smem = fwd_smem(bn, 1) + rag_stage_bytes(bn);
   int rc = ensure_smem(kernel, smem);
   if (rc) return rc;

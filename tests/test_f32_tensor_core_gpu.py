@@ -116,7 +116,7 @@ def test_engines_run_the_forward_kernel_they_name(rows, n, columns):
                 torch.cuda.synchronize()
         names = " ".join(e.key for e in prof.key_averages())
         # rounding type, output stage, pairs, element type, ragged, columns staged per CTA
-        ran[engine] = re.search(r"fwd_tc_kernel<\d+, -?\d+, (\w+), \d+, \w+, (\d+)>", names).groups()
+        ran[engine] = re.search(r"fwd_tc_kernel<\d+, -?\d+, (\w+), \d+, \w+, (\d+)[,>]", names).groups()
     assert ran == {"tcgen05_single": ("false", str(columns)), "tcgen05_pair": ("true", "64")}
     # one order of the sum over k on either
     assert rel_fro(outs["tcgen05_single"], outs["tcgen05_pair"]) <= 1e-6

@@ -20,6 +20,7 @@ SHAPES = [
     (32, 4100, 1030, -1),     # a tile wider than a warp keeps in registers
     (1000, 2500, 1500, 512),
     (300, 1001, 67, 77),      # 13 narrow tiles of 77, few channels
+    (8193, 1000, 1300, 250),  # sums over the rows in two chunks
     (1, 70, 9, 35),           # the smallest calls: one row, a few channels, tiles narrower than a k-step
 ]
 OPTIONS = {
@@ -147,3 +148,45 @@ def test_operand_pitch_is_checked_on_the_host():
     args.x = args.w = args.out = args.xq = args.w_mod = args.ir_rows = buf.data_ptr()
     args.tile_ends = ends
     assert lib.al_forward(even, args, None) != _lib.AL_OK
+
+
+@pytest.mark.parametrize("rows,k,n,tile", [(65536, 1000, 1281, 250), (1024, 1001, 20001, -1),
+                                           (2048, 16385, 515, -1), (2048, 24601, 130, -1)],
+                         ids=["rows_many_blocks", "channels", "features", "features_narrow"])
+def test_long_sums_are_not_truncated(rows, k, n, tile):
+    """Outputs and gradients are sums over features, rows or channels, in chunks of 8192 terms.  The tensor core adds 16
+    terms at a time into a truncated accumulator: each of the 512 additions of a chunk shortens its sum by up to an ulp
+    (2^-23; half of one on average, of a sum that grows like the root of the terms so far, so a third of 512 * 2^-23 =
+    2e-5 of the whole); roundings of the bf16 result have no direction.  A sum in one accumulator loses four and more
+    times as much."""
+    layer = _layer(k, n, tile, OPTIONS["plain"])
+    layer.train()
+    layer.bias.data.zero_()
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    x = torch.randn(rows, k, device="cuda", generator=gen, dtype=torch.float32).bfloat16()
+    g = torch.randn(rows, n, device="cuda", generator=gen, dtype=torch.float32).bfloat16()
+    out, gx, grads, xq, w_mod = _pass(layer, x, g, "auto")
+    assert xq.shape[1] != k  # on the tensor cores
+    xq, w_mod = _dense(xq, layer.in_sizes), _dense(w_mod, layer.in_sizes).double()
+    inside = x.abs() < 2.5  # the static range blocks the others
+    exact_w = torch.zeros(n, k, device="cuda", dtype=torch.float64)
+    shrink, size, square, count = [0.0, 0.0], [0.0, 0.0], [0.0, 0.0], [0, 0]
+
+    def add(i, value, exact):
+        shrink[i] += (exact.abs() - value.double() * exact.sign()).sum().item()
+        size[i] += exact.abs().sum().item()
+        square[i] += (value.double() - exact).square().sum().item()
+        count[i] += exact.numel()
+
+    for a in range(0, rows, 8192):
+        rr = slice(a, a + 8192)
+        exact_w += g[rr].double().t() @ xq[rr].double()
+        if len(layer.in_sizes) == 1:  # more tiles: rounded to bf16 after each
+            add(0, out[rr], xq[rr].double() @ w_mod.t())
+        add(1, gx[rr][inside[rr]], (g[rr].double() @ w_mod)[inside[rr]])
+    shrink.append(0.0), size.append(0.0), square.append(0.0), count.append(0)
+    add(2, grads["weight"], exact_w)
+    for i in range(3):
+        if count[i]:
+            noise = 4.0 * (square[i] ** 0.5) / size[i]  # four standard errors of a sum of independent roundings
+            assert abs(shrink[i] / size[i]) <= 2e-5 + noise, (i, shrink[i] / size[i], noise)
