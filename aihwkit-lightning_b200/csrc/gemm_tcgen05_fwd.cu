@@ -838,15 +838,17 @@ int launch_fwd_tc(int round_dt, const void* xq, const void* w_mod, int K, const 
 //   333 x 1000 x 777 evaluation                99 -> 25     64 x 300 x 100       40 -> 20,  65 -> 49
 //   16 x 4001 x 4001                          408 -> 66     32 x 70 x 70         25 -> 18,  42 -> 36
 //   100 x 2000 x 20 (tiles of 20)            1039 -> 261    8000 x 100 x 10      36 -> 22, 125 -> 97
+//   65536 x 1000 x 777                        4689 -> 351, 14007 -> 853
 // so there is no lower size.  Three lines: tiles narrower than 8 columns would be mostly padding; tiles that are not as
-// even as possible have no closed-form start (no module makes them); and the weight gradient here does not split its
-// reduction over the rows, so a layer of few output blocks leaves from 8192 rows on.
+// even as possible have no closed-form start (no module makes them); and beyond 8192 rows a layer with few products a
+// row stays with the CUDA cores, which split the rows of a weight gradient over the chip where one CTA walks them all
+// here (forward + backward: 32768 x 100 x 10 135 -> 193, 65536 x 147 x 64 309 -> 339, 65536 x 288 x 33 428 -> 424,
+// 65536 x 500 x 100 1225 -> 574), and an evaluation with next to none (65536 x 27 x 16 56 -> 60, 65536 x 33 x 30 73 -> 63).
 bool tc_ragged_supported(const AlDesc& d, const TileTable& tt, RaggedTiles* rt) {
   if (d.dtype != AL_BF16 || (d.engine != AL_ENGINE_AUTO && d.engine != AL_ENGINE_PITCHED) || tc_tiling_ok(d, tt) ||
       !ragged_tiles(tt, rt))
     return false;
-  const int64_t blocks = (int64_t)((d.N + BM - 1) / BM) * rt->T * ((rt->widest() + 255) / 256);
-  if (rt->widest() < 8 || (d.M > 8192 && blocks < 37)) return false;
+  if (rt->widest() < 8 || (d.M > 8192 && (int64_t)d.K * d.N < (d.save_for_backward ? 10000 : 500))) return false;
   return (int64_t)rt->T * rt->pitch < (1ll << 31);
 }
 

@@ -20,7 +20,8 @@ SHAPES = [
     (32, 4100, 1030, -1),     # a tile wider than a warp keeps in registers
     (1000, 2500, 1500, 512),
     (300, 1001, 67, 77),      # 13 narrow tiles of 77, few channels
-    (8193, 1000, 1300, 250),  # sums over the rows in two chunks
+    (8193, 515, 130, 260),    # sums over the rows in two chunks, 64- and 128-column blocks
+    (24577, 1000, 777, 512),  # in four
     (1, 70, 9, 35),           # the smallest calls: one row, a few channels, tiles narrower than a k-step
 ]
 OPTIONS = {
@@ -137,8 +138,14 @@ def test_operand_pitch_is_checked_on_the_host():
     with F.operator_settings(engine="simt"):
         other = F.make_desc(layer.rpu_config, 130, 1001, 515, 2, torch.bfloat16, False)
     assert lib.al_operand_pitch(other, ends) == 0  # another engine: the dense layout
-    tall = F.make_desc(layer.rpu_config, 8193, 1001, 515, 2, torch.bfloat16, False)
-    assert lib.al_operand_pitch(tall, ends) == 0   # 5 x 4 blocks of the weight gradient, a long reduction
+    # beyond 8192 rows a training call with few products a row stays with the CUDA cores, an evaluation does not
+    for rows, k, n, train, pitch in ((8193, 1001, 515, True, 1008), (8192, 100, 10, True, 104), (8193, 100, 10, True, 0),
+                                     (8193, 100, 100, True, 104), (8193, 100, 10, False, 104), (8193, 27, 16, False, 0),
+                                     (8192, 27, 16, False, 32)):
+        tiles = [k] if k < 1001 else layer.in_sizes
+        tall = F.make_desc(layer.rpu_config, rows, k, n, len(tiles), torch.bfloat16, train)
+        tall.save_for_backward = int(train)
+        assert lib.al_operand_pitch(tall, _lib.tile_ends_array(tiles)) == pitch, (rows, k, n, train)
     even = F.make_desc(layer.rpu_config, 130, 1024, 512, 2, torch.bfloat16, False)
     ends = _lib.tile_ends_array([512, 512])
     even.engine = _lib.AL_ENGINE_PITCHED  # announced for a layer that has no pitched layout
@@ -150,9 +157,9 @@ def test_operand_pitch_is_checked_on_the_host():
     assert lib.al_forward(even, args, None) != _lib.AL_OK
 
 
-@pytest.mark.parametrize("rows,k,n,tile", [(65536, 1000, 1281, 250), (1024, 1001, 20001, -1),
+@pytest.mark.parametrize("rows,k,n,tile", [(65536, 1000, 1281, 250), (262144, 500, 100, -1), (1024, 1001, 20001, -1),
                                            (2048, 16385, 515, -1), (2048, 24601, 130, -1)],
-                         ids=["rows_many_blocks", "channels", "features", "features_narrow"])
+                         ids=["rows_many_blocks", "rows_few_blocks", "channels", "features", "features_narrow"])
 def test_long_sums_are_not_truncated(rows, k, n, tile):
     """Outputs and gradients are sums over features, rows or channels, in chunks of 8192 terms.  The tensor core adds 16
     terms at a time into a truncated accumulator: each of the 512 additions of a chunk shortens its sum by up to an ulp
