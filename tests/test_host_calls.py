@@ -76,3 +76,30 @@ def test_static_ranges_are_copied_back_only_where_they_were_copied():
         assert (copies.count > 0) == strided
         ranges.append(layer.input_range.detach().clone())
     assert torch.equal(*ranges) and not bool((ranges[0] == 3.0).any())  # updated from the data
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_convolution_takes_gradients_of_any_layout(dtype):
+    """The operator transposes the gradient of its images: one that is not contiguous gives what its copy gives."""
+    from aihwkit_lightning_b200.nn import AnalogConv2d
+    from aihwkit_lightning_b200.simulator.configs import TorchInferenceRPUConfig
+
+    rpu = TorchInferenceRPUConfig()
+    rpu.mapping.max_input_size, rpu.forward.inp_res = 64, 254.0
+    rpu.pre_post.input_range.enable = rpu.pre_post.input_range.dynamic = True
+    torch.manual_seed(0)
+    conv = AnalogConv2d(8, 20, 3, padding=1, rpu_config=rpu, device="cuda", dtype=dtype).train()
+    x = torch.randn(3, 8, 9, 7, device="cuda").to(dtype)
+    g = torch.randn(3, 20, 9, 7, device="cuda").to(dtype)
+    layouts = [g, g.contiguous(memory_format=torch.channels_last), g.transpose(2, 3).contiguous().transpose(2, 3),
+               torch.cat([g, g], dim=1)[:, 20:], g[:, :, :1, :1].expand(3, 20, 9, 7)]
+    for grad in layouts:
+        results = []
+        for gg in (grad, grad.clone(memory_format=torch.contiguous_format)):
+            conv.zero_grad()
+            xs = x.clone().requires_grad_(True)
+            conv(xs).backward(gg)
+            results.append((xs.grad, conv.weight.grad.clone(), conv.bias.grad.clone()))
+        for a, b in zip(*results):
+            assert torch.equal(a, b)

@@ -1,9 +1,11 @@
-"""bf16 layers whose sizes are no multiples of 8 on the tensor cores, against the CUDA-core GEMMs of the same layer:
-the operands of the two (DAC output, modified weights, noise included) are the same bits, laid out differently."""
+"""bf16 layers whose sizes are no multiples of 8 on the tensor cores, against the oracle and the CUDA-core GEMMs of the same
+layer: the operands of the two (DAC output, modified weights, noise included) are the same bits, laid out differently."""
 import pytest
 import torch
 
-from util import rel_fro
+import cases as C
+from test_parity_gpu import check_close
+from util import oracle_run, rel_fro, run_product_layer
 
 pytestmark = pytest.mark.gpu
 
@@ -124,6 +126,49 @@ def test_ragged_layer_unaligned_inputs_and_gradients():
     a, b = _pass(layer, x, g, "auto"), _pass(layer, x, g, "simt")
     assert rel_fro(a[0], b[0]) <= BF16_REL and rel_fro(a[1], b[1]) <= BF16_REL
     assert rel_fro(a[2]["weight"], b[2]["weight"]) <= BF16_REL
+
+
+@pytest.mark.parametrize("name", OPTIONS)
+@pytest.mark.parametrize("k,n,tile", [(1000, 777, 512), (1001, 515, 77), (1024, 131, 512)])
+def test_ragged_layer_unaligned_weights(k, n, tile, name):
+    """Weights two bytes into an allocation: the same modified weights, noise included, as the dense pass writes."""
+    rows = 70
+    layer = _layer(k, n, tile, OPTIONS[name])
+    layer.train()
+    flat = torch.empty(n * k + 1, device="cuda", dtype=torch.bfloat16)
+    view = flat[1:].view(n, k)
+    view.copy_(layer.weight.data)
+    layer.weight.data = view
+    x, g = torch.randn(rows, k, device="cuda").bfloat16(), torch.randn(rows, n, device="cuda").bfloat16()
+    out, gx, grads, xq, w_mod = _pass(layer, x, g, "auto")
+    out_s, gx_s, grads_s, xq_s, w_mod_s = _pass(layer, x, g, "simt")
+    assert (xq.shape[1] != k) == any(w % 8 for w in layer.in_sizes)
+    assert torch.equal(_dense(xq, layer.in_sizes), xq_s) and torch.equal(_dense(w_mod, layer.in_sizes), w_mod_s)
+    assert rel_fro(out, out_s) <= BF16_REL and rel_fro(gx, gx_s) <= BF16_REL
+    assert rel_fro(grads["weight"], grads_s["weight"]) <= BF16_REL
+
+
+@pytest.mark.parametrize("base,over", [
+    ("bf16_static_adc", dict(in_shape=(130, 777), out_features=515, max_input_size=260, ir_init_value=2.0)),
+    ("bf16_dynamic_eval", dict(in_shape=(65, 1001), out_features=70, max_input_size=512)),
+    ("bf16_discretize", dict(in_shape=(200, 300), out_features=131, max_input_size=77, ir_init_value=2.0)),
+    ("bf16_learnable_clip", dict(in_shape=(70, 500), out_features=33, max_input_size=250, ir_init_value=2.0)),
+])
+def test_ragged_layer_matches_oracle(base, over):
+    from aihwkit_lightning_b200 import _lib
+    from aihwkit_lightning_b200.nn import functional as F
+
+    case = dict(C.CASES_BY_NAME[base], weight_scale=0.05, steps=1)
+    case.update(over, noise_type="None", out_noise=0.0)  # replayed noise would keep the layer on the CUDA cores
+    data = C.make_inputs(case)
+    rec, grads = oracle_run(case, data)
+    layer, x, out = run_product_layer(case, dict(data, w_noise=[None], out_noise=[None]))
+    rows, k = x.shape
+    desc = F.make_desc(layer.rpu_config, rows, k, data["n"], len(layer.in_sizes), torch.bfloat16, case["training"])
+    assert _lib.load().al_operand_pitch(desc, _lib.tile_ends_array(layer.in_sizes)) > 0
+    check_close("out", out, rec.out, torch.bfloat16, case)
+    check_close("grad_x", x.grad, grads["grad_x"], torch.bfloat16, case)
+    check_close("grad_w", layer.weight.grad, grads["grad_w"], torch.bfloat16, case)
 
 
 def test_operand_pitch_is_checked_on_the_host():
