@@ -21,7 +21,8 @@ constexpr int kRows = 16;  // columns of one MMA, rows of the layer's input; row
 // warps read the same stage once more from shared memory for the abs-max of its channels.  A CTA per (64 channels,
 // tile) with mma.sync, which staged (and quantised) its 16 KiB of inputs for 64 KiB of weights before its first product
 // and left its last wave mostly empty, was slower at every size, calls replayed from a graph, in us (then -> now):
-//   1 x 512 x 512 10.4 -> 8.0, 1 x 4096 x 4096 20.9 -> 16.1, 16 x 8192 x 3072 35.0 -> 25.8, 16 x 3072 x 16384 42.8 -> 33.1.
+//   1 x 512 x 512 10.3 -> 8.1, 1 x 4096 x 4096 20.5 -> 15.4, 16 x 8192 x 3072 34.9 -> 25.5, 16 x 3072 x 16384 42.0 -> 31.8.
+// Launched call by call the DAC pass in front costs a launch: a single row of 2048 x 2048 21.5 -> 24.1.
 // Results differ from 64 bits by the same 1.664e-3 (bf16 outputs) as before.
 constexpr int S_CH = 128;                                  // channels of an item: rows of the MMA
 constexpr int S_W_BYTES = S_CH * BK * 2, S_X_BYTES = kRows * BK * 2;

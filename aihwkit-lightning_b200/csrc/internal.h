@@ -221,7 +221,7 @@ int launch_wgrad_tc_f32(const void* g_planes, int sets, const void* codes16, int
                         const float* scale_ir, float inp_res, int pairing, void* grad_w, cudaStream_t s, int splits = 1,
                         float* partial = nullptr);
 int tc_read_device_error(cudaStream_t s, uint32_t* code);
-// limit of the device-side waits of all tcgen05 kernels (both translation units)
+// limit of the device-side waits of all tcgen05 kernels (three translation units)
 int tc_set_wait_limit(unsigned long long ns);
 cudaError_t tc_fwd_set_wait_limit(unsigned long long ns);
 // the few-rows translation unit's own limit and error word

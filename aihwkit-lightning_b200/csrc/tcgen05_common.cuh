@@ -497,7 +497,8 @@ constexpr int bwd_smem(int bn) { return bwd_stages(bn) * bwd_stage_bytes(bn) + (
 // 4096).  Against 128-wide (forward) and 128- or 256-wide (backward) blocks throughout: 1.12x (geometric mean of 41 sizes
 // from 17 x 1024 x 1024 to 4096^3), 512 x 1024 x 1024 training 39.8 -> 33.9 us, 2048^3 105 -> 82, none slower by over 1 %.
 // n_pairs: CTA pairs the device runs at once (0: none), pair_blocks their blocks (32 KiB per CTA and k-step);
-// blocks_of(bn): blocks of 128 x bn columns, which stage `planes` planes of their second operand.  Returns 0 for pairs, else the block width; the narrower of two that cost the same.
+// blocks_of(bn): blocks of 128 x bn columns, which stage `planes` planes of their second operand.  Returns 0 for pairs, else
+// the block width; the narrower of two that cost the same.
 template <class BlocksOf>
 int pick_blocks(int n_pairs, int64_t pair_blocks, int sms, int widest, int narrowest, BlocksOf blocks_of, int planes = 1) {
   int best = 0;
