@@ -218,8 +218,9 @@ static_ir_partial_kernel(const void* __restrict__ x, const void* __restrict__ ir
 #pragma unroll
     for (int w = 1; w < 8; ++w) sum += part[w][threadIdx.x];
     float* const p = partial + (((int64_t)t * gridDim.x + blockIdx.x) * 3 + threadIdx.x) * 2;
-    p[0] = (float)sum;
-    p[1] = (float)(sum - (double)p[0]);
+    const float high = (float)sum;
+    p[0] = high;
+    p[1] = isfinite(high) ? (float)(sum - (double)high) : 0.0f;  // an infinite sum stays infinite
   }
 }
 

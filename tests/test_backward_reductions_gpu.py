@@ -1,5 +1,7 @@
 """Reductions of the backward pass against float64 sums: the bias gradient (column sums over a cluster of CTAs) and
 the gradient of a static input range with its straight-through zeroing."""
+import math
+
 import pytest
 import torch
 
@@ -67,13 +69,23 @@ def test_static_range_gradient_and_clipped_inputs(dtype, m, k, tiles):
                          ids=["row_per_warp", "rows_of_a_warp", "two_blocks", "two_short_blocks"])
 def test_range_gradient_keeps_small_terms_between_large_ones(m, rows):
     """Rows of 2^24, 1 and -2^24: fp32 sums over rows lose the 1, which the result consists of."""
+    _range_gradient(m, rows, (2.0 ** 24, 1.0, -(2.0 ** 24)), 1.0)
+
+
+@pytest.mark.parametrize("values,want", [((math.inf, 1.0, -2.0), math.inf), ((1.0, -math.inf, 2.0), -math.inf),
+                                         ((3e38, 3e38, 3e38), math.inf)])
+def test_range_gradient_of_infinite_gradients(values, want):
+    _range_gradient(18976, (0, 1, 18975), values, want)
+
+
+def _range_gradient(m, rows, values, want):
     from aihwkit_lightning_b200 import _lib
 
     lib = _lib.load()
     k = 32
     x = torch.zeros(m, k, device="cuda")
     g = torch.zeros(m, 1, device="cuda")
-    for row, v in zip(rows, (2.0 ** 24, 1.0, -(2.0 ** 24))):
+    for row, v in zip(rows, values):
         x[row, 5], g[row, 0] = 2.0, v
     w, ir = torch.ones(1, k, device="cuda"), torch.ones(1, device="cuda")
     grad_x, grad_ir = torch.empty(m, k, device="cuda"), torch.empty(1, device="cuda")
@@ -88,7 +100,7 @@ def test_range_gradient_keeps_small_terms_between_large_ones(m, rows):
     args.grad_x, args.grad_input_range = grad_x.data_ptr(), grad_ir.data_ptr()
     args.reduce_scratch, args.reduce_scratch_floats = scratch.data_ptr(), scratch.numel()
     _lib.check(lib.al_backward(desc, args, torch.cuda.current_stream().cuda_stream))
-    assert grad_ir.item() == 1.0
+    assert grad_ir.item() == want
     assert not bool(grad_x[x > 1].any())
 
 
