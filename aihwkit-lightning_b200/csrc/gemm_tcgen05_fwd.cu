@@ -844,11 +844,14 @@ int launch_fwd_tc(int round_dt, const void* xq, const void* w_mod, int K, const 
 // row stays with the CUDA cores, which split the rows of a weight gradient over the chip where one CTA walks them all
 // here (forward + backward: 32768 x 100 x 10 135 -> 193, 65536 x 147 x 64 309 -> 339, 65536 x 288 x 33 428 -> 424,
 // 65536 x 500 x 100 1225 -> 574), and an evaluation with next to none (65536 x 27 x 16 56 -> 60, 65536 x 33 x 30 73 -> 63).
+// Each tile is a block of its own here and a pass of its own there: the products count once per tile (65536 x 100 x 10
+// in 5 tiles 448 -> 503, in 10 826 -> 688; 65536 x 300 x 30 in 38 3543 -> 1930).
 bool tc_ragged_supported(const AlDesc& d, const TileTable& tt, RaggedTiles* rt) {
   if (d.dtype != AL_BF16 || (d.engine != AL_ENGINE_AUTO && d.engine != AL_ENGINE_PITCHED) || tc_tiling_ok(d, tt) ||
       !ragged_tiles(tt, rt))
     return false;
-  if (rt->widest() < 8 || (d.M > 8192 && (int64_t)d.K * d.N < (d.save_for_backward ? 10000 : 500))) return false;
+  const int64_t row_work = (int64_t)d.K * d.N * rt->T;
+  if (rt->widest() < 8 || (d.M > 8192 && row_work < (d.save_for_backward ? 10000 : 500))) return false;
   return (int64_t)rt->T * rt->pitch < (1ll << 31);
 }
 

@@ -186,8 +186,8 @@ def test_operand_pitch_is_checked_on_the_host():
     # beyond 8192 rows a training call with few products a row stays with the CUDA cores, an evaluation does not
     for rows, k, n, train, pitch in ((8193, 1001, 515, True, 1008), (8192, 100, 10, True, 104), (8193, 100, 10, True, 0),
                                      (8193, 100, 100, True, 104), (8193, 100, 10, False, 104), (8193, 27, 16, False, 0),
-                                     (8192, 27, 16, False, 32)):
-        tiles = [k] if k < 1001 else layer.in_sizes
+                                     (8192, 27, 16, False, 32), (8193, 296, 1, True, 37 * 8), (8193, 296, 1, False, 37 * 8)):
+        tiles = [8] * 37 if k == 296 else [k] if k < 1001 else layer.in_sizes
         tall = F.make_desc(layer.rpu_config, rows, k, n, len(tiles), torch.bfloat16, train)
         tall.save_for_backward = int(train)
         assert lib.al_operand_pitch(tall, _lib.tile_ends_array(tiles)) == pitch, (rows, k, n, train)
